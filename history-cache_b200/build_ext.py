@@ -1,13 +1,15 @@
-"""Builds libhiscache_b200.so in-tree with nvcc for sm_100a.
+"""Builds libhiscache_b200.so and the Python module hiscache_backend._native in-tree (nvcc for sm_100a).
 
     python history-cache_b200/build_ext.py [--force] [--verbose]
 
 The library has no torch or Python dependency: it is compiled from csrc/*.cu
-against include/hiscache_b200.h only and loaded with ctypes.
+against include/hiscache_b200.h only and loaded with ctypes.  The module (csrc/torch_ops.cpp) is
+host code only: it wraps the library's functions for torch tensors.
 """
 from __future__ import annotations
 
 import os
+import shutil
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -46,15 +48,44 @@ def _stale(target, inputs):
 
 
 CHECKED_LIB_PATH = os.path.join(LIB_DIR, "libhiscache_b200_checked.so")
+NATIVE_SRC = os.path.join(CSRC, "torch_ops.cpp")
+NATIVE_PATH = os.path.join(HERE, "hiscache_backend", "_native.so")
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compiles every kernel source and links the shared library; returns its path.  Also builds
     libhiscache_b200_checked.so: the same sources with -DHC_CHECK_BOUNDS (index checks in front
-    of the aggregation operators, see hc_last_status in the header)."""
-    path = _build_one(force, verbose, OBJ_DIR, LIB_PATH, [])
-    _build_one(force, False, os.path.join(LIB_DIR, "obj_checked"), CHECKED_LIB_PATH, ["-DHC_CHECK_BOUNDS"])
+    of the aggregation operators, see hc_last_status in the header), and the Python module."""
+    with ThreadPoolExecutor(max_workers=1) as ex:
+        native = ex.submit(_build_native, force, verbose)
+        path = _build_one(force, verbose, OBJ_DIR, LIB_PATH, [])
+        _build_one(force, False, os.path.join(LIB_DIR, "obj_checked"), CHECKED_LIB_PATH, ["-DHC_CHECK_BOUNDS"])
+        native.result()
     return path
+
+
+def _build_native(force, verbose):
+    deps = [NATIVE_SRC] + [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE) if f.endswith(".h")]
+    if not (force or _stale(NATIVE_PATH, deps)):
+        return
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc")))
+    cmd = ["g++", "-O2", "-std=c++20", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_native",
+           "-DTORCH_API_INCLUDE_EXTENSION_H",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI), "-I", INCLUDE,
+           "-isystem", os.path.join(root, "include"),
+           "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           "-isystem", sysconfig.get_paths()["include"], "-isystem", os.path.join(cuda, "include"),
+           NATIVE_SRC, "-o", NATIVE_PATH, "-L", os.path.join(root, "lib"), "-Wl,-rpath," + os.path.join(root, "lib"),
+           "-lc10", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-ltorch_cuda", "-ltorch_python"]
+    p = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or p.returncode != 0:
+        sys.stderr.write(" ".join(cmd) + "\n" + p.stdout + p.stderr)
+    if p.returncode != 0:
+        raise RuntimeError("g++ failed for " + NATIVE_SRC)
 
 
 def _build_one(force, verbose, obj_dir, lib_path, extra):

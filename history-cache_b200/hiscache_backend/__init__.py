@@ -26,6 +26,7 @@ import os
 import torch
 
 from . import _capi
+from . import _native
 from ._capi import (HC_F16, HC_F32, HC_SCORE_L1, HC_SCORE_L2, AggrArgs, check, dtype_code, i64c,
                     lib, on_device, ptr, require_cuda, rows2d, scratch, stream_of)
 
@@ -40,17 +41,12 @@ __all__ = [
     "PeerRegion", "peer_open", "peer_close", "peer_ptrs", "peer_lookup", "peer_publish", "peer_pull", "peer_admit", "make_shard",
 ]
 
-_launches = 0
-
-
 def launch_count() -> int:
     """Number of kernels of this library launched so far in this process."""
-    return _launches
+    return _native.launches()
 
 
-def _called(n=1):
-    global _launches
-    _launches += n
+_called = _native.add_launches
 
 
 class KernelTimer:
@@ -79,6 +75,7 @@ def set_kernel_timer(t):
     stream it launches on."""
     global _timer
     _timer = t
+    _native.set_timed(t is not None)
 
 
 class _span:
@@ -101,17 +98,15 @@ class _span:
         return False
 
 
+_native.open_library(_capi.lib._handle)
+_native.set_span(_span)
+
+
 def _tag(name, t):
     return f"{name}[{'f16' if t.dtype == torch.float16 else 'f32'},F={t.shape[-1]}]"
 
 
-class ScoreSink:
-    """Where the aggregation's backward pass leaves the per-row admission score.
-    `fresh` turns True when a backward pass has written `tensor` since the last reset."""
-
-    def __init__(self, tensor):
-        self.tensor = tensor
-        self.fresh = False
+ScoreSink = _native.ScoreSink
 
 
 def _empty(t):
@@ -144,105 +139,6 @@ def _aggr_args(inp, ptr_t, idx_t, num_node, edge_value, hmap, hbuf, h_indexed, s
     return a
 
 
-class _AggrFunction(torch.autograd.Function):
-    """Counterpart of AggrHistoryFunction / AggrHistoryEdgeValueFunction
-    (src/cpp/src/history_aggr.cu:475-596).  Saves the index tensors themselves
-    (the reference keeps raw device pointers across forward and backward,
-    history_aggr.cu:406-408)."""
-
-    @staticmethod
-    def forward(ctx, inp, ptr_t, idx_t, edge_value, hmap, hbuf, num_node, h_indexed, src_map,
-                src_alt, score_out, score_kind):
-        dev = require_cuda(inp, ptr_t, idx_t, edge_value, hmap, hbuf, src_map, src_alt)
-        inp = rows2d(inp)
-        ptr_t, idx_t = i64c(ptr_t, "ptr"), i64c(idx_t, "idx")
-        hmap, src_map = i64c(hmap, "history_map"), i64c(src_map, "src_map")
-        if edge_value is not None:
-            edge_value = edge_value.contiguous()
-            if edge_value.dtype != torch.float32:
-                raise TypeError("edge_value must be float32")
-        if hbuf is not None:
-            hbuf = rows2d(hbuf)
-        if src_alt is not None:
-            src_alt = rows2d(src_alt)
-        multi = inp.dim() == 3
-        if idx_t.numel() == 0:  # a block without edges still needs a valid address
-            idx_t = torch.zeros(1, dtype=torch.int64, device=dev)
-        if ptr_t.shape[0] < num_node + 1:
-            raise RuntimeError(f"aggr_forward: ptr has {ptr_t.shape[0]} entries, need {num_node + 1}")
-        if hmap is not None and hmap.shape[0] < num_node:
-            raise RuntimeError("aggr_forward: history_map shorter than num_node")
-        if hmap is not None and not h_indexed and hbuf.shape[0] < num_node:
-            raise RuntimeError("aggr_forward: row-aligned history_buffer shorter than num_node")
-        shape = (num_node, inp.shape[1], inp.shape[2]) if multi else (num_node, inp.shape[1])
-        out = torch.empty(shape, dtype=torch.float32, device=dev)
-        a = _aggr_args(inp, ptr_t, idx_t, num_node, edge_value, hmap, hbuf, h_indexed, src_map, src_alt)
-        with on_device(dev), _span(_tag("hc_aggr_fwd", inp), dev):
-            check(lib.hc_aggr_fwd(C.byref(a), ptr(out), stream_of(dev)), "hc_aggr_fwd")
-        _called()
-        ctx.save_for_backward(inp, ptr_t, idx_t, edge_value, hmap, hbuf, src_map, src_alt)
-        ctx.num_node, ctx.h_indexed = num_node, h_indexed
-        ctx.score_out, ctx.score_kind = score_out, score_kind
-        return out
-
-    @staticmethod
-    def backward(ctx, grad_out):
-        inp, ptr_t, idx_t, edge_value, hmap, hbuf, src_map, src_alt = ctx.saved_tensors
-        dev = inp.device
-        grad_out = grad_out.contiguous()
-        if grad_out.dtype != torch.float32:
-            grad_out = grad_out.float()
-        need_in = ctx.needs_input_grad[0]
-        need_ev = edge_value is not None and ctx.needs_input_grad[3]
-        need_h = hbuf is not None and ctx.needs_input_grad[5]
-        if need_h and ctx.h_indexed:
-            raise RuntimeError("gradients w.r.t. an indexed history table are not defined; "
-                               "pass a row-aligned history_buffer")
-        a = _aggr_args(inp, ptr_t, idx_t, ctx.num_node, edge_value, hmap, hbuf, ctx.h_indexed,
-                       src_map, src_alt)
-        g_in = torch.empty(inp.shape, dtype=torch.float32, device=dev) if need_in else None
-        g_ev = torch.empty_like(edge_value) if need_ev else None
-        # gather over the transposed block instead of the atomic scatter: always when a
-        # reproducible backward is asked for, else for blocks large enough to pay for it
-        gathered = False
-        can_gather = (need_in and edge_value is None and inp.dim() == 2 and inp.shape[1] % 4 == 0
-                      and inp.shape[1] <= 1024)
-        if can_gather and (DETERMINISTIC_BWD or (inp.shape[1] >= GATHER_MIN_FEAT and
-                                                 inp.shape[0] * inp.shape[1] * 4 >= GATHER_MIN_BYTES)):
-            pa = PreparedAggr(a, None, dev, _tag("", inp))
-            shared = shared_transpose(ptr_t, idx_t)
-            if shared is not None and shared[0].shape[0] - 1 >= inp.shape[0]:
-                t_ptr, t_dst, t_w, n_edges = shared
-            else:       # a block nobody declared: its own transposition
-                n_edges = idx_t.numel()
-                t_ptr, t_dst, t_w = transpose_block(pa, n_edges)
-            run_aggr_bwd_gather(pa, t_ptr, t_dst, t_w, grad_out, g_in, n_edges=n_edges)
-            gathered = True
-        g_h = None
-        if need_h:
-            g_h = torch.zeros(hbuf.shape, dtype=torch.float32, device=dev)
-            a.hsize = hbuf.shape[-1]  # grad_history is dense
-        sink = ctx.score_out
-        score = sink.tensor if isinstance(sink, ScoreSink) else sink
-        if score is not None and (inp.dim() == 3):
-            score = None
-        if not (need_in or need_ev or need_h or score is not None):
-            return (None,) * 12
-        if not gathered or need_h or score is not None:
-            with on_device(dev), _span(_tag("hc_aggr_bwd", inp), dev):
-                check(lib.hc_aggr_bwd(C.byref(a), ptr(grad_out), None if gathered else ptr(g_in), 1,
-                                      ptr(g_h), ptr(g_ev), ptr(score), ctx.score_kind, stream_of(dev)),
-                      "hc_aggr_bwd")
-            _called()
-        if score is not None and isinstance(sink, ScoreSink):
-            sink.fresh = True
-        if g_in is not None and g_in.dtype != inp.dtype:
-            g_in = g_in.to(inp.dtype)
-        if g_h is not None and g_h.dtype != hbuf.dtype:
-            g_h = g_h.to(hbuf.dtype)
-        return g_in, None, None, g_ev, None, g_h, None, None, None, None, None, None
-
-
 def aggr_forward(input, ptr, idx, num_node=0, *, history_map=None, history_buffer=None,
                  indexed=False, edge_value=None, src_map=None, src_alt=None, score_out=None,
                  score_kind=HC_SCORE_L2, force_grad=True):
@@ -257,20 +153,9 @@ def aggr_forward(input, ptr, idx, num_node=0, *, history_map=None, history_buffe
     With force_grad (the default) the result requires grad even when no input does
     (history_aggr.cu:604), which is what lets a caller retain_grad() it.
     """
-    if num_node == 0:
-        num_node = ptr.shape[0] - 1
-    if _empty(history_map) or _empty(history_buffer):
-        history_map = history_buffer = None
-    if _empty(edge_value):
-        edge_value = None
-    if _empty(src_map):
-        src_map = src_alt = None
-    out = _AggrFunction.apply(input, ptr, idx, edge_value, history_map, history_buffer,
-                              int(num_node), bool(indexed), src_map, src_alt, score_out,
-                              int(score_kind))
-    if force_grad and not out.requires_grad:
-        out.requires_grad_(True)
-    return out
+    return _native.aggr(input, ptr, idx, int(num_node), history_map, history_buffer, indexed, edge_value, src_map,
+                        src_alt, score_out, score_kind, force_grad, DETERMINISTIC_BWD, GATHER_MIN_BYTES,
+                        GATHER_MIN_FEAT)
 
 
 class PreparedAggr:
@@ -337,45 +222,19 @@ def transpose_block(p: PreparedAggr, max_edges):
     return t_ptr, t_dst, t_w
 
 
-_shared_t = {}
-_declared = {}
-
-
-def _graph_key(ptr_t, idx_t):
-    return (ptr_t.data_ptr(), idx_t.data_ptr(), ptr_t.shape[0], idx_t.shape[0], ptr_t._version, idx_t._version)
-
-
 def declare_batch(ptr_t, idx_t, n_nodes):
     """Tells the library that (ptr, idx) is the CSR of one sampled batch over `n_nodes` local ids
     that all layers aggregate over (layer k uses the rows [0, num_node_k)).  The backward passes
     of the batch can then share ONE transposition (see shared_transpose)."""
-    _declared[ptr_t.device] = (_graph_key(ptr_t, idx_t), int(n_nodes))
-    # a declaration opens a new batch: the same buffers may have been refilled by a library call
-    # (which leaves no trace in the tensors' version counters), and a step that is being captured
-    # must record its own transposition instead of borrowing the one of the warm-up
-    _shared_t.pop(ptr_t.device, None)
+    _native.declare_batch(ptr_t, idx_t, int(n_nodes))
 
 
 def shared_transpose(ptr_t, idx_t):
-    """Transposition of a declared batch's whole CSR, built once and reused by the backward pass of
-    every layer: all layers aggregate over a prefix of the same (ptr, idx), and a source's list is
-    sorted by destination row, so the list of a smaller layer is a prefix of it
+    """(t_ptr, t_dst, t_w, n_edges) of a declared batch's whole CSR, built once and reused by the
+    backward pass of every layer: all layers aggregate over a prefix of the same (ptr, idx), and a
+    source's list is sorted by destination row, so the list of a smaller layer is a prefix of it
     (hc_aggr_bwd_gather skips the rest).  None when (ptr, idx) was not declared."""
-    dev = ptr_t.device
-    key = _graph_key(ptr_t, idx_t)
-    decl = _declared.get(dev)
-    if decl is None or decl[0] != key:
-        return None
-    hit = _shared_t.get(dev)
-    if hit is not None and hit[0] == key:
-        return hit[1]
-    a = AggrArgs()
-    a.struct_size = C.sizeof(AggrArgs)
-    a.ptr, a.idx, a.num_node = ptr(ptr_t), ptr(idx_t), ptr_t.shape[0] - 1
-    a.feat, a.num_head, a.n_src = 4, 1, decl[1]
-    res = transpose_block(PreparedAggr(a, None, dev, ""), idx_t.shape[0]) + (int(idx_t.shape[0]),)
-    _shared_t[dev] = (key, res, (ptr_t, idx_t))   # the tensors stay alive with the entry
-    return res
+    return _native.shared_transpose(ptr_t, idx_t)
 
 
 def run_aggr_bwd_gather(p: PreparedAggr, t_ptr, t_dst, t_w, grad_out, grad_input, n_edges=None):
@@ -423,70 +282,13 @@ def aggr_forward_history_edge_value(input, ptr, idx, edge_value, history_map, hi
 # ---------------------------------------------------------------------------
 # batch norm + ReLU + dropout in one forward pair / one backward pair
 # ---------------------------------------------------------------------------
-def _norm_args(x, valid, weight, bias, rmean, rvar, momentum, eps, p, relu, seed, state, save):
-    a = _capi.NormArgs()
-    a.struct_size = C.sizeof(_capi.NormArgs)
-    a.x, a.n, a.feat, a.x_stride = ptr(x), x.shape[0], x.shape[1], x.stride(0) if x.shape[0] > 1 else x.shape[1]
-    a.valid, a.weight, a.bias = ptr(valid), ptr(weight), ptr(bias)
-    a.running_mean, a.running_var = ptr(rmean), ptr(rvar)
-    a.momentum, a.eps, a.drop_p, a.relu, a.seed = float(momentum), float(eps), float(p), 1 if relu else 0, int(seed)
-    a.state = ptr(state)
-    a.save_mean, a.save_rstd, a.save_count = ptr(save[0]), ptr(save[1]), ptr(save[2])
-    return a
-
-
-class _NormActFunction(torch.autograd.Function):
-
-    @staticmethod
-    def forward(ctx, x, weight, bias, valid, rmean, rvar, momentum, eps, p, relu, seed, state):
-        dev = require_cuda(x, weight, bias, valid, rmean, rvar, state)
-        x = rows2d(x)
-        if x.dtype != torch.float32 or x.dim() != 2:
-            raise TypeError("norm_act: x must be a float32 matrix")
-        if valid is not None:
-            valid = valid.contiguous()
-            if valid.dtype == torch.bool:
-                valid = valid.view(torch.uint8)
-            if valid.shape[0] < x.shape[0]:
-                raise RuntimeError("norm_act: row mask shorter than x")
-        feat = x.shape[1]
-        save = (torch.empty(feat, dtype=torch.float32, device=dev), torch.empty(feat, dtype=torch.float32, device=dev),
-                torch.empty(1, dtype=torch.float32, device=dev))
-        y = torch.empty((x.shape[0], feat), dtype=torch.float32, device=dev)
-        a = _norm_args(x, valid, weight, bias, rmean, rvar, momentum, eps, p, relu, seed, state, save)
-        sc = scratch(dev, lib.hc_norm_scratch_bytes(feat), "norm")
-        with on_device(dev), _span("hc_norm_act_fwd", dev):
-            check(lib.hc_norm_act_fwd(C.byref(a), ptr(y), ptr(sc), stream_of(dev)), "hc_norm_act_fwd")
-        _called(2)
-        ctx.save_for_backward(x, weight, bias, valid, state, *save)
-        ctx.cfg = (momentum, eps, p, relu, seed)
-        return y
-
-    @staticmethod
-    def backward(ctx, grad_y):
-        x, weight, bias, valid, state, sm, sr, scnt = ctx.saved_tensors
-        momentum, eps, p, relu, seed = ctx.cfg
-        dev = x.device
-        grad_y = grad_y.contiguous()
-        gx = torch.empty_like(x, memory_format=torch.contiguous_format)
-        gw = torch.empty_like(weight) if weight is not None and ctx.needs_input_grad[1] else None
-        gb = torch.empty_like(bias) if bias is not None and ctx.needs_input_grad[2] else None
-        a = _norm_args(x, valid, weight, bias, None, None, momentum, eps, p, relu, seed, state, (sm, sr, scnt))
-        sc = scratch(dev, lib.hc_norm_scratch_bytes(x.shape[1]), "norm")
-        with on_device(dev), _span("hc_norm_act_bwd", dev):
-            check(lib.hc_norm_act_bwd(C.byref(a), ptr(grad_y), ptr(gx), ptr(gw), ptr(gb), ptr(sc), stream_of(dev)),
-                  "hc_norm_act_bwd")
-        _called(2)
-        return gx, gw, gb, None, None, None, None, None, None, None, None, None
-
-
 def norm_act(x, weight, bias, state, *, valid=None, running_mean=None, running_var=None, momentum=0.1,
              eps=1e-5, p=0.0, relu=True, seed=0):
     """y = dropout(relu(batch_norm(x))) with batch statistics (training mode), as two kernels
     forward and two backward (csrc/norm_act.cu).  `state`: int64[4] CUDA tensor, zero-initialised
     once and private to the calling layer (dropout step counter).  `valid`: optional row mask."""
-    return _NormActFunction.apply(x, weight, bias, valid, running_mean, running_var, float(momentum),
-                                  float(eps), float(p), bool(relu), int(seed), state)
+    return _native.norm_act(x, weight, bias, state, valid, running_mean, running_var, momentum, eps, p, relu,
+                            seed & 0xFFFFFFFFFFFFFFFF)
 
 
 def norm_act_supported(x) -> bool:
