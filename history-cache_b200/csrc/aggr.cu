@@ -7,6 +7,8 @@
 // request, narrow rows are shared by several edges per request, and the
 // choice between a fresh source row, an alternative (cached) source row and a
 // history row is made inside the gather.  Memory bound: no tensor cores.
+#include <atomic>
+
 #include "common.cuh"
 
 namespace hc {
@@ -61,170 +63,416 @@ __global__ void __launch_bounds__(256) aggr_check_kernel(const hc_aggr_args a) {
 #define HC_BAIL_IF_BAD()
 #endif
 
-// ---------------------------------------------------------------------------
-// history row -> fp32 output row
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void copy_history_row(const hc_aggr_args& a, int64_t hrow, int head,
-                                                 float* __restrict__ orow, int lane, int h_vec) {
+// history row -> columns [v0 * EL, ...) of the fp32 output row
+template <int EL>
+__device__ __forceinline__ void copy_history_part(const hc_aggr_args& a, int64_t hrow, float* __restrict__ orow,
+                                                  int width, int v0, int v1, int lane, int h_vec) {
   const int F = a.feat;
-  const int64_t off = hrow * a.hsize + (a.hsize == F ? 0 : (int64_t)head * F);
+  const bool shared_row = a.hsize == F;      // one history row for all heads
+  const int c0 = v0 * EL, c1 = v1 * EL < width ? v1 * EL : width;
+  const int64_t base = hrow * a.hsize;
   if (h_vec) {
-    if (a.h_dtype == HC_F32) {
-      const float* src = reinterpret_cast<const float*>(a.hbuf) + off;
-      for (int v = lane; v < (F >> 2); v += kWarp)
-        reinterpret_cast<uint4*>(orow)[v] = ldg16(src + 4 * v);
-    } else {
-      const __half* src = reinterpret_cast<const __half*>(a.hbuf) + off;
-      for (int v = lane; v < (F >> 3); v += kWarp) {
-        float f[8];
-        Vec16<__half>::unpack(ldg16(src + 8 * v), f);
-        reinterpret_cast<float4*>(orow)[2 * v] = make_float4(f[0], f[1], f[2], f[3]);
-        reinterpret_cast<float4*>(orow)[2 * v + 1] = make_float4(f[4], f[5], f[6], f[7]);
+    for (int c = c0 + 4 * lane; c < c1; c += 4 * kWarp) {
+      const int64_t off = base + (shared_row ? c % F : c);
+      float4 o;
+      if (a.h_dtype == HC_F32) {
+        o = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.hbuf) + off);
+      } else {
+        LaneVec<__half, 8> h;
+        h.load(reinterpret_cast<const __half*>(a.hbuf) + off);
+        float f[4];
+        h.unpack(f);
+        o = make_float4(f[0], f[1], f[2], f[3]);
       }
+      *reinterpret_cast<float4*>(orow + c) = o;
     }
   } else {
-    for (int c = lane; c < F; c += kWarp) orow[c] = load_as_f32(a.hbuf, a.h_dtype, off + c);
+    for (int c = c0 + lane; c < c1; c += kWarp)
+      orow[c] = load_as_f32(a.hbuf, a.h_dtype, base + (shared_row ? c % F : c));
   }
 }
 
 // ---------------------------------------------------------------------------
-// forward, 16-byte vector path (num_head == 1)
-//   T   storage type of source rows
-//   G   lanes that share one source row (G < 32: 32/G edges per request)
-//   V   16-byte vectors per lane
-//   EV  weighted sum with edge values instead of mean
-//   IDX32  source ids fit 31 bits (n_src < 2^31): they travel in one shuffle
+// forward, rows of at least 4-byte units: a stream of edges through shared memory
+//   T    storage type of source rows
+//   VB   bytes per lane and request: 16 where rows allow it, else 8 or 4
+//   G    lanes that share one source row (G < 32: 32/G edges per request)
+//   V    vectors per lane; a row of more than G*V vectors is cut into column parts (gridDim.y)
+//   EV   0 mean, 1 sum weighted per edge, 2 sum weighted per edge and head
+//   MAP  per-source select between input and src_alt
 // ---------------------------------------------------------------------------
-// Tuning, measured on B200 with 2 M x 10-neighbour blocks larger than L2: throughput follows
-// the bytes in flight per SM (resident warps x U x 16 B per lane).  Six independent loads
-// per lane cover a sampled row (<= 12 edges of 256 B, <= 6 of 512 B) in one batch, and 48
-// registers keep five blocks resident; more unrolling or forcing more blocks spills and
-// loses (U=4: 4.3 TB/s, U=6 @5 blocks: 5.1 TB/s, U=8: 3.8 TB/s for fp16 dim-128 rows).
-// Two other layouts were built and measured on the same block and lost: staging each block's
-// idx slice in shared memory with one lane group per row (3.7 TB/s), and fetching every
-// source row with the bulk-copy engine into a double-buffered shared-memory ring (4.1 TB/s:
-// the engine tops out near 13 G row copies/s, below the 16 G rows/s the register path moves).
-#ifndef HC_FWD_MINBLOCKS
-#define HC_FWD_MINBLOCKS 5
-#endif
-#ifndef HC_FWD_U1
-#define HC_FWD_U1 6
-#endif
-//   MH  several heads: a warp owns one (row, head) target; with MH == false the head arithmetic
-//       folds away and the kernel is the single-head one
-template <typename T, int G, int V, bool EV, bool IDX32, bool MH = false>
-__global__ void __launch_bounds__(256, HC_FWD_MINBLOCKS)
-    aggr_fwd_vec_kernel(const hc_aggr_args a, float* __restrict__ out, const int nvec,
-                        const int h_vec) {
+// A destination row costs three dependent memory latencies: ptr -> idx -> source rows.  A warp per
+// row has its bytes in flight during the last of them only, and more unrolling did not help (ragged
+// rows of 10 edges of 256 B: 370 us with 6 loads in flight per lane and 40 warps, 415 with 8 and 32:
+// the time followed the number of warps).  Here a warp owns a run of consecutive rows, whose edges
+// are one contiguous slice of idx, and walks them as a stream: asynchronous copies keep D requests in
+// flight at all times, across row boundaries, while the oldest is added up; idx comes in chunks of 32,
+// one chunk ahead.  A lane copies and reads back only its own bytes, so the ring needs no barrier.
+// Measured, start -> now: 500 K ragged rows, 5 M edges of 256 B (fp16) out of 2 M rows 370 -> 231 us
+// (1.58 GB gathered, read and written: 6.8 TB/s, a tenth of the gathers hit the L2); 200 K rows, 1.8 M
+// skewed edges of 1 KB 294 -> 243 us; 100 K rows, 1 M edges with weights for 4 heads of 64 285 -> 175 us;
+// 60 K rows, 720 K edges of 75 fp32 columns 112 -> 62 us (was the scalar kernel).
+// Two requests per slot halve the walking (row switches, ring, commit) per edge: with one the issue
+// slots were 84 % busy at 5.5 TB/s.  Ring size and blocks per SM are what the sweep over U = 1..4,
+// 4 / 6 / 8 KB per warp and 3..5 blocks left (weighted sums, which also load weights through the L1,
+// want the fourth block).
+template <int VB, int V, int EV>
+struct StreamShape {
+  static constexpr int U = 2;                                             // requests per slot
+  static constexpr int kReq = V * VB * kWarp;                             // bytes of one request of the warp
+  static constexpr int kSlot = U * kReq;
+  static constexpr int kRing = EV ? 6144 : 8192;
+  static constexpr int D = kRing / kSlot < 3 ? 3 : (kRing / kSlot > 8 ? 8 : kRing / kSlot);   // slots in flight
+  static constexpr int kWarpBytes = D * kSlot + 64 * 8;                   // + ring of row addresses
+  static constexpr int kSmem = 8 * kWarpBytes;
+  static constexpr int kFit = 220 * 1024 / (kSmem + 1024);
+  static constexpr int kMinBlocks = kFit < (EV ? 4 : 3) ? kFit : (EV ? 4 : 3);
+};
+constexpr int kMaxRun = 31;      // rows of a run: one ptr entry per lane
+
+template <typename T, int VB, int G, int V, int EV, bool MAP>
+__global__ void __launch_bounds__(256, (StreamShape<VB, V, EV>::kMinBlocks))
+    aggr_fwd_stream_kernel(const hc_aggr_args a, float* __restrict__ out, const int nvec, const int part_vec,
+                           const int h_vec, const int stream_out, const int run_rows) {
   HC_BAIL_IF_BAD()
-  constexpr int EL = Vec16<T>::kElems;
+  using Vec = LaneVec<T, VB>;
+  using Shape = StreamShape<VB, V, EV>;
+  constexpr int EL = Vec::kElems;
   constexpr int EPW = kWarp / G;
-  constexpr int U = V == 1 ? HC_FWD_U1 : (V == 2 ? 4 : (V <= 4 ? 2 : 1));
-  const int lane = threadIdx.x & 31;
-  const int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int H = MH ? a.num_head : 1;
-  if (t >= a.num_node * H) return;
-  const int64_t r = MH ? t / H : t;
-  const int h = MH ? (int)(t - r * H) : 0;
-  const int F = a.feat;
-  float* __restrict__ orow = out + t * F;
-
-  const int64_t hid = a.hmap ? a.hmap[r] : -1;
-  if (hid != -1) {
-    copy_history_row(a, a.h_indexed ? hid : r, h, orow, lane, h_vec);
-    return;
-  }
-
+  constexpr int D = Shape::D, U = Shape::U;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned char* mine = smem + (size_t)warp * Shape::kWarpBytes + lane * VB;
+  const uint32_t mine_s = smem_u32(mine);
+  unsigned long long* ring = reinterpret_cast<unsigned long long*>(smem + (size_t)warp * Shape::kWarpBytes + D * Shape::kSlot);
+  const int H = a.num_head;
+  const int width = H * a.feat;
+  const int v0 = blockIdx.y * part_vec;                       // this block's columns of the row
+  const int v1 = v0 + part_vec < nvec ? v0 + part_vec : nvec;
   const int sub = lane / G, gl = lane % G;
-  float acc[V][EL];
+  const char* __restrict__ in = reinterpret_cast<const char*>(a.input);
+  const char* __restrict__ alt = reinterpret_cast<const char*>(a.src_alt);
+  const int64_t in_bytes = a.in_stride * (int64_t)sizeof(T), alt_bytes = a.alt_stride * (int64_t)sizeof(T);
+  const uint64_t policy = l2_policy(stream_out != 0);
+  int head[V];
 #pragma unroll
-  for (int k = 0; k < V; ++k)
-#pragma unroll
-    for (int e = 0; e < EL; ++e) acc[k][e] = 0.f;
+  for (int k = 0; k < V; ++k) head[k] = EV == 2 ? (v0 + gl + k * G) * EL / a.feat : 0;
 
-  const int64_t begin = a.ptr[r], end = a.ptr[r + 1];
-  const T* __restrict__ in = reinterpret_cast<const T*>(a.input) + (MH ? (int64_t)h * F : 0);
-  const T* __restrict__ alt = reinterpret_cast<const T*>(a.src_alt) + (MH ? (int64_t)h * F : 0);
-  const bool has_map = a.src_map != nullptr;
-
-  for (int64_t i = begin; i < end; i += kWarp) {
-    int64_t my_s = 0, my_alt = -1;
-    float my_w = 0.f;
-    if (i + lane < end) {
-      my_s = a.idx[i + lane];
-      if (has_map) my_alt = a.src_map[my_s];
-      if (EV) my_w = MH ? a.edge_value[(i + lane) * H + h] : a.edge_value[i + lane];
+  const int64_t runs = ceil_div(a.num_node, run_rows);
+  const int64_t step = (int64_t)gridDim.x * 8;
+  int64_t run = (int64_t)blockIdx.x * 8 + warp;
+  int64_t my_p = 0, my_h = -1;      // lane l: ptr and history entry of row l of the run
+  auto fetch_run = [&](int64_t q) {
+    const int64_t row = q * run_rows + lane;
+    my_p = 0;
+    my_h = -1;
+    if (q < runs && lane <= run_rows && row <= a.num_node) {
+      my_p = a.ptr[row];
+      if (a.hmap && lane < run_rows && row < a.num_node) my_h = a.hmap[row];
     }
-    const int cnt = (int)((end - i) < (int64_t)kWarp ? (end - i) : (int64_t)kWarp);
-    for (int j = 0; j < cnt; j += EPW * U) {
-      uint4 buf[U][V];
-      float w[U];
+  };
+  fetch_run(run);
+  for (; run < runs; run += step) {
+    const int64_t r0 = run * run_rows;
+    const int nr = (int)(a.num_node - r0 < run_rows ? a.num_node - r0 : run_rows);
+    const int64_t e0 = shfl64(my_p, 0);
+    const int off = (int)(my_p - e0);                // lane l <= nr: first edge of row l of the run
+    const int64_t hrow = my_h;
+    const unsigned miss = __ballot_sync(kFull, lane < nr && my_h == -1);
+    const unsigned hits = __ballot_sync(kFull, lane < nr && my_h != -1);
+    const int total = __shfl_sync(kFull, off, nr);
+    int64_t next_i = lane < total ? a.idx[e0 + lane] : 0;      // chunk [loaded, loaded + 32) of the run's edges
+    fetch_run(run + step);                                     // in flight during this run
+    int loaded = 0;
+    // producer: edge pe of a row that ends at pend, rows left in pm
+    unsigned pm = miss;
+    int pe = 0, pend = 0;
+    auto produce = [&](int slot) {
+      while (pe >= pend && pm) {
+        const int row = __ffs(pm) - 1;
+        pm &= pm - 1;
+        pe = __shfl_sync(kFull, off, row);
+        pend = __shfl_sync(kFull, off, row + 1);
+      }
+      if (pe < pend) {
+        const int need = pe + U * EPW < pend ? pe + U * EPW : pend;
+        if (pe >= loaded + kWarp) {      // rows served from history were skipped
+          loaded = pe & ~31;
+          next_i = loaded + lane < total ? a.idx[e0 + loaded + lane] : 0;
+        }
+        while (need > loaded) {
+          const char* p = in + next_i * in_bytes;
+          if (MAP && loaded + lane < total) {
+            const int64_t m = a.src_map[next_i];
+            if (m != -1) p = alt + m * alt_bytes;
+          }
+          __syncwarp();
+          ring[(loaded + lane) & 63] = reinterpret_cast<unsigned long long>(p);
+          __syncwarp();
+          loaded += kWarp;
+          next_i = loaded + lane < total ? a.idx[e0 + loaded + lane] : 0;
+        }
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int jj = j + u * EPW + sub;
-        const int from = jj & 31;
-        const int64_t s = IDX32 ? (int64_t)__shfl_sync(kFull, (int)my_s, from) : shfl64(my_s, from);
-        const int64_t al = has_map ? shfl64(my_alt, from) : -1;
-        w[u] = EV ? __shfl_sync(kFull, my_w, from) : 1.f;
-        const bool ok = jj < cnt;
-        if (EV && !ok) w[u] = 0.f;
-        const T* row = (al != -1) ? alt + al * a.alt_stride : in + s * a.in_stride;
+        for (int u = 0; u < U; ++u) {
+          const int e = pe + u * EPW + sub;
+          if (e < pend) {
+            const char* p = reinterpret_cast<const char*>(ring[e & 63]);
+            const uint32_t dst = mine_s + slot * Shape::kSlot + u * Shape::kReq;
+#pragma unroll
+            for (int k = 0; k < V; ++k) {
+              const int v = v0 + gl + k * G;
+              if (v < v1) cp_async<VB>(dst + k * VB * kWarp, p + v * VB);
+            }
+          }
+        }
+        pe += U * EPW;
+      }
+      cp_async_commit();
+    };
+#pragma unroll 1
+    for (int d = 0; d < D; ++d) produce(d);
+    for (unsigned h = hits; h; h &= h - 1) {
+      const int row = __ffs(h) - 1;
+      const int64_t hr = shfl64(hrow, row);
+      copy_history_part<EL>(a, a.h_indexed ? hr : r0 + row, out + (r0 + row) * width, width, v0, v1, lane, h_vec);
+    }
+    int slot = 0;
+    for (unsigned m = miss; m; m &= m - 1) {
+      const int row = __ffs(m) - 1;
+      const int b = __shfl_sync(kFull, off, row), end = __shfl_sync(kFull, off, row + 1);
+      float acc[V][EL];
+#pragma unroll
+      for (int k = 0; k < V; ++k)
+#pragma unroll
+        for (int q = 0; q < EL; ++q) acc[k][q] = 0.f;
+#pragma unroll 1
+      for (int e = b; e < end; e += U * EPW) {
+        float w[U][EV == 2 ? V : 1];     // neighbouring edges' weights share lines of the L1
+        if (EV) {
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int k = 0; k < (EV == 2 ? V : 1); ++k) {
+              const int64_t ee = e0 + e + u * EPW + sub;
+              w[u][k] = e + u * EPW + sub < end ? __ldg(a.edge_value + (EV == 2 ? ee * H + head[k] : ee)) : 0.f;
+            }
+        }
+        cp_async_wait<D - 1>();
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (e + u * EPW + sub < end) {
+            const int at = slot * Shape::kSlot + u * Shape::kReq;
+#pragma unroll
+            for (int k = 0; k < V; ++k) {
+              if (v0 + gl + k * G < v1) {
+                Vec x;
+                x.load_shared(mine + at + k * VB * kWarp);
+                if (EV) {
+                  float f[EL];
+                  x.unpack(f);
+#pragma unroll
+                  for (int q = 0; q < EL; ++q) acc[k][q] = fmaf(w[u][EV == 2 ? k : 0], f[q], acc[k][q]);
+                } else {
+                  x.add_to(acc[k]);
+                }
+              }
+            }
+          }
+        }
+        produce(slot);
+        slot = slot + 1 == D ? 0 : slot + 1;
+      }
+      if (EPW > 1) {
+#pragma unroll
+        for (int o = G; o < kWarp; o <<= 1)
+#pragma unroll
+          for (int k = 0; k < V; ++k)
+#pragma unroll
+            for (int q = 0; q < EL; ++q) acc[k][q] += __shfl_xor_sync(kFull, acc[k][q], o);
+      }
+      if (sub == 0) {
+        float* orow = out + (r0 + row) * width;
+        if (!EV && end > b) {
+          const float inv = __frcp_rn((float)(end - b));  // one correctly rounded reciprocal per row
+#pragma unroll
+          for (int k = 0; k < V; ++k)
+#pragma unroll
+            for (int q = 0; q < EL; ++q) acc[k][q] *= inv;
+        }
 #pragma unroll
         for (int k = 0; k < V; ++k) {
-          const int v = gl + k * G;
-          buf[u][k] = (ok && v < nvec) ? ldg16(row + v * EL) : make_uint4(0u, 0u, 0u, 0u);
+          const int v = v0 + gl + k * G;
+          if (v < v1) store_f32<EL>(orow + v * EL, acc[k], policy);
         }
       }
+    }
+    cp_async_wait<0>();
+  }
+}
+
+// ---------------------------------------------------------------------------
+// forward, fp16 rows on odd 2-byte addresses: no asynchronous copy is that narrow, so the rows come
+// through registers, U requests at a time; while they are on their way the warp loads the indices of
+// its next row and the ptr / history entries of the one after.
+// ---------------------------------------------------------------------------
+template <int VB, int V>
+struct FwdShape {
+  static constexpr int words = (VB >= 4 ? VB / 4 : 1) * V;            // registers of one row per lane
+  static constexpr int U = words >= 8 ? 4 : 8;                        // rows in flight per lane group
+  static constexpr int kMinBlocks = words * U >= 32 ? 4 : 5;
+};
+
+template <typename T, int VB, int G, int V, int EV, bool MAP>
+__global__ void __launch_bounds__(256, (FwdShape<VB, V>::kMinBlocks))
+    aggr_fwd_kernel(const hc_aggr_args a, float* __restrict__ out, const int nvec, const int part_vec,
+                    const int h_vec, const int stream_out) {
+  HC_BAIL_IF_BAD()
+  using Vec = LaneVec<T, VB>;
+  constexpr int EL = Vec::kElems;
+  constexpr int EPW = kWarp / G;
+  constexpr int U = FwdShape<VB, V>::U;
+  const int lane = threadIdx.x & 31;
+  const int64_t step = (int64_t)gridDim.x * (blockDim.x >> 5);
+  int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (r >= a.num_node) return;
+  const int H = a.num_head;
+  const int width = H * a.feat;
+  const int v0 = blockIdx.y * part_vec;                       // this block's columns of the row
+  const int v1 = v0 + part_vec < nvec ? v0 + part_vec : nvec;
+  const int sub = lane / G, gl = lane % G;
+  const T* __restrict__ in = reinterpret_cast<const T*>(a.input);
+  const T* __restrict__ alt = reinterpret_cast<const T*>(a.src_alt);
+  const uint64_t policy = l2_policy(stream_out != 0);
+  int head[V];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (j + u * EPW < cnt) {  // warp-uniform: slots past the end of the chunk do nothing
+  for (int k = 0; k < V; ++k) head[k] = EV == 2 ? (v0 + gl + k * G) * EL / a.feat : 0;
+
+  // what is known of a row ahead of time, one value per lane: ptr[r], ptr[r + 1], hmap[r]
+  auto row_meta = [&](int64_t row) -> int64_t {
+    if (row < a.num_node) {
+      if (lane < 2) return a.ptr[row + lane];
+      if (lane == 2 && a.hmap) return a.hmap[row];
+    }
+    return lane < 2 ? 0 : -1;
+  };
+  int64_t meta = row_meta(r), meta_n = row_meta(r + step);
+  uint32_t my_s = 0u;
+  {   // the shuffles stand outside the condition: every lane takes part in them
+    const int64_t at = shfl64(meta, 0) + lane, end = shfl64(meta, 1), hit = shfl64(meta, 2);
+    if (at < end && hit == -1) my_s = (uint32_t)a.idx[at];
+  }
+  while (true) {
+    const int64_t b = shfl64(meta, 0), e = shfl64(meta, 1), hid = shfl64(meta, 2);
+    float acc[V][EL];
 #pragma unroll
-          for (int k = 0; k < V; ++k) {
-            if (EV) {
-              float f[EL];
-              Vec16<T>::unpack(buf[u][k], f);
+    for (int k = 0; k < V; ++k)
 #pragma unroll
-              for (int e = 0; e < EL; ++e) acc[k][e] = fmaf(w[u], f[e], acc[k][e]);
-            } else {
-              accumulate_vec<T>(acc[k], buf[u][k]);
+      for (int q = 0; q < EL; ++q) acc[k][q] = 0.f;
+    uint32_t next_s = 0u;
+    int64_t meta_2 = -1;
+    bool fetched = false;
+    // what the following rows need, issued behind the first batch of this row's loads
+    auto fetch_next = [&]() {
+      if (fetched) return;
+      fetched = true;
+      const int64_t at = shfl64(meta_n, 0) + lane, end = shfl64(meta_n, 1), hit = shfl64(meta_n, 2);
+      if (at < end && hit == -1) next_s = (uint32_t)a.idx[at];
+      meta_2 = row_meta(r + 2 * step);
+    };
+    float* __restrict__ orow = out + r * width;
+    if (hid == -1) {
+      for (int64_t i = b; i < e; i += kWarp) {
+        const int cnt = (int)((e - i) < (int64_t)kWarp ? (e - i) : (int64_t)kWarp);
+        if (i != b) my_s = i + lane < e ? (uint32_t)a.idx[i + lane] : 0u;
+        bool my_alt = false;
+        if (MAP && lane < cnt) {
+          const int64_t m = a.src_map[my_s];
+          my_alt = m != -1;
+          if (my_alt) my_s = (uint32_t)m;
+        }
+        float my_w = 0.f;
+        if (EV == 1 && lane < cnt) my_w = a.edge_value[i + lane];
+        const unsigned alts = MAP ? __ballot_sync(kFull, my_alt) : 0u;
+        for (int j = 0; j < cnt; j += EPW * U) {
+          Vec buf[U][V];
+          float w[U][EV == 2 ? V : 1];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            if (j + u * EPW < cnt) {  // warp-uniform
+              const int jj = j + u * EPW + sub;
+              const bool ok = jj < cnt;
+              const uint32_t s = __shfl_sync(kFull, my_s, jj & 31);
+              if (EV == 1) w[u][0] = __shfl_sync(kFull, my_w, jj & 31);   // lanes behind cnt hold 0
+              const T* row = (MAP && ((alts >> (jj & 31)) & 1u)) ? alt + (int64_t)s * a.alt_stride
+                                                                 : in + (int64_t)s * a.in_stride;
+#pragma unroll
+              for (int k = 0; k < V; ++k) {
+                const int v = v0 + gl + k * G;
+                buf[u][k].clear();
+                if (EV == 2) w[u][k] = 0.f;
+                if (ok && v < v1) {
+                  buf[u][k].load(row + v * EL);
+                  if (EV == 2) w[u][k] = __ldg(a.edge_value + (i + jj) * H + head[k]);
+                }
+              }
+            }
+          }
+          fetch_next();
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            if (j + u * EPW < cnt) {
+#pragma unroll
+              for (int k = 0; k < V; ++k) {
+                if (EV) {
+                  float f[EL];
+                  buf[u][k].unpack(f);
+#pragma unroll
+                  for (int q = 0; q < EL; ++q) acc[k][q] = fmaf(w[u][EV == 2 ? k : 0], f[q], acc[k][q]);
+                } else {
+                  buf[u][k].add_to(acc[k]);
+                }
+              }
             }
           }
         }
       }
+      fetch_next();      // a row without edges
+      if (EPW > 1) {
+#pragma unroll
+        for (int off = G; off < kWarp; off <<= 1)
+#pragma unroll
+          for (int k = 0; k < V; ++k)
+#pragma unroll
+            for (int q = 0; q < EL; ++q) acc[k][q] += __shfl_xor_sync(kFull, acc[k][q], off);
+      }
+      if (sub == 0) {
+        if (!EV && e > b) {
+          const float inv = __frcp_rn((float)(e - b));  // one correctly rounded reciprocal per row
+#pragma unroll
+          for (int k = 0; k < V; ++k)
+#pragma unroll
+            for (int q = 0; q < EL; ++q) acc[k][q] *= inv;
+        }
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+          const int v = v0 + gl + k * G;
+          if (v < v1) store_f32<EL>(orow + v * EL, acc[k], policy);
+        }
+      }
+    } else {
+      fetch_next();
+      copy_history_part<EL>(a, a.h_indexed ? hid : r, orow, width, v0, v1, lane, h_vec);
     }
-  }
-
-  if (EPW > 1) {
-#pragma unroll
-    for (int off = G; off < kWarp; off <<= 1)
-#pragma unroll
-      for (int k = 0; k < V; ++k)
-#pragma unroll
-        for (int e = 0; e < EL; ++e) acc[k][e] += __shfl_xor_sync(kFull, acc[k][e], off);
-  }
-  if (sub != 0) return;
-
-  const int64_t deg = end - begin;
-  if (!EV && deg > 0) {
-    const float inv = __frcp_rn((float)deg);  // one correctly rounded reciprocal per row
-#pragma unroll
-    for (int k = 0; k < V; ++k)
-#pragma unroll
-      for (int e = 0; e < EL; ++e) acc[k][e] *= inv;
-  }
-#pragma unroll
-  for (int k = 0; k < V; ++k) {
-    const int v = gl + k * G;
-    if (v < nvec) {
-      float4* dst = reinterpret_cast<float4*>(orow + v * EL);
-      dst[0] = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
-      if (EL == 8) dst[1] = make_float4(acc[k][EL - 4], acc[k][EL - 3], acc[k][EL - 2], acc[k][EL - 1]);
-    }
+    r += step;
+    if (r >= a.num_node) return;
+    meta = meta_n;
+    meta_n = meta_2;
+    my_s = next_s;
   }
 }
 
 // ---------------------------------------------------------------------------
-// forward, generic path: any F, any dtype mix, multi-head
+// forward, generic path: any dtype mix, source ids beyond 32 bits, odd widths with weights per head
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
     aggr_fwd_generic_kernel(const hc_aggr_args a, float* __restrict__ out) {
@@ -238,7 +486,8 @@ __global__ void __launch_bounds__(256)
   float* __restrict__ orow = out + t * F;
   const int64_t hid = a.hmap ? a.hmap[r] : -1;
   if (hid != -1) {
-    copy_history_row(a, a.h_indexed ? hid : r, h, orow, lane, 0);
+    const int64_t off = (a.h_indexed ? hid : r) * a.hsize + (a.hsize == F ? 0 : (int64_t)h * F);
+    for (int c = lane; c < F; c += kWarp) orow[c] = load_as_f32(a.hbuf, a.h_dtype, off + c);
     return;
   }
   const int64_t begin = a.ptr[r], end = a.ptr[r + 1];
@@ -515,33 +764,105 @@ static int vec_shape(int nvec, int* G, int* V) {
   return 1;
 }
 
-// several heads (edge-weighted sums only; source ids must fit 31 bits)
-template <typename T>
-static void launch_fwd_heads(int G, int V, dim3 grid, cudaStream_t st, const hc_aggr_args& a,
-                             float* out, int nvec, int h_vec) {
-#define HC_FWD_CASE(g, v)                                                                          \
-  if (G == g && V == v) {                                                                          \
-    aggr_fwd_vec_kernel<T, g, v, true, true, true><<<grid, 256, 0, st>>>(a, out, nvec, h_vec);     \
-    return;                                                                                        \
-  }
-  HC_FWD_CASE(8, 1) HC_FWD_CASE(16, 1) HC_FWD_CASE(32, 1) HC_FWD_CASE(32, 2)
-  HC_FWD_CASE(32, 3) HC_FWD_CASE(32, 4) HC_FWD_CASE(32, 6) HC_FWD_CASE(32, 8)
-#undef HC_FWD_CASE
+// Raises a kernel's shared-memory limit, once per kernel (`done` is its own) and device; not a stream
+// operation, so it may happen during a capture.
+template <typename K>
+static void raise_smem(K kernel, int bytes, std::atomic<uint64_t>& done) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev > 63) dev = 63;
+  if (done.load(std::memory_order_relaxed) >> dev & 1) return;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
+    done.fetch_or(1ull << dev, std::memory_order_relaxed);
 }
 
-template <typename T, bool EV>
-static void launch_fwd_vec(int G, int V, dim3 grid, cudaStream_t st, const hc_aggr_args& a,
-                           float* out, int nvec, int h_vec) {
-  const bool idx32 = a.n_src < 0x7fffffffLL;
-#define HC_FWD_CASE(g, v)                                                                     \
-  if (G == g && V == v) {                                                                     \
-    if (idx32) aggr_fwd_vec_kernel<T, g, v, EV, true><<<grid, 256, 0, st>>>(a, out, nvec, h_vec);  \
-    else aggr_fwd_vec_kernel<T, g, v, EV, false><<<grid, 256, 0, st>>>(a, out, nvec, h_vec);  \
-    return;                                                                                   \
+// Widest unit (16, 8, 4 or 2 bytes) that divides every given address or length; never below `es`.
+static int lane_bytes(uintptr_t bits, int es) {
+  for (int vb = 16; vb > es; vb >>= 1)
+    if (bits % vb == 0) return vb;
+  return es;
+}
+
+struct FwdLaunch {
+  hc_aggr_args a;
+  float* out;
+  int nvec, h_vec, stream_out;
+  cudaStream_t st;
+};
+
+struct FwdGrid {
+  dim3 grid;
+  int part_vec, run_rows;
+};
+// column parts of about equal width that start on a float4 of the output row, and one wave of blocks
+static FwdGrid fwd_grid(const FwdLaunch& l, int el, int most_vec, int min_blocks, int max_run) {
+  FwdGrid g;
+  const int parts = (int)ceil_div(l.nvec, most_vec);
+  const int unit = el < 4 ? 4 / el : 1;
+  g.part_vec = (int)ceil_div(ceil_div(l.nvec, parts), unit) * unit;
+  if (g.part_vec > most_vec) g.part_vec = most_vec;           // most_vec is a multiple of 4
+  g.grid.y = (unsigned)ceil_div(l.nvec, g.part_vec);
+  int64_t most = 148 * min_blocks / g.grid.y;
+  if (most < 1) most = 1;
+  // every warp gets the same number of runs, as long as they may be: a short run leaves the start of its
+  // pipeline uncovered
+  const int64_t per_warp = ceil_div(l.a.num_node, most * 8);
+  const int64_t run = ceil_div(per_warp, ceil_div(per_warp, max_run));
+  const int64_t blocks = ceil_div(ceil_div(l.a.num_node, run), 8);
+  g.run_rows = (int)run;
+  g.grid.x = (unsigned)(blocks < most ? blocks : most);
+  return g;
+}
+
+template <typename T, int VB, int G, int V, int EV, bool MAP>
+static void launch_fwd_one(const FwdLaunch& l) {
+  if constexpr (VB == 2) {
+    const FwdGrid g = fwd_grid(l, 1, G * V, FwdShape<VB, V>::kMinBlocks, 1);
+    aggr_fwd_kernel<T, VB, G, V, EV, MAP><<<g.grid, 256, 0, l.st>>>(l.a, l.out, l.nvec, g.part_vec, l.h_vec, l.stream_out);
+  } else {
+    using Shape = StreamShape<VB, V, EV>;
+    auto kernel = aggr_fwd_stream_kernel<T, VB, G, V, EV, MAP>;
+    static std::atomic<uint64_t> raised{0};
+    if (Shape::kSmem > 48 * 1024) raise_smem(kernel, Shape::kSmem, raised);
+    const FwdGrid g = fwd_grid(l, LaneVec<T, VB>::kElems, G * V, Shape::kMinBlocks, kMaxRun);
+    kernel<<<g.grid, 256, Shape::kSmem, l.st>>>(l.a, l.out, l.nvec, g.part_vec, l.h_vec, l.stream_out, g.run_rows);
   }
-  HC_FWD_CASE(8, 1) HC_FWD_CASE(16, 1) HC_FWD_CASE(32, 1) HC_FWD_CASE(32, 2)
-  HC_FWD_CASE(32, 3) HC_FWD_CASE(32, 4) HC_FWD_CASE(32, 6) HC_FWD_CASE(32, 8)
-#undef HC_FWD_CASE
+}
+
+template <typename T, int EV, bool MAP>
+static void launch_fwd_wide(const FwdLaunch& l) {
+  if (l.nvec <= 8) launch_fwd_one<T, 16, 8, 1, EV, MAP>(l);
+  else if (l.nvec <= 16) launch_fwd_one<T, 16, 16, 1, EV, MAP>(l);
+  else if (l.nvec <= 32) launch_fwd_one<T, 16, 32, 1, EV, MAP>(l);
+  else launch_fwd_one<T, 16, 32, 2, EV, MAP>(l);
+}
+template <typename T, int VB, int EV>
+static void launch_fwd_narrow(const FwdLaunch& l) {
+  if (l.nvec <= 16) launch_fwd_one<T, VB, 16, 1, EV, false>(l);
+  else if (l.nvec <= 32) launch_fwd_one<T, VB, 32, 1, EV, false>(l);
+  else if (l.nvec <= 64) launch_fwd_one<T, VB, 32, 2, EV, false>(l);
+  else if (l.nvec <= 96) launch_fwd_one<T, VB, 32, 3, EV, false>(l);
+  else launch_fwd_one<T, VB, 32, 4, EV, false>(l);
+}
+template <typename T, int EV>
+static bool launch_fwd_any(const FwdLaunch& l, int vb) {
+  if (vb == 16) {
+    if (l.a.src_map) launch_fwd_wide<T, EV, true>(l);
+    else launch_fwd_wide<T, EV, false>(l);
+    return true;
+  }
+  if constexpr (EV != 2) {
+    if (l.a.src_map) return false;
+    if (vb == 8) launch_fwd_narrow<T, 8, EV>(l);
+    else if (vb == 4) launch_fwd_narrow<T, 4, EV>(l);
+    else if constexpr (sizeof(T) == 2) launch_fwd_narrow<T, 2, EV>(l);
+    return true;
+  }
+  return false;
+}
+template <typename T>
+static bool launch_fwd(const FwdLaunch& l, int vb) {
+  if (!l.a.edge_value) return launch_fwd_any<T, 0>(l, vb);
+  return l.a.num_head == 1 ? launch_fwd_any<T, 1>(l, vb) : launch_fwd_any<T, 2>(l, vb);
 }
 
 template <bool EV>
@@ -623,41 +944,36 @@ extern "C" int hc_aggr_fwd(const hc_aggr_args* args, float* out, void* stream) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   HC_CHECK_BLOCK(a, st);
   const int s = dtype_size(a.in_dtype);
-  const int64_t row_bytes = (int64_t)a.feat * s;
-  const bool out_vec = aligned16(out) && a.feat % 4 == 0;
-  int h_vec = 0;
+  // The vector kernels take rows of one storage type and source ids of 32 bits.  The unit that a lane
+  // moves has to divide a row's length and every row's address, and with weights per head it may not
+  // straddle two heads.
+  const int64_t width = (int64_t)a.num_head * a.feat;
+  const bool per_head = a.edge_value != nullptr && a.num_head > 1;
+  uintptr_t bits = reinterpret_cast<uintptr_t>(a.input) | (uintptr_t)(a.in_stride * s) |
+                   (uintptr_t)((per_head ? a.feat : width) * s);
+  bool vec = width * s <= (1 << 20) && a.n_src <= 0xffffffffLL;
+  if (a.src_map) {
+    vec = vec && a.alt_dtype == a.in_dtype;
+    bits |= reinterpret_cast<uintptr_t>(a.src_alt) | (uintptr_t)(a.alt_stride * s);
+  }
+  int vb = lane_bytes(bits, s);
+  while (vb > s && !aligned_to(out, (size_t)(vb / s * 4 < 16 ? vb / s * 4 : 16))) vb >>= 1;
+  FwdLaunch l;
+  l.a = a;
+  l.out = out;
+  l.st = st;
+  l.nvec = (int)(width * s / vb);
+  // results of more than half the L2 are not read from it again
+  l.stream_out = a.num_node * width * 4 > (64 << 20);
+  l.h_vec = 0;
   if (a.hmap) {
     const int hs = dtype_size(a.h_dtype);
-    h_vec = out_vec && aligned16(a.hbuf) && (a.hsize * hs) % 16 == 0 && ((int64_t)a.feat * hs) % 16 == 0;
+    l.h_vec = aligned16(out) && a.feat % 4 == 0 && aligned_to(a.hbuf, 4 * hs) && a.hsize % 4 == 0;
   }
-  // several heads take the vector path when they are an edge-weighted sum (the only multi-head
-  // operator of the reference, history_aggr.cu:80-125) and source ids fit 31 bits
-  const bool heads = a.num_head > 1;
-  bool vec = (!heads || (a.edge_value != nullptr && a.n_src < 0x7fffffffLL)) && out_vec &&
-             row_bytes % 16 == 0 && aligned16(a.input) && (a.in_stride * s) % 16 == 0;
-  if (vec && a.src_map)
-    vec = a.alt_dtype == a.in_dtype && aligned16(a.src_alt) && (a.alt_stride * s) % 16 == 0;
-  if (vec && a.edge_value) vec = aligned_to(a.edge_value, 4);
-  int G = 0, V = 0;
-  const int nvec = (int)(row_bytes / 16);
-  if (vec) vec = vec_shape(nvec, &G, &V) != 0;
-  const int64_t targets = a.num_node * a.num_head;
-  const int64_t blocks = ceil_div(targets, 8);
-  HC_REQUIRE(blocks <= 0x7fffffffLL, HC_ERR_SIZE);
-  dim3 grid((unsigned)blocks);
-  if (vec && heads) {
-    if (a.in_dtype == HC_F32) launch_fwd_heads<float>(G, V, grid, st, a, out, nvec, h_vec);
-    else launch_fwd_heads<__half>(G, V, grid, st, a, out, nvec, h_vec);
-  } else if (vec) {
-    if (a.in_dtype == HC_F32) {
-      if (a.edge_value) launch_fwd_vec<float, true>(G, V, grid, st, a, out, nvec, h_vec);
-      else launch_fwd_vec<float, false>(G, V, grid, st, a, out, nvec, h_vec);
-    } else {
-      if (a.edge_value) launch_fwd_vec<__half, true>(G, V, grid, st, a, out, nvec, h_vec);
-      else launch_fwd_vec<__half, false>(G, V, grid, st, a, out, nvec, h_vec);
-    }
-  } else {
-    aggr_fwd_generic_kernel<<<grid, 256, 0, st>>>(a, out);
+  if (!(vec && (a.in_dtype == HC_F32 ? launch_fwd<float>(l, vb) : launch_fwd<__half>(l, vb)))) {
+    const int64_t blocks = ceil_div(a.num_node * a.num_head, 8);
+    HC_REQUIRE(blocks <= 0x7fffffffLL, HC_ERR_SIZE);
+    aggr_fwd_generic_kernel<<<(unsigned)blocks, 256, 0, st>>>(a, out);
   }
   HC_LAUNCH_OK();
   return 0;

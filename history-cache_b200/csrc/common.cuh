@@ -83,29 +83,115 @@ struct Vec16<__half> {
   }
 };
 
-// acc[0..EL) += the EL elements of a 16-byte vector of T.  For fp16 this uses the
-// mixed-precision add of sm_100 (f32 += f16 in one instruction; the widening is exact, so
-// the result equals convert-then-add).
-template <typename T>
-__device__ __forceinline__ void accumulate_vec(float* acc, const uint4& v);
-template <>
-__device__ __forceinline__ void accumulate_vec<float>(float* acc, const uint4& v) {
-  acc[0] += __uint_as_float(v.x);
-  acc[1] += __uint_as_float(v.y);
-  acc[2] += __uint_as_float(v.z);
-  acc[3] += __uint_as_float(v.w);
-}
+// acc0 += low half of the word, acc1 += high half, with the mixed-precision add of sm_100 (f32 += f16
+// in one instruction; the widening is exact, so the result equals convert-then-add).
 #define HC_MIXED_ADD2(a0, a1, word)                                                   \
   asm("{.reg .b16 lo, hi; mov.b32 {lo, hi}, %2; add.f32.f16 %0, lo, %0; "             \
       "add.f32.f16 %1, hi, %1;}"                                                      \
       : "+f"(a0), "+f"(a1)                                                            \
       : "r"(word))
-template <>
-__device__ __forceinline__ void accumulate_vec<__half>(float* acc, const uint4& v) {
-  HC_MIXED_ADD2(acc[0], acc[1], v.x);
-  HC_MIXED_ADD2(acc[2], acc[3], v.y);
-  HC_MIXED_ADD2(acc[4], acc[5], v.z);
-  HC_MIXED_ADD2(acc[6], acc[7], v.w);
+
+// What one lane moves of a row per request: VB bytes (16, 8, 4 or 2) of elements of type T.  Rows
+// whose length or address is no multiple of 16 bytes are moved in the widest unit that divides both.
+template <typename T, int VB>
+struct LaneVec {
+  static constexpr int kElems = VB / (int)sizeof(T);
+  static constexpr int kWords = VB >= 4 ? VB / 4 : 1;
+  uint32_t w[kWords];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) w[i] = 0u;
+  }
+  __device__ __forceinline__ void load(const void* p) {
+    if constexpr (VB == 16) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+      w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+    } else if constexpr (VB == 8) {
+      const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+      w[0] = v.x; w[1] = v.y;
+    } else if constexpr (VB == 4) {
+      w[0] = __ldg(reinterpret_cast<const uint32_t*>(p));
+    } else {
+      w[0] = __ldg(reinterpret_cast<const uint16_t*>(p));
+    }
+  }
+  __device__ __forceinline__ void load_shared(const void* p) {
+    if constexpr (VB == 16) {
+      const uint4 v = *reinterpret_cast<const uint4*>(p);
+      w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+    } else if constexpr (VB == 8) {
+      const uint2 v = *reinterpret_cast<const uint2*>(p);
+      w[0] = v.x; w[1] = v.y;
+    } else {
+      w[0] = *reinterpret_cast<const uint32_t*>(p);
+    }
+  }
+  __device__ __forceinline__ void unpack(float* f) const {
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int i = 0; i < kWords; ++i) f[i] = __uint_as_float(w[i]);
+    } else if constexpr (VB == 2) {
+      f[0] = __half2float(__ushort_as_half((unsigned short)w[0]));
+    } else {
+#pragma unroll
+      for (int i = 0; i < kWords; ++i) {
+        const float2 p = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+        f[2 * i] = p.x;
+        f[2 * i + 1] = p.y;
+      }
+    }
+  }
+  __device__ __forceinline__ void add_to(float* acc) const {
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int i = 0; i < kWords; ++i) acc[i] += __uint_as_float(w[i]);
+    } else if constexpr (VB == 2) {
+      acc[0] += __half2float(__ushort_as_half((unsigned short)w[0]));
+    } else {
+#pragma unroll
+      for (int i = 0; i < kWords; ++i) HC_MIXED_ADD2(acc[2 * i], acc[2 * i + 1], w[i]);
+    }
+  }
+};
+
+// 4-, 8- or 16-byte asynchronous copy of one lane into shared memory (past the L1 where it can)
+template <int VB>
+__device__ __forceinline__ void cp_async(uint32_t dst_smem, const void* src) {
+  if constexpr (VB == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst_smem), "l"(src), "n"(VB) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Store of N consecutive fp32 values (N * 4 bytes aligned, at most 16) under an L2 policy.
+template <int N>
+__device__ __forceinline__ void store_f32(float* p, const float* f, uint64_t policy) {
+  if constexpr (N >= 4) {
+#pragma unroll
+    for (int i = 0; i < N; i += 4)
+      asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(p + i), "f"(f[i]), "f"(f[i + 1]),
+                   "f"(f[i + 2]), "f"(f[i + 3]), "l"(policy) : "memory");
+  } else if constexpr (N == 2) {
+    asm volatile("st.global.L2::cache_hint.v2.f32 [%0], {%1, %2}, %3;" ::"l"(p), "f"(f[0]), "f"(f[1]), "l"(policy)
+                 : "memory");
+  } else {
+    asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(p), "f"(f[0]), "l"(policy) : "memory");
+  }
+}
+// evict-first for results that will not stay in the L2 anyway, so that they do not push out the rows
+// the kernel still gathers; the default otherwise
+__device__ __forceinline__ uint64_t l2_policy(bool stream) {
+  uint64_t p;
+  if (stream)
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  else
+    asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+  return p;
 }
 
 // Vectorised fp32 reduction into global memory (one 16-byte transaction).
@@ -113,6 +199,17 @@ __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float 
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b),
                "f"(c), "f"(d)
                : "memory");
+}
+
+// fp32 reductions of N = 1, 2 or 4 consecutive values
+template <int N>
+__device__ __forceinline__ void red_add(float* p, const float* f) {
+  if constexpr (N == 4)
+    red_add_v4(p, f[0], f[1], f[2], f[3]);
+  else if constexpr (N == 2)
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(f[0]), "f"(f[1]) : "memory");
+  else
+    asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(f[0]) : "memory");
 }
 
 // ---- bulk-copy engine (TMA, untiled cp.async.bulk) and mbarrier helpers -----

@@ -305,3 +305,27 @@ def test_shared_transposition_is_rebuilt_for_buffers_refilled_behind_torch(backe
         gb, _, _ = oracle.aggr_bwd(ptr, idx, x, num_dst, np.abs(g), want_grad_history=False)
         close(xs.grad, want, 1e-5, bound=gb, terms=int(np.bincount(idx, minlength=n_src).max()),
               label="bwd_gather_shared")
+
+
+@pytest.mark.parametrize("feat,dtype", [(75, torch.float32), (130, torch.float32), (100, torch.float16),
+                                        (258, torch.float16), (77, torch.float16), (256, torch.float16)])
+@pytest.mark.parametrize("num_dst", [1, 31, 40_000])
+def test_forward_stream_of_edges(backend, oracle, feat, dtype, num_dst):
+    """Every unit a lane can move (16, 8, 4, 2 bytes), rows in several column parts, runs of one row and
+    of the longest length with empty rows, rows of more than one index chunk and stretches of history
+    rows longer than a chunk between them."""
+    rng = np.random.default_rng(feat + num_dst)
+    n_src = 500
+    deg = rng.integers(0, 9, num_dst)
+    deg[rng.random(num_dst) < 0.02] = 70
+    ptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)
+    idx = rng.integers(0, n_src, max(int(ptr[-1]), 1)).astype(np.int64)
+    x = rng.standard_normal((n_src, feat), dtype=np.float32)
+    hmap = np.where((np.arange(num_dst) // 20) % 3 == 1, np.arange(num_dst) % 13, -1).astype(np.int64)
+    table = rng.standard_normal((13, feat), dtype=np.float32)
+    xs, tb = cu(x, dtype), cu(table, dtype)
+    out = backend.aggr_forward(xs, cu(ptr), cu(idx), num_dst, history_map=cu(hmap), history_buffer=tb, indexed=True)
+    x, table = xs.float().cpu().numpy(), tb.float().cpu().numpy()
+    want = oracle.aggr_fwd(ptr, idx, x, num_dst, hmap=hmap, hbuf=table, h_indexed=True)
+    bound = oracle.aggr_fwd(ptr, idx, np.abs(x), num_dst, hmap=hmap, hbuf=np.abs(table), h_indexed=True)
+    close(out, want, RTOL[torch.float32], bound=bound, terms=int(deg.max()), label="fwd")
