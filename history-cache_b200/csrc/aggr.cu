@@ -236,6 +236,19 @@ __global__ void __launch_bounds__(256, (StreamShape<VB, V, EV>::kMinBlocks))
       const int64_t hr = shfl64(hrow, row);
       copy_history_part<EL>(a, a.h_indexed ? hr : r0 + row, out + (r0 + row) * width, width, v0, v1, lane, h_vec);
     }
+    // weights of the next slot, one slot ahead: a slot is a new sector of them
+    float w_next[U][EV == 2 ? V : 1];
+    int w_at = -1;
+    auto load_weights = [&](int from) {
+      w_at = from;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int k = 0; k < (EV == 2 ? V : 1); ++k) {
+          const int ee = from + u * EPW + sub;
+          w_next[u][k] = ee < total ? __ldg(a.edge_value + (EV == 2 ? (e0 + ee) * H + head[k] : e0 + ee)) : 0.f;
+        }
+    };
     int slot = 0;
     for (unsigned m = miss; m; m &= m - 1) {
       const int row = __ffs(m) - 1;
@@ -247,15 +260,14 @@ __global__ void __launch_bounds__(256, (StreamShape<VB, V, EV>::kMinBlocks))
         for (int q = 0; q < EL; ++q) acc[k][q] = 0.f;
 #pragma unroll 1
       for (int e = b; e < end; e += U * EPW) {
-        float w[U][EV == 2 ? V : 1];     // neighbouring edges' weights share lines of the L1
+        float w[U][EV == 2 ? V : 1];
         if (EV) {
+          if (e != w_at) load_weights(e);      // rows served from history were skipped
 #pragma unroll
           for (int u = 0; u < U; ++u)
 #pragma unroll
-            for (int k = 0; k < (EV == 2 ? V : 1); ++k) {
-              const int64_t ee = e0 + e + u * EPW + sub;
-              w[u][k] = e + u * EPW + sub < end ? __ldg(a.edge_value + (EV == 2 ? ee * H + head[k] : ee)) : 0.f;
-            }
+            for (int k = 0; k < (EV == 2 ? V : 1); ++k) w[u][k] = w_next[u][k];
+          load_weights(e + U * EPW < end ? e + U * EPW : end);
         }
         cp_async_wait<D - 1>();
 #pragma unroll
@@ -762,17 +774,6 @@ static int vec_shape(int nvec, int* G, int* V) {
   else if (nvec <= 256) { *G = 32; *V = 8; }
   else return 0;
   return 1;
-}
-
-// Raises a kernel's shared-memory limit, once per kernel (`done` is its own) and device; not a stream
-// operation, so it may happen during a capture.
-template <typename K>
-static void raise_smem(K kernel, int bytes, std::atomic<uint64_t>& done) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev > 63) dev = 63;
-  if (done.load(std::memory_order_relaxed) >> dev & 1) return;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
-    done.fetch_or(1ull << dev, std::memory_order_relaxed);
 }
 
 // Widest unit (16, 8, 4 or 2 bytes) that divides every given address or length; never below `es`.

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "hiscache_b200.h"
 
 #define HC_CUDA(call)                        \
@@ -35,6 +37,17 @@ __host__ __device__ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 inline bool aligned_to(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 inline int dtype_size(int dt) { return dt == HC_F32 ? 4 : (dt == HC_F16 ? 2 : 0); }
+
+// Raises a kernel's shared-memory limit, once per kernel (`done` is its own) and device; not a stream
+// operation, so it may happen during a capture.
+template <typename K>
+inline void raise_smem(K kernel, int bytes, std::atomic<uint64_t>& done) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev > 63) dev = 63;
+  if (done.load(std::memory_order_relaxed) >> dev & 1) return;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
+    done.fetch_or(1ull << dev, std::memory_order_relaxed);
+}
 
 // 64-bit shuffle (two 32-bit shuffles).
 __device__ __forceinline__ int64_t shfl64(int64_t v, int src) {
@@ -114,6 +127,12 @@ struct LaneVec {
     } else {
       w[0] = __ldg(reinterpret_cast<const uint16_t*>(p));
     }
+  }
+  // read once: not kept in the L1, first to leave the L2 (`policy` from l2_policy(true))
+  __device__ __forceinline__ void load_once(const void* p, uint64_t policy) {
+    static_assert(VB == 16, "wide units only");
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "l"(p), "l"(policy));
   }
   __device__ __forceinline__ void load_shared(const void* p) {
     if constexpr (VB == 16) {

@@ -38,7 +38,8 @@ namespace {
 // ---------------------------------------------------------------------------
 #define HC_FUNCTIONS(X)                                                                            \
   X(hc_error_string) X(hc_aggr_fwd) X(hc_aggr_bwd) X(hc_transpose_scratch_bytes)                   \
-  X(hc_transpose_block) X(hc_gather_scratch_bytes) X(hc_aggr_bwd_gather) X(hc_norm_scratch_bytes)  \
+  X(hc_transpose_block) X(hc_gather_scratch_bytes) X(hc_aggr_bwd_gather)                           \
+  X(hc_aggr_bwd_source_scratch_bytes) X(hc_aggr_bwd_source) X(hc_norm_scratch_bytes)               \
   X(hc_norm_act_fwd) X(hc_norm_act_bwd)
 
 struct Lib {
@@ -384,17 +385,26 @@ variable_list AggrBackward::apply(variable_list&& grads) {
   Tensor g_in, g_ev, g_h;
   if (need_in) g_in = new_f32(b.inp.sizes(), dev);
   if (need_ev) g_ev = new_f32(b.ev.sizes(), dev);
-  // gather over the transposed block instead of the atomic scatter: always when a reproducible
-  // backward is asked for, else for blocks large enough to pay for it
-  bool gathered = false;
-  if (need_in && !b.ev.defined() && !multi && a.feat % 4 == 0 && a.feat <= 1024 &&
-      (rule.deterministic || (a.feat >= rule.gather_min_feat &&
-                              a.n_src * (int64_t)a.feat * 4 >= rule.gather_min_bytes))) {
+  // Three forms.  A reproducible backward gathers over the sorted transposition.  Otherwise blocks
+  // that gather enough are differentiated by source, and the rest scatter.
+  bool gathered = false, edges_done = false;
+  if (need_in && rule.deterministic && !b.ev.defined() && !multi && a.feat % 4 == 0 && a.feat <= 1024) {
     Transposed t = shared_transpose(b.ptr, b.idx);
     if (t.n_edges < 0 || t.t_ptr.size(0) - 1 < a.n_src)      // a block nobody declared: its own transposition
       t = transpose_block(a, b.idx.numel(), dev);
     aggr_bwd_gather(a, t, go, g_in, dev, b.inp);
     gathered = true;
+  } else if ((need_in || need_ev) && !rule.deterministic && (int64_t)a.feat * a.num_head >= rule.gather_min_feat &&
+             a.n_src * (int64_t)a.feat * a.num_head * 4 >= rule.gather_min_bytes) {
+    const int64_t bytes = lib.hc_aggr_bwd_source_scratch_bytes(&a, b.idx.numel(), g_ev.defined());
+    if (bytes >= 0) {
+      Tensor sc = new_scratch(bytes, dev);
+      HC_SPAN_ROWS("hc_aggr_bwd_source", b.inp, dev);
+      check(lib.hc_aggr_bwd_source(&a, b.idx.numel(), fdata(go), fdata(g_in), fdata(g_ev), data(sc), stream_of(dev)),
+            "hc_aggr_bwd_source");
+      g_launches += 5;
+      gathered = edges_done = true;
+    }
   }
   if (need_h) {
     g_h = at::zeros(b.hbuf.sizes(), b.hbuf.options().dtype(at::kFloat));
@@ -402,7 +412,7 @@ variable_list AggrBackward::apply(variable_list&& grads) {
   }
   if (!gathered || need_h || row_score.defined()) {
     HC_SPAN_ROWS("hc_aggr_bwd", b.inp, dev);
-    check(lib.hc_aggr_bwd(&a, fdata(go), gathered ? nullptr : fdata(g_in), 1, fdata(g_h), fdata(g_ev),
+    check(lib.hc_aggr_bwd(&a, fdata(go), gathered ? nullptr : fdata(g_in), 1, fdata(g_h), edges_done ? nullptr : fdata(g_ev),
                           fdata(row_score), score_kind, stream_of(dev)),
           "hc_aggr_bwd");
     ++g_launches;

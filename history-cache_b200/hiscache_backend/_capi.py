@@ -81,6 +81,8 @@ _SIGS = {
     "hc_transpose_block": (C.c_int, [C.POINTER(AggrArgs), i64, vp, vp, vp, vp, vp]),
     "hc_gather_scratch_bytes": (i64, [i64, i32]),
     "hc_aggr_bwd_gather": (C.c_int, [C.POINTER(AggrArgs), vp, vp, vp, i64, i64, vp, vp, vp, vp]),
+    "hc_aggr_bwd_source_scratch_bytes": (i64, [C.POINTER(AggrArgs), i64, i32]),
+    "hc_aggr_bwd_source": (C.c_int, [C.POINTER(AggrArgs), i64, vp, vp, vp, vp, vp]),
     "hc_score_rows": (C.c_int, [vp, i64, i32, i64, i32, vp, vp]),
     "hc_select_scratch_bytes": (i64, [i64]),
     "hc_select_threshold": (C.c_int, [vp, i64, f32, vp, vp, vp]),

@@ -192,6 +192,24 @@ int hc_aggr_bwd_gather(const hc_aggr_args* a, const int64_t* t_ptr, const int64_
                        const float* t_w, int64_t t_n_src, int64_t n_edges, const float* grad_out,
                        float* grad_input, void* scratch, void* stream);
 
+/*
+ * Backward by source, for callers that do not need a fixed order of additions:
+ * grad_input (fp32 [n_src, num_head, feat], every row written, or NULL) and
+ * edge_grad (fp32 [E(, num_head)] of an edge-weighted sum, or NULL) from one
+ * pass over lists of edges per source that the call builds itself in scratch.
+ * n_edges >= ptr[num_node].  Same results as hc_aggr_bwd up to the order of
+ * additions.  scratch: device, 16-byte aligned,
+ * >= hc_aggr_bwd_source_scratch_bytes(a, n_edges, edge_grad != NULL); a
+ * negative size means that the call does not serve this block (-HC_ERR_UNSUPPORTED;
+ * hc_aggr_bwd does): num_node, n_src or n_edges of 0 or beyond 31 bits,
+ * weights per head with feat % 4 != 0, and with edge_grad also: fp16 rows,
+ * src_map, feat % 4 != 0, more than 512 columns of a single head or 128 of one
+ * of several.
+ */
+int64_t hc_aggr_bwd_source_scratch_bytes(const hc_aggr_args* a, int64_t n_edges, int32_t want_edge_grad);
+int hc_aggr_bwd_source(const hc_aggr_args* a, int64_t n_edges, const float* grad_out,
+                       float* grad_input, float* edge_grad, void* scratch, void* stream);
+
 /* ------------------------------------------------------------------------ */
 /* Scores and thresholds                                                    */
 /* ------------------------------------------------------------------------ */

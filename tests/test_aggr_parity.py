@@ -329,3 +329,39 @@ def test_forward_stream_of_edges(backend, oracle, feat, dtype, num_dst):
     want = oracle.aggr_fwd(ptr, idx, x, num_dst, hmap=hmap, hbuf=table, h_indexed=True)
     bound = oracle.aggr_fwd(ptr, idx, np.abs(x), num_dst, hmap=hmap, hbuf=np.abs(table), h_indexed=True)
     close(out, want, RTOL[torch.float32], bound=bound, terms=int(deg.max()), label="fwd")
+
+
+@pytest.mark.parametrize("feat,heads,weighted", [(32, 1, False), (64, 1, False), (75, 1, False), (130, 1, True),
+                                                 (300, 1, False), (300, 1, True), (16, 1, True), (64, 4, True),
+                                                 (12, 5, True), (48, 8, True), (20, 2, True)])
+@pytest.mark.parametrize("num_dst", [3, 9000])
+def test_backward_by_source(backend, oracle, monkeypatch, feat, heads, weighted, num_dst):
+    """Lists of 0, of about 64 and of thousands of entries, more sources than one scan block, history
+    rows, every unit of a lane, heads whose lanes are and are not a power of two."""
+    monkeypatch.setattr(backend, "GATHER_MIN_BYTES", 0)
+    monkeypatch.setattr(backend, "GATHER_MIN_FEAT", 0)
+    rng = np.random.default_rng(feat * heads + num_dst)
+    n_src = 5000 if num_dst > 100 else 7
+    deg = rng.integers(0, 7, num_dst)
+    ptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)
+    E = int(ptr[-1])
+    idx = (rng.random(max(E, 1)) ** 3 * n_src).astype(np.int64)
+    if E > 400:
+        idx[rng.permutation(E)[:65]] = n_src - 1        # one entry more than a warp takes
+    multi = heads > 1
+    x = rng.standard_normal((n_src, heads, feat) if multi else (n_src, feat), dtype=np.float32)
+    ev = rng.standard_normal((E, heads) if multi else (E,), dtype=np.float32) if weighted else None
+    hmap = np.where(rng.random(num_dst) < 0.1, np.arange(num_dst), -1).astype(np.int64)
+    hbuf = rng.standard_normal((num_dst, feat), dtype=np.float32)
+    xs = cu(x).requires_grad_(True)
+    evs = cu(ev).requires_grad_(True) if weighted else None
+    out = backend.aggr_forward(xs, cu(ptr), cu(idx), num_dst, edge_value=evs, history_map=cu(hmap), history_buffer=cu(hbuf))
+    g = rng.standard_normal(tuple(out.shape), dtype=np.float32)
+    out.backward(cu(g))
+    kw = dict(edge_value=ev, hmap=hmap, hsize=feat, want_edge_grad=weighted)
+    gi, _, eg = oracle.aggr_bwd(ptr, idx, x, num_dst, g, **kw)
+    kw["edge_value"] = None if ev is None else np.abs(ev)
+    gb, _, eb = oracle.aggr_bwd(ptr, idx, np.abs(x), num_dst, np.abs(g), **kw)
+    close(xs.grad, gi, 1e-5, bound=gb, terms=int(np.bincount(idx, minlength=n_src).max()), label="bwd_source")
+    if weighted:
+        close(evs.grad, eg, 1e-5, bound=eb, terms=feat, label="edge_grad_source")
