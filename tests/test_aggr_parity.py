@@ -365,3 +365,21 @@ def test_backward_by_source(backend, oracle, monkeypatch, feat, heads, weighted,
     close(xs.grad, gi, 1e-5, bound=gb, terms=int(np.bincount(idx, minlength=n_src).max()), label="bwd_source")
     if weighted:
         close(evs.grad, eg, 1e-5, bound=eb, terms=feat, label="edge_grad_source")
+
+
+@pytest.mark.parametrize("feat", [5, 6, 7, 9, 129, 511])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_backward_scatter_of_shifted_rows(backend, oracle, feat, weighted):
+    """Rows that start at every offset from a 16-byte boundary; the last word of the last row."""
+    rng = np.random.default_rng(feat)
+    num_dst, n_src = 60, 33
+    ptr, idx = csr_block(rng, num_dst, n_src, "mixed")
+    idx[-1] = n_src - 1
+    x = rng.standard_normal((n_src, feat), dtype=np.float32)
+    ev = rng.standard_normal(len(idx), dtype=np.float32) if weighted else None
+    g = rng.standard_normal((num_dst, feat), dtype=np.float32)
+    xs = cu(x).requires_grad_(True)
+    backend.aggr_forward(xs, cu(ptr), cu(idx), num_dst, edge_value=cu(ev)).backward(cu(g))
+    gi, _, _ = oracle.aggr_bwd(ptr, idx, x, num_dst, g, edge_value=ev)
+    gb, _, _ = oracle.aggr_bwd(ptr, idx, x, num_dst, np.abs(g), edge_value=None if ev is None else np.abs(ev))
+    close(xs.grad, gi, 1e-5, bound=gb, terms=int(np.bincount(idx, minlength=n_src).max()), label="bwd_shift")
