@@ -70,16 +70,35 @@ __device__ __forceinline__ void move_row(const void* src, int sdt, int64_t soff,
 
 __global__ void map_lookup_kernel(const int64_t* __restrict__ map, int64_t map_len,
                                   const int64_t* __restrict__ ids, int64_t n, int64_t offset,
-                                  int64_t force_miss_below, int64_t* __restrict__ out) {
+                                  int64_t force_miss_below, const uint8_t* __restrict__ valid,
+                                  int64_t* __restrict__ out) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int64_t v = -1;
-  if (i >= force_miss_below) {
+  if (i >= force_miss_below && (!valid || valid[i] != 0)) {
     int64_t p = ids[i] + offset;
     if (p < 0) p += map_len;  // torch negative indexing
     if (p >= 0 && p < map_len) v = map[p];
   }
   out[i] = v;
+}
+
+// both lookups of a cache step: the embedding entry of the first n1 nodes and the feature entry of all
+__global__ void __launch_bounds__(256)
+    cache_lookup_kernel(const int64_t* __restrict__ map, int64_t map_len, const int64_t* __restrict__ ids, int64_t n,
+                        int64_t n1, int64_t offset, int64_t* __restrict__ sub2embed, int64_t* __restrict__ sub2feat) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int64_t id = ids[i];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    if (k == 1 && i >= n1) break;
+    int64_t p = k == 0 ? id + offset : id;
+    if (p < 0) p += map_len;  // torch negative indexing
+    const int64_t v = p >= 0 && p < map_len ? map[p] : -1;
+    if (k == 0) sub2feat[i] = v;
+    else sub2embed[i] = v;
+  }
 }
 
 template <int G>
@@ -422,15 +441,38 @@ __global__ void __launch_bounds__(kStageThreads)
 
 }  // namespace hc
 
-extern "C" int hc_map_lookup(const int64_t* map, int64_t map_len, const int64_t* ids, int64_t n,
-                             int64_t offset, int64_t force_miss_below, int64_t* out, void* stream) {
+static int map_lookup(const int64_t* map, int64_t map_len, const int64_t* ids, int64_t n, int64_t offset,
+                      int64_t force_miss_below, const uint8_t* valid, int64_t* out, void* stream) {
   HC_REQUIRE(n >= 0 && map_len >= 0, HC_ERR_SIZE);
   if (n == 0) return 0;
   HC_REQUIRE(map && ids && out, HC_ERR_NULL);
   const int64_t blocks = ceil_div(n, 256);
   HC_REQUIRE(blocks <= 0x7fffffffLL, HC_ERR_SIZE);
   map_lookup_kernel<<<(unsigned)blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      map, map_len, ids, n, offset, force_miss_below, out);
+      map, map_len, ids, n, offset, force_miss_below, valid, out);
+  HC_LAUNCH_OK();
+  return 0;
+}
+
+extern "C" int hc_map_lookup(const int64_t* map, int64_t map_len, const int64_t* ids, int64_t n,
+                             int64_t offset, int64_t force_miss_below, int64_t* out, void* stream) {
+  return map_lookup(map, map_len, ids, n, offset, force_miss_below, nullptr, out, stream);
+}
+
+extern "C" int hc_map_lookup_masked(const int64_t* map, int64_t map_len, const int64_t* ids, int64_t n,
+                                    int64_t force_miss_below, const uint8_t* valid, int64_t* out, void* stream) {
+  return map_lookup(map, map_len, ids, n, 0, force_miss_below, valid, out, stream);
+}
+
+extern "C" int hc_cache_lookup(const int64_t* map, int64_t map_len, const int64_t* ids, int64_t n, int64_t n1,
+                               int64_t offset, int64_t* sub2embed, int64_t* sub2feat, void* stream) {
+  HC_REQUIRE(n >= 0 && map_len >= 0 && n1 >= 0 && n1 <= n, HC_ERR_SIZE);
+  if (n == 0) return 0;
+  HC_REQUIRE(map && ids && sub2feat && (sub2embed || n1 == 0), HC_ERR_NULL);
+  const int64_t blocks = ceil_div(n, 256);
+  HC_REQUIRE(blocks <= 0x7fffffffLL, HC_ERR_SIZE);
+  cache_lookup_kernel<<<(unsigned)blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(map, map_len, ids, n, n1, offset,
+                                                                                          sub2embed, sub2feat);
   HC_LAUNCH_OK();
   return 0;
 }

@@ -14,12 +14,34 @@
 // the host-driven one.  What does not fit is cut in a memory-safe way and counted: a new node beyond
 // its layer's capacity is not added and the edges to it become self loops of their destination row;
 // edges beyond edge_cap are dropped.
-#include "common.cuh"
+#include "grid_sync.cuh"
 
 namespace hc {
 
 constexpr int kAbsentF = (int)0x80000000;
 constexpr int kMaxHops = 8;
+
+// ---------------------------------------------------------------------------
+// One kernel draws the whole batch.
+//
+// A hop is: draw and claim, count what is new, number it, translate the edges; each stage needs the
+// stage before it from every block.  As separate launches (35 for three hops of some thousands of
+// rows) a batch took 172 us, 166 of them the host's launches and 113 the GPU's, nearly all of it the
+// start and end of tiny kernels.  Here the stages are separated by a barrier of all blocks of one
+// cooperative launch, three per hop:
+//   A  draw, claim (the lowest position of a node wins), sum up the draws per block        | barrier
+//   B  count per block the positions that won their node                                   | barrier
+//   C  number the new nodes, give them rows                                                | barrier
+//   D  edges of the hop into idx, ptr entries
+// Positions are row * fanout + draw, so their order needs no scan; a block owns the same rows through
+// all stages and keeps their draw counts in shared memory and most draws in registers.  The others are
+// kept in two buffers, because a fast block is already drawing hop h + 1 while a slow one still
+// translates hop h.  A cluster of 16 blocks with the hardware's barrier took 61 us against 50: hashing
+// and the memory latencies of a hop want more SMs.
+// ---------------------------------------------------------------------------
+constexpr int kSampleThreads = 512;
+constexpr int kSampleKeep = 2;           // draws per thread that stay in registers
+constexpr int kSampleBlocks = 96;        // leaves SMs to the kernels it runs beside; 64..148 blocks: 50..53 us
 
 struct FixedPlan {
   int num_hops;
@@ -31,218 +53,229 @@ struct FixedPlan {
   int64_t* sub_to_full;
   uint8_t* mask;
   int64_t* counters;     // [0] real nodes [1] real edges [2] new nodes cut [3] edges cut
+  // inputs
+  const int64_t* gptr;
+  const int64_t* gidx;
+  const int64_t* seeds;
+  int64_t n_seeds;
+  int* local_map;
+  uint64_t seed;
+  int64_t* batch_no;
+  const int64_t* labels;   // with y [caps[0]]: y = labels[seed], -100 in padding rows
+  int64_t* y;
   // scratch
-  int64_t* state;        // [0] batch seed [1] edge offset [2] frontier base [3] hop edges [4] hop new nodes
-  int64_t* cnt;          // [max frontier + 1] counts, then their exclusive scan
-  int64_t* nbr;          // [max frontier * fanout]
-  int64_t* new_nodes;    // [max frontier * fanout]
-  int64_t* block_counts; // [blocks]
+  unsigned* barrier;
+  int* draws;              // [blocks] draws per block of the current hop
+  int* firsts;             // [blocks] new nodes per block
+  int64_t* nbr[2];         // [max rows * fanout] drawn neighbours, -1: none
+  int* row_at;             // [blocks][rows_cap] when a block's rows do not fit its shared memory
 };
 
-__global__ void fixed_begin_kernel(const FixedPlan p, const int64_t* __restrict__ seeds, int64_t n_seeds,
-                                   int* local_map, uint64_t seed, int64_t* batch_no) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kSampleThreads) sample_fixed_kernel(const FixedPlan p, const int rows_cap) {
+  extern __shared__ int sh_rows[];
+  // [rows_cap] draws of a row, then where its edges start in the hop
+  int* row_at = p.row_at ? p.row_at + (int64_t)blockIdx.x * rows_cap : sh_rows;
+  const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, threads = (int64_t)gridDim.x * blockDim.x;
+  GridSync grid(p.barrier);
   const int64_t total = p.caps[p.num_hops];
-  if (i < total) {
-    const bool s = i < n_seeds;
-    p.sub_to_full[i] = s ? seeds[i] : 0;
+  const uint64_t batch_seed = mix64(p.seed * 1000003ull + (uint64_t)p.batch_no[0]);
+  for (int64_t i = gtid; i < total; i += threads) {
+    const bool s = i < p.n_seeds;
+    const int64_t v = s ? p.seeds[i] : 0;
+    p.sub_to_full[i] = v;
     p.mask[i] = s ? 1 : 0;
-    if (s) local_map[seeds[i]] = (int)i;
+    if (s) p.local_map[v] = (int)i;
+    if (p.y && i < p.caps[0]) p.y[i] = s ? p.labels[v] : -100;
   }
-  if (i == 0) {
-    // the same arithmetic as the host-driven sampler: mix64(seed * 1000003 + batch number)
-    p.state[0] = (int64_t)mix64(seed * 1000003ull + (uint64_t)batch_no[0]);
-    batch_no[0] += 1;
-    p.state[1] = 0;
-    p.state[2] = 0;
-    p.counters[0] = n_seeds;
-    p.counters[1] = 0;
-    p.counters[2] = 0;
-    p.counters[3] = 0;
-  }
-}
+  for (int64_t e = gtid; e < p.edge_cap; e += threads) p.idx[e] = 0;
+  if (!grid.wait()) return;
 
-__global__ void fixed_counts_kernel(const FixedPlan p, const int64_t* __restrict__ gptr, int64_t fs, int64_t nf,
-                                    int fanout) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nf) return;
-  int64_t c = 0;
-  if (p.mask[fs + i]) {
-    const int64_t v = p.sub_to_full[fs + i];
-    const int64_t deg = gptr[v + 1] - gptr[v];
-    c = deg < fanout ? deg : fanout;
-  }
-  p.cnt[i] = c;
-}
-
-// exclusive scan of cnt[0..n) in place by one block; cnt[n] = total, also kept in state[3]
-__global__ void __launch_bounds__(1024) fixed_scan_kernel(const FixedPlan p, int64_t n) {
-  __shared__ int64_t part[1024];
-  __shared__ int64_t carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int64_t base = 0; base < n; base += 1024) {
-    const int64_t b = base + threadIdx.x;
-    const int64_t c = b < n ? p.cnt[b] : 0;
-    part[threadIdx.x] = c;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-      const int64_t v = threadIdx.x >= off ? part[threadIdx.x - off] : 0;
-      __syncthreads();
-      part[threadIdx.x] += v;
-      __syncthreads();
+  int64_t base = 0;                    // real frontier rows of the earlier hops
+  int64_t frontier = p.n_seeds;        // real rows of this hop's frontier
+  int64_t e_off = 0, nodes = p.n_seeds, cut_nodes = 0, cut_edges = 0;
+  for (int h = 0; h < p.num_hops; ++h) {
+    const int64_t fs = h == 0 ? 0 : p.caps[h - 1];
+    const int64_t nf = p.caps[h] - fs;                // frontier capacity (rows [fs, caps[h]))
+    const int64_t row0 = p.caps[h];                   // the new nodes' first row
+    const int64_t cap_new = p.caps[h + 1] - p.caps[h];
+    const int fan = p.fanout[h];
+    if (nf == 0) continue;
+    int64_t* nbr = p.nbr[h & 1];
+    // rows of this block; real rows come first, so they are cut evenly
+    const int64_t per = ceil_div(frontier, (int64_t)gridDim.x);
+    const int64_t r0 = per * blockIdx.x < frontier ? per * blockIdx.x : frontier;
+    const int rows = (int)(r0 + per < frontier ? per : frontier - r0);
+    const int slots = rows * fan;
+    // a thread keeps its first draws, and whether they won, in registers; the rest is read again
+    int64_t kept_d[kSampleKeep];
+    bool kept_won[kSampleKeep];
+    auto won_at = [&](int t, int64_t d) { return d >= 0 && __ldcg(p.local_map + d) == -(int)(r0 * fan + t + 2); };
+    // A
+    int mine = 0;
+    for (int i = threadIdx.x; i < rows; i += blockDim.x) {
+      const int64_t v = __ldcg(p.sub_to_full + fs + r0 + i);
+      const int64_t deg = p.gptr[v + 1] - p.gptr[v];
+      const int c = (int)(deg < fan ? deg : fan);
+      row_at[i] = c;
+      mine += c;
     }
-    if (b < n) p.cnt[b] = carry + part[threadIdx.x] - c;
-    __syncthreads();
-    if (threadIdx.x == 1023) carry += part[1023];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    p.cnt[n] = carry;
-    p.state[3] = carry;
-  }
-}
-
-__global__ void fixed_picks_kernel(const FixedPlan p, const int64_t* __restrict__ gptr,
-                                   const int64_t* __restrict__ gidx, int64_t fs, int64_t nf, int fanout) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t i = t / fanout;
-  const int j = (int)(t % fanout);
-  if (i >= nf) return;
-  const int64_t o = p.cnt[i];
-  if (j >= p.cnt[i + 1] - o) return;
-  const int64_t v = p.sub_to_full[fs + i];
-  const int64_t b = gptr[v];
-  const uint64_t deg = (uint64_t)(gptr[v + 1] - b);
-  const uint64_t seed = (uint64_t)p.state[0];
-  const uint64_t u = mix64(seed ^ mix64((uint64_t)(p.state[2] + i) * (uint64_t)fanout + (uint64_t)j));
-  p.nbr[o + j] = gidx[b + (int64_t)(u % deg)];
-}
-
-// position q claims node nbr[q] unless the node already has a local id; the lowest q wins
-__global__ void fixed_claim_kernel(const FixedPlan p, int* local_map) {
-  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < p.state[3]) atomicMax(local_map + p.nbr[q], -(int)(q + 2));
-}
-
-__device__ __forceinline__ bool fixed_is_first(const FixedPlan& p, const int* local_map, int64_t q) {
-  return q < p.state[3] && local_map[p.nbr[q]] == -(int)(q + 2);
-}
-
-__global__ void __launch_bounds__(1024)
-    fixed_first_count_kernel(const FixedPlan p, const int* __restrict__ local_map) {
-  const int64_t q = (int64_t)blockIdx.x * 1024 + threadIdx.x;
-  const int c = __syncthreads_count(fixed_is_first(p, local_map, q));
-  if (threadIdx.x == 0) p.block_counts[blockIdx.x] = c;
-}
-
-__global__ void __launch_bounds__(1024) fixed_first_scan_kernel(const FixedPlan p, int64_t nblocks) {
-  __shared__ int64_t part[1024];
-  __shared__ int64_t carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int64_t base = 0; base < nblocks; base += 1024) {
-    const int64_t b = base + threadIdx.x;
-    const int64_t c = b < nblocks ? p.block_counts[b] : 0;
-    part[threadIdx.x] = c;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-      const int64_t v = threadIdx.x >= off ? part[threadIdx.x - off] : 0;
-      __syncthreads();
-      part[threadIdx.x] += v;
-      __syncthreads();
+    auto pick = [&](int i, int j, int64_t first, int64_t deg) {
+      const uint64_t u = mix64(batch_seed ^ mix64((uint64_t)(base + r0 + i) * (uint64_t)fan + (uint64_t)j));
+      return first + (int64_t)(u % (uint64_t)deg);
+    };
+    {
+      // the draws of a thread side by side: three latencies for all of them
+      int64_t v[kSampleKeep], first[kSampleKeep], deg[kSampleKeep];
+#pragma unroll
+      for (int k = 0; k < kSampleKeep; ++k) {
+        const int t = threadIdx.x + k * kSampleThreads;
+        v[k] = t < slots ? __ldcg(p.sub_to_full + fs + r0 + t / fan) : -1;
+      }
+#pragma unroll
+      for (int k = 0; k < kSampleKeep; ++k) {
+        first[k] = v[k] >= 0 ? p.gptr[v[k]] : 0;
+        deg[k] = v[k] >= 0 ? p.gptr[v[k] + 1] : 0;
+      }
+#pragma unroll
+      for (int k = 0; k < kSampleKeep; ++k) {
+        const int t = threadIdx.x + k * kSampleThreads, i = t / fan, j = t - i * fan;
+        deg[k] -= first[k];
+        kept_d[k] = j < deg[k] ? p.gidx[pick(i, j, first[k], deg[k])] : -1;
+      }
+#pragma unroll
+      for (int k = 0; k < kSampleKeep; ++k)
+        if (kept_d[k] >= 0) atomicMax(p.local_map + kept_d[k], -(int)(r0 * fan + threadIdx.x + k * kSampleThreads + 2));
+      for (int t = threadIdx.x + kSampleKeep * kSampleThreads; t < slots; t += kSampleThreads) {
+        const int i = t / fan, j = t - i * fan;
+        const int64_t w = __ldcg(p.sub_to_full + fs + r0 + i);
+        const int64_t b = p.gptr[w], n = p.gptr[w + 1] - b;
+        int64_t d = -1;
+        if (j < n) {
+          d = p.gidx[pick(i, j, b, n)];
+          atomicMax(p.local_map + d, -(int)(r0 * fan + t + 2));
+        }
+        nbr[r0 * fan + t] = d;
+      }
     }
-    if (b < nblocks) p.block_counts[b] = carry + part[threadIdx.x] - c;
-    __syncthreads();
-    if (threadIdx.x == 1023) carry += part[1023];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) p.state[4] = carry;
-}
-
-// new nodes in order of first occurrence; those beyond the layer's capacity are cut
-__global__ void __launch_bounds__(1024)
-    fixed_place_kernel(const FixedPlan p, int* local_map, int64_t row0, int64_t cap_new) {
-  __shared__ int warp_sums[32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t q = (int64_t)blockIdx.x * 1024 + threadIdx.x;
-  const bool f = fixed_is_first(p, local_map, q);
-  const unsigned bal = __ballot_sync(kFull, f);
-  if (lane == 0) warp_sums[warp] = __popc(bal);
-  __syncthreads();
-  int before = 0;
-  for (int w = 0; w < warp; ++w) before += warp_sums[w];
-  if (f) {
-    const int64_t rank = p.block_counts[blockIdx.x] + before + __popc(bal & ((1u << lane) - 1u));
-    const int64_t v = p.nbr[q];
-    if (rank < cap_new) {
-      p.sub_to_full[row0 + rank] = v;
-      p.mask[row0 + rank] = 1;
-      p.new_nodes[rank] = v;
-    } else {
-      p.new_nodes[rank] = -1 - v;     // cut: remembered so that its claim can be withdrawn
+    int block_draws;
+    block_exclusive<kSampleThreads>(mine, &block_draws);
+    if (threadIdx.x == 0) p.draws[blockIdx.x] = block_draws;
+    if (!grid.wait()) return;
+    // B
+    int won = 0;
+    {
+#pragma unroll
+      for (int k = 0; k < kSampleKeep; ++k) {
+        const int t = threadIdx.x + k * kSampleThreads;
+        const int64_t d = kept_d[k];
+        kept_won[k] = won_at(t, d);
+        won += kept_won[k];
+      }
+      for (int t = threadIdx.x + kSampleKeep * kSampleThreads; t < slots; t += blockDim.x)
+        won += won_at(t, nbr[r0 * fan + t]);
     }
+    int block_new;
+    block_exclusive<kSampleThreads>(won, &block_new);
+    if (threadIdx.x == 0) p.firsts[blockIdx.x] = block_new;
+    int hop_draws, first_edge;
+    block_prefix(p.draws, gridDim.x, blockIdx.x, &hop_draws, &first_edge);
+    // where each row's edges start
+    for (int i0 = 0; i0 < rows; i0 += blockDim.x) {
+      const int i = i0 + threadIdx.x;
+      const int c = i < rows ? row_at[i] : 0;
+      int n_here;
+      const int at = first_edge + block_exclusive<kSampleThreads>(c, &n_here);
+      if (i < rows) row_at[i] = at;
+      first_edge += n_here;
+    }
+    if (!grid.wait()) return;
+    // C
+    int hop_new, first_new;
+    block_prefix(p.firsts, gridDim.x, blockIdx.x, &hop_new, &first_new);
+    {
+      int n = 0;
+      for (int t0 = 0; t0 < slots; t0 += blockDim.x, ++n) {
+        const int t = t0 + threadIdx.x;
+        int64_t d = -1;
+        bool f = false;
+        if (t < slots) {
+#pragma unroll
+          for (int k = 0; k < kSampleKeep; ++k)
+            if (n == k) { d = kept_d[k]; f = kept_won[k]; }
+          if (n >= kSampleKeep) { d = nbr[r0 * fan + t]; f = won_at(t, d); }
+        }
+        int n_here;
+        const int64_t rank = first_new + block_exclusive<kSampleThreads>(f ? 1 : 0, &n_here);
+        first_new += n_here;
+        if (f && rank < cap_new) {       // those beyond the layer's capacity keep their claim: they are cut
+          p.sub_to_full[row0 + rank] = d;
+          p.mask[row0 + rank] = 1;
+          p.local_map[d] = (int)(row0 + rank);
+        }
+      }
+    }
+    if (!grid.wait()) return;
+    // D
+    for (int i = threadIdx.x; i < rows; i += blockDim.x) {
+      const int64_t at = e_off + row_at[i];
+      p.ptr[fs + r0 + i] = at < p.edge_cap ? at : p.edge_cap;
+    }
+    for (int64_t i = frontier + gtid; i < nf; i += threads) {      // padding rows have no edges
+      const int64_t at = e_off + hop_draws;
+      p.ptr[fs + i] = at < p.edge_cap ? at : p.edge_cap;
+    }
+    auto put_edge = [&](int t, int loc) {
+      const int i = t / fan, j = t - i * fan;
+      const int64_t e = e_off + row_at[i] + j;
+      // a node that was cut has no row: the edge becomes a self loop of its destination row
+      if (e < p.edge_cap) p.idx[e] = loc >= 0 ? (int64_t)loc : fs + r0 + i;
+    };
+    {
+      int loc[kSampleKeep];
+#pragma unroll
+      for (int k = 0; k < kSampleKeep; ++k) loc[k] = kept_d[k] >= 0 ? __ldcg(p.local_map + kept_d[k]) : 0;
+#pragma unroll
+      for (int k = 0; k < kSampleKeep; ++k)
+        if (kept_d[k] >= 0) put_edge(threadIdx.x + k * kSampleThreads, loc[k]);
+      for (int t = threadIdx.x + kSampleKeep * kSampleThreads; t < slots; t += kSampleThreads) {
+        const int64_t d = nbr[r0 * fan + t];
+        if (d >= 0) put_edge(t, __ldcg(p.local_map + d));
+      }
+    }
+    if (hop_new > cap_new) {           // the claims of cut nodes are withdrawn once every block has read them
+      if (!grid.wait()) return;
+      int n = 0;
+      for (int t = threadIdx.x; t < slots; t += blockDim.x, ++n) {
+        int64_t d = -1;
+#pragma unroll
+        for (int k = 0; k < kSampleKeep; ++k)
+          if (n == k) d = kept_d[k];
+        if (n >= kSampleKeep) d = nbr[r0 * fan + t];
+        if (d >= 0 && __ldcg(p.local_map + d) == -(int)(r0 * fan + t + 2)) p.local_map[d] = kAbsentF;
+      }
+      cut_nodes += hop_new - cap_new;
+      if (!grid.wait()) return;
+    }
+    const int64_t kept = hop_new < cap_new ? hop_new : cap_new;
+    base += frontier;
+    frontier = kept;
+    nodes += kept;
+    const int64_t e_end = e_off + hop_draws;
+    if (e_end > p.edge_cap) cut_edges += e_end - (e_off > p.edge_cap ? e_off : p.edge_cap);
+    e_off = e_end;
+    __syncthreads();                   // row_at is reused
   }
-}
-
-// local ids of the nodes that got a row; the claims of cut nodes are withdrawn
-__global__ void fixed_assign_kernel(const FixedPlan p, int* local_map, int64_t row0, int64_t cap_new) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= p.state[4]) return;
-  const int64_t v = p.new_nodes[r];
-  if (v >= 0) local_map[v] = (int)(row0 + r);
-}
-
-// edges of this hop into idx (behind the edges of the earlier hops) and the rows' ptr entries
-__global__ void fixed_translate_kernel(const FixedPlan p, const int* __restrict__ local_map, int64_t fs, int64_t nf,
-                                       int fanout) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t i = t / fanout;
-  const int j = (int)(t % fanout);
-  if (i >= nf) return;
-  const int64_t e_off = p.state[1];
-  const int64_t o = p.cnt[i];
-  if (j == 0) {
-    const int64_t at = e_off + o;
-    p.ptr[fs + i] = at < p.edge_cap ? at : p.edge_cap;
+  if (!grid.wait()) return;
+  for (int64_t i = gtid; i < total; i += threads)
+    if (__ldcg(p.mask + i)) p.local_map[__ldcg(p.sub_to_full + i)] = kAbsentF;
+  if (gtid == 0) {
+    p.ptr[p.caps[p.num_hops - 1]] = e_off < p.edge_cap ? e_off : p.edge_cap;
+    p.counters[0] = nodes;
+    p.counters[1] = e_off < p.edge_cap ? e_off : p.edge_cap;
+    p.counters[2] = cut_nodes;
+    p.counters[3] = cut_edges;
+    p.batch_no[0] += 1;
   }
-  if (j >= p.cnt[i + 1] - o) return;
-  const int64_t e = e_off + o + j;
-  if (e >= p.edge_cap) {
-    atomicAdd(reinterpret_cast<unsigned long long*>(p.counters + 3), 1ull);
-    return;
-  }
-  const int loc = local_map[p.nbr[o + j]];
-  // a node that was cut has no row: the edge becomes a self loop of its destination row
-  p.idx[e] = loc >= 0 ? (int64_t)loc : fs + i;
-}
-
-__global__ void fixed_unclaim_kernel(const FixedPlan p, int* local_map) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= p.state[4]) return;
-  const int64_t v = p.new_nodes[r];
-  if (v < 0) {
-    local_map[-1 - v] = kAbsentF;
-    atomicAdd(reinterpret_cast<unsigned long long*>(p.counters + 2), 1ull);
-  }
-}
-
-__global__ void fixed_hop_end_kernel(const FixedPlan p, int64_t cap_new, int last, int64_t ptr_end_row) {
-  // advance the device-side offsets for the next hop
-  const int64_t edges = p.state[3];
-  int64_t kept = p.state[4] < cap_new ? p.state[4] : cap_new;
-  int64_t e_off = p.state[1] + edges;
-  p.state[2] += p.state[5];          // frontier base: real nodes of the frontier just expanded
-  p.state[5] = kept;                 // size of the next frontier
-  p.state[1] = e_off;
-  p.counters[0] += kept;
-  p.counters[1] = e_off < p.edge_cap ? e_off : p.edge_cap;
-  if (last) p.ptr[ptr_end_row] = e_off < p.edge_cap ? e_off : p.edge_cap;
-}
-
-__global__ void fixed_finish_kernel(const FixedPlan p, int* local_map) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < p.caps[p.num_hops] && p.mask[i]) local_map[p.sub_to_full[i]] = kAbsentF;
 }
 
 }  // namespace hc
@@ -266,14 +299,19 @@ static int64_t max_draws(const hc_fixed_batch* b) {
   return m;
 }
 
+// rows of a block, and whether they need memory behind the draws
+static int sample_rows(const hc_fixed_batch* b) { return (int)ceil_div(max_frontier(b), kSampleBlocks); }
+static constexpr int kSampleSharedRows = 8 * 1024;
+
 extern "C" int64_t hc_sample_fixed_scratch_bytes(const hc_fixed_batch* b) {
   if (!b || b->num_hops < 1 || b->num_hops > kMaxHops) return 0;
-  const int64_t draws = max_draws(b);
-  return (16 + (max_frontier(b) + 2) + 2 * (draws + 1) + (draws / 1024 + 2)) * (int64_t)sizeof(int64_t);
+  const int64_t rows = sample_rows(b);
+  return 64 + 2 * kSampleBlocks * (int64_t)sizeof(int) + 2 * (max_draws(b) + 1) * (int64_t)sizeof(int64_t) +
+         (rows > kSampleSharedRows ? rows * kSampleBlocks * (int64_t)sizeof(int) : 0);
 }
 
-extern "C" int hc_sample_fixed(const int64_t* gptr, const int64_t* gidx, const int64_t* seeds, int64_t n_seeds,
-                               int32_t* local_map, uint64_t seed, int64_t* batch_no,
+extern "C" int hc_sample_batch(const int64_t* gptr, const int64_t* gidx, const int64_t* seeds, int64_t n_seeds,
+                               int32_t* local_map, uint64_t seed, int64_t* batch_no, const int64_t* labels, int64_t* y,
                                const hc_fixed_batch* b, void* scratch, void* stream) {
   HC_REQUIRE(b != nullptr, HC_ERR_NULL);
   HC_REQUIRE(b->struct_size == sizeof(hc_fixed_batch), HC_ERR_STRUCT);
@@ -281,53 +319,38 @@ extern "C" int hc_sample_fixed(const int64_t* gptr, const int64_t* gidx, const i
   HC_REQUIRE(n_seeds >= 0 && n_seeds <= b->caps[0] && b->edge_cap >= 0, HC_ERR_SIZE);
   for (int h = 0; h < b->num_hops; ++h)
     HC_REQUIRE(b->fanout[h] >= 1 && b->caps[h + 1] >= b->caps[h] && b->caps[h] >= 0, HC_ERR_SIZE);
-  HC_REQUIRE(b->caps[b->num_hops] < 0x7fffffffLL, HC_ERR_SIZE);
+  HC_REQUIRE(b->caps[b->num_hops] < 0x7fffffffLL && max_draws(b) < 0x7ffffff0LL, HC_ERR_SIZE);
   HC_REQUIRE(gptr && gidx && local_map && batch_no && scratch && b->ptr && b->idx && b->sub_to_full && b->mask &&
-                 b->counters && (seeds || n_seeds == 0),
+                 b->counters && (seeds || n_seeds == 0) && (!y || labels),
              HC_ERR_NULL);
   HC_REQUIRE(aligned_to(scratch, 8), HC_ERR_ALIGN);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  FixedPlan p;
+  FixedPlan p{};
   p.num_hops = b->num_hops;
-  for (int h = 0; h < kMaxHops; ++h) p.fanout[h] = h < b->num_hops ? b->fanout[h] : 0;
-  for (int h = 0; h <= kMaxHops; ++h) p.caps[h] = h <= b->num_hops ? b->caps[h] : 0;
+  for (int h = 0; h < b->num_hops; ++h) p.fanout[h] = b->fanout[h];
+  for (int h = 0; h <= b->num_hops; ++h) p.caps[h] = b->caps[h];
   p.edge_cap = b->edge_cap;
   p.ptr = b->ptr; p.idx = b->idx; p.sub_to_full = b->sub_to_full; p.mask = b->mask; p.counters = b->counters;
-  const int64_t draws = max_draws(b), mf = max_frontier(b);
-  int64_t* w = reinterpret_cast<int64_t*>(scratch);
-  p.state = w; w += 16;
-  p.cnt = w; w += mf + 2;
-  p.nbr = w; w += draws + 1;
-  p.new_nodes = w; w += draws + 1;
-  p.block_counts = w;
-  const int64_t total = p.caps[p.num_hops];
-  auto blocks = [](int64_t n, int per) { return (unsigned)ceil_div(n > 0 ? n : 1, per); };
-  if (p.edge_cap > 0) HC_CUDA(cudaMemsetAsync(p.idx, 0, (size_t)p.edge_cap * sizeof(int64_t), st));
-  fixed_begin_kernel<<<blocks(total, 256), 256, 0, st>>>(p, seeds, n_seeds, local_map, seed, batch_no);
-  // state[5] = size of the current frontier (real nodes)
-  HC_CUDA(cudaMemcpyAsync(p.state + 5, b->counters, sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
-  for (int h = 0; h < p.num_hops; ++h) {
-    const int64_t fs = h == 0 ? 0 : p.caps[h - 1];
-    const int64_t nf = p.caps[h] - fs;                  // frontier capacity (rows [fs, caps[h]))
-    const int64_t row0 = p.caps[h];                     // the new nodes' first row
-    const int64_t cap_new = p.caps[h + 1] - p.caps[h];
-    const int fan = p.fanout[h];
-    const int64_t m = nf * fan;                         // draw capacity of this hop
-    if (nf == 0) continue;
-    fixed_counts_kernel<<<blocks(nf, 256), 256, 0, st>>>(p, gptr, fs, nf, fan);
-    fixed_scan_kernel<<<1, 1024, 0, st>>>(p, nf);
-    fixed_picks_kernel<<<blocks(m, 256), 256, 0, st>>>(p, gptr, gidx, fs, nf, fan);
-    fixed_claim_kernel<<<blocks(m, 256), 256, 0, st>>>(p, local_map);
-    const unsigned nb = blocks(m, 1024);
-    fixed_first_count_kernel<<<nb, 1024, 0, st>>>(p, local_map);
-    fixed_first_scan_kernel<<<1, 1024, 0, st>>>(p, nb);
-    fixed_place_kernel<<<nb, 1024, 0, st>>>(p, local_map, row0, cap_new);
-    fixed_assign_kernel<<<blocks(m, 256), 256, 0, st>>>(p, local_map, row0, cap_new);
-    fixed_translate_kernel<<<blocks(m, 256), 256, 0, st>>>(p, local_map, fs, nf, fan);
-    fixed_unclaim_kernel<<<blocks(m, 256), 256, 0, st>>>(p, local_map);
-    fixed_hop_end_kernel<<<1, 1, 0, st>>>(p, cap_new, h == p.num_hops - 1 ? 1 : 0, p.caps[p.num_hops - 1]);
+  p.gptr = gptr; p.gidx = gidx; p.seeds = seeds; p.n_seeds = n_seeds; p.local_map = local_map;
+  p.seed = seed; p.batch_no = batch_no; p.labels = labels; p.y = y;
+  char* w = reinterpret_cast<char*>(scratch);
+  const int64_t draws = max_draws(b);
+  p.barrier = reinterpret_cast<unsigned*>(w); w += 64;
+  p.nbr[0] = reinterpret_cast<int64_t*>(w); w += (draws + 1) * sizeof(int64_t);
+  p.nbr[1] = reinterpret_cast<int64_t*>(w); w += (draws + 1) * sizeof(int64_t);
+  p.draws = reinterpret_cast<int*>(w); w += kSampleBlocks * sizeof(int);
+  p.firsts = reinterpret_cast<int*>(w); w += kSampleBlocks * sizeof(int);
+  const int rows = sample_rows(b);
+  size_t smem = (size_t)rows * sizeof(int);
+  if (rows > kSampleSharedRows) {
+    p.row_at = reinterpret_cast<int*>(w);
+    smem = 0;
   }
-  fixed_finish_kernel<<<blocks(total, 256), 256, 0, st>>>(p, local_map);
-  HC_LAUNCH_OK();
-  return 0;
+  return launch_together(sample_fixed_kernel, kSampleBlocks, kSampleThreads, smem, p.barrier, st, p, rows);
+}
+
+extern "C" int hc_sample_fixed(const int64_t* gptr, const int64_t* gidx, const int64_t* seeds, int64_t n_seeds,
+                               int32_t* local_map, uint64_t seed, int64_t* batch_no,
+                               const hc_fixed_batch* b, void* scratch, void* stream) {
+  return hc_sample_batch(gptr, gidx, seeds, n_seeds, local_map, seed, batch_no, nullptr, nullptr, b, scratch, stream);
 }

@@ -40,6 +40,15 @@ namespace {
   X(hc_error_string) X(hc_aggr_fwd) X(hc_aggr_bwd) X(hc_transpose_scratch_bytes)                   \
   X(hc_transpose_block) X(hc_gather_scratch_bytes) X(hc_aggr_bwd_gather)                           \
   X(hc_aggr_bwd_source_scratch_bytes) X(hc_aggr_bwd_source) X(hc_norm_scratch_bytes)               \
+  X(hc_score_rows) X(hc_select_scratch_bytes) X(hc_select_threshold)                               \
+  X(hc_select_threshold_counted) X(hc_select_threshold_masked) X(hc_admit_scratch_bytes)           \
+  X(hc_record_history_masked) X(hc_cache_admit) X(hc_evict_stale) X(hc_evict_stale_dev)            \
+  X(hc_evict_by_score) X(hc_evict_both) X(hc_stamp_checkin) X(hc_used_masks_scratch_bytes)         \
+  X(hc_used_masks_together) X(hc_count_num) X(hc_map_lookup) X(hc_map_lookup_masked)               \
+  X(hc_cache_lookup) X(hc_gather_rows) X(hc_load_rows) X(hc_load_rows_staged)                      \
+  X(hc_stage_host_rows) X(hc_sample_fixed_scratch_bytes) X(hc_sample_batch) X(hc_sample_counts)    \
+  X(hc_sample_picks) X(hc_relabel_scratch_bytes) X(hc_relabel) X(hc_relabel_seed)                  \
+  X(hc_relabel_reset) X(hc_edge_types) X(hc_rgcn_group_scratch_bytes) X(hc_rgcn_group)             \
   X(hc_norm_act_fwd) X(hc_norm_act_bwd)
 
 struct Lib {
@@ -618,6 +627,517 @@ Tensor norm_act(const Tensor& x_in, const OptTensor& weight, const OptTensor& bi
   return y;
 }
 
+
+// ---------------------------------------------------------------------------
+// scores, threshold, admission, eviction
+// ---------------------------------------------------------------------------
+#define HC_ON(dev) c10::cuda::CUDAGuard guard_(dev)
+
+Tensor f32_rows(const Tensor& t) {
+  Tensor x = rows2d(t);
+  return x.scalar_type() == at::kFloat ? x : x.to(at::kFloat);
+}
+// a row mask: one byte per row
+Tensor byte_mask(const OptTensor& m, int64_t n, const char* what) {
+  Tensor t = some(m);
+  if (!t.defined()) return t;
+  TORCH_CHECK(t.element_size() == 1 && t.size(0) >= n, what, " must have one byte per row");
+  return t.is_contiguous() ? t : t.contiguous();
+}
+
+Tensor score_rows(const Tensor& x_in, int kind, const OptTensor& out_in) {
+  const at::Device dev = require_cuda(x_in);
+  HC_ON(dev);
+  at::NoGradGuard no_grad;
+  const Tensor x = f32_rows(x_in);
+  const int64_t n = x.size(0), F = x.size(1);
+  Tensor out = out_in ? *out_in : new_f32({n}, dev);
+  {
+    HC_SPAN("hc_score_rows", dev);
+    check(lib.hc_score_rows(fdata(x), n, (int32_t)F, row_stride(x, F), kind, fdata(out), stream_of(dev)), "hc_score_rows");
+  }
+  ++g_launches;
+  return out;
+}
+
+Tensor select_threshold(const Tensor& score_in, double q, const OptTensor& out_in, const OptTensor& n_valid,
+                        const OptTensor& valid_in) {
+  const at::Device dev = require_cuda(score_in);
+  HC_ON(dev);
+  const Tensor score = score_in.contiguous();
+  if (score.scalar_type() != at::kFloat) throw py::type_error("select_threshold: scores must be float32");
+  Tensor out = out_in ? *out_in : new_f32({1}, dev);
+  const int64_t n = score.size(0), bytes = lib.hc_select_scratch_bytes(n);
+  const Tensor valid = byte_mask(valid_in, n, "select_threshold: valid");
+  Tensor sc;
+  if (bytes) sc = new_scratch(bytes, dev);
+  {
+    HC_SPAN("hc_select_threshold", dev);
+    if (valid.defined())
+      check(lib.hc_select_threshold_masked(fdata(score), data<uint8_t>(valid), n, (float)q, fdata(out), data(sc),
+                                           stream_of(dev)), "hc_select_threshold_masked");
+    else if (n_valid)
+      check(lib.hc_select_threshold_counted(fdata(score), n, idata(*n_valid), (float)q, fdata(out), data(sc),
+                                            stream_of(dev)), "hc_select_threshold_counted");
+    else
+      check(lib.hc_select_threshold(fdata(score), n, (float)q, fdata(out), data(sc), stream_of(dev)),
+            "hc_select_threshold");
+  }
+  g_launches += bytes ? 9 : 1;
+  return out;
+}
+
+void record_history(const Tensor& new_in, const Tensor& buffer_all, const OptTensor& used_in, const Tensor& sub_to_full,
+                    const Tensor& sub_to_history, const Tensor& history_to_full, const Tensor& full_to_history,
+                    const Tensor& header, const Tensor& score_in, const Tensor& thres_in, const Tensor& checkin_iter,
+                    int64_t glb_iter, const OptTensor& n_admitted, const OptTensor& valid_in) {
+  const at::Device dev = require_cuda(new_in, buffer_all, sub_to_full, sub_to_history, history_to_full, full_to_history,
+                                      header, score_in, thres_in, checkin_iter);
+  HC_ON(dev);
+  at::NoGradGuard no_grad;
+  const Tensor rows = f32_rows(new_in);
+  const int64_t n = rows.size(0), hs = rows.size(1);
+  TORCH_CHECK(buffer_all.is_contiguous(), "record_history: buffer_all must be contiguous");
+  TORCH_CHECK(buffer_all.size(1) == hs, "record_history: row widths differ");
+  const std::pair<const char*, const Tensor*> maps[] = {{"history_to_full", &history_to_full},
+                                                        {"full_to_history", &full_to_history},
+                                                        {"header", &header},
+                                                        {"checkin_iter", &checkin_iter}};
+  for (auto& m : maps)
+    if (m.second->scalar_type() != at::kLong || !m.second->is_contiguous())
+      throw py::type_error(std::string("record_history: ") + m.first + " must be contiguous int64");
+  Tensor used = some(used_in);
+  if (used.defined()) {
+    if (used.scalar_type() != at::kBool && used.scalar_type() != at::kByte)
+      throw py::type_error("record_history: used_mask must be bool");
+    used = used.contiguous();
+    TORCH_CHECK(used.size(0) >= n, "record_history: used_mask shorter than buffer_new");
+  }
+  const Tensor valid = byte_mask(valid_in, n, "record_history: valid");
+  TORCH_CHECK(sub_to_full.size(0) >= n && sub_to_history.size(0) >= n && score_in.size(0) >= n,
+              "record_history: per-row arguments shorter than buffer_new");
+  const Tensor thres = thres_in.scalar_type() == at::kFloat ? thres_in : thres_in.to(at::kFloat);
+  const Tensor score = (score_in.scalar_type() == at::kFloat ? score_in : score_in.to(at::kFloat)).contiguous();
+  const Tensor s2f = i64c(sub_to_full), s2h = i64c(sub_to_history);
+  Tensor sc = new_scratch(lib.hc_admit_scratch_bytes(n), dev);
+  {
+    HC_SPAN("hc_record_history", dev);
+    check(lib.hc_record_history_masked(fdata(rows), row_stride(rows, hs), n, data(buffer_all), dtype_code(buffer_all),
+                                       buffer_all.size(0), (int32_t)hs, data<uint8_t>(used), data<uint8_t>(valid),
+                                       idata(s2f), idata(s2h), data<int64_t>(history_to_full),
+                                       data<int64_t>(full_to_history), data<int64_t>(header), fdata(score),
+                                       fdata(thres), data<int64_t>(checkin_iter), glb_iter,
+                                       n_admitted ? data<int64_t>(*n_admitted) : nullptr, data(sc), stream_of(dev)),
+          "hc_record_history");
+  }
+  ++g_launches;
+}
+
+void cache_admit(const Tensor& produced, const Tensor& buffer, int64_t hidden, int64_t in_feat, int64_t embed_capacity,
+                 const Tensor& sub_to_full, const Tensor& sub2embed, const Tensor& score, const Tensor& thres,
+                 const Tensor& full2embed, int64_t total_num_node, const Tensor& embed2full, const OptTensor& feat2full,
+                 const Tensor& header, bool reset_header, const OptTensor& n_admitted, const OptTensor& valid) {
+  const at::Device dev = require_cuda(produced, buffer, sub_to_full, sub2embed, score, thres, full2embed, embed2full, header);
+  HC_ON(dev);
+  at::NoGradGuard no_grad;
+  const Tensor rows = f32_rows(produced);
+  const int64_t n = rows.size(0);
+  const Tensor s2f = i64c(sub_to_full), s2e = i64c(sub2embed), f2f = some(feat2full), v = some(valid);
+  Tensor sc = new_scratch(lib.hc_admit_scratch_bytes(n), dev);
+  {
+    HC_SPAN("hc_cache_admit", dev);
+    check(lib.hc_cache_admit(fdata(rows), row_stride(rows, hidden), n, data(buffer), dtype_code(buffer), (int32_t)hidden,
+                             (int32_t)in_feat, embed_capacity, idata(s2f), idata(s2e), fdata(score), fdata(thres),
+                             data<int64_t>(full2embed), total_num_node, data<int64_t>(embed2full), idata(f2f),
+                             f2f.defined() ? f2f.size(0) : 0, data<int64_t>(header), reset_header ? 1 : 0,
+                             data<uint8_t>(v), n_admitted ? data<int64_t>(*n_admitted) : nullptr, data(sc),
+                             stream_of(dev)),
+          "hc_cache_admit");
+  }
+  ++g_launches;
+}
+
+void evict_stale(const Tensor& checkin, const Tensor& h2f, const Tensor& f2h, int64_t glb_iter, int64_t limit) {
+  const at::Device dev = require_cuda(checkin, h2f, f2h);
+  HC_ON(dev);
+  HC_SPAN("hc_evict_stale", dev);
+  check(lib.hc_evict_stale(data<int64_t>(checkin), data<int64_t>(h2f), data<int64_t>(f2h), checkin.size(0), glb_iter, limit,
+                           stream_of(dev)), "hc_evict_stale");
+  ++g_launches;
+}
+void evict_stale_dev(const Tensor& checkin, const Tensor& h2f, const Tensor& f2h, const Tensor& iter_dev, int64_t limit) {
+  const at::Device dev = require_cuda(checkin, h2f, f2h, iter_dev);
+  HC_ON(dev);
+  HC_SPAN("hc_evict_stale", dev);
+  check(lib.hc_evict_stale_dev(data<int64_t>(checkin), data<int64_t>(h2f), data<int64_t>(f2h), checkin.size(0),
+                               idata(iter_dev), limit, stream_of(dev)), "hc_evict_stale_dev");
+  ++g_launches;
+}
+void stamp_checkin(const Tensor& checkin, const Tensor& iter_dev, int64_t marker) {
+  const at::Device dev = require_cuda(checkin, iter_dev);
+  HC_ON(dev);
+  HC_SPAN("hc_stamp_checkin", dev);
+  check(lib.hc_stamp_checkin(data<int64_t>(checkin), checkin.size(0), marker, idata(iter_dev), stream_of(dev)),
+        "hc_stamp_checkin");
+  ++g_launches;
+}
+void evict_by_score(const Tensor& s2h_in, const Tensor& score_in, const Tensor& thres, const Tensor& checkin,
+                    const Tensor& h2f, const Tensor& f2h) {
+  const at::Device dev = require_cuda(s2h_in, score_in, thres, checkin);
+  HC_ON(dev);
+  const Tensor s2h = i64c(s2h_in), score = score_in.contiguous();
+  HC_SPAN("hc_evict_by_score", dev);
+  check(lib.hc_evict_by_score(idata(s2h), fdata(score), fdata(thres), std::min(s2h.size(0), score.size(0)),
+                              data<int64_t>(checkin), data<int64_t>(h2f), data<int64_t>(f2h), stream_of(dev)),
+        "hc_evict_by_score");
+  ++g_launches;
+}
+// evict_by_score and the eviction by age in one launch; iter_dev (or None) replaces glb_iter
+void evict_both(const Tensor& s2h_in, const Tensor& score_in, const Tensor& thres, const Tensor& checkin,
+                const Tensor& h2f, const Tensor& f2h, int64_t glb_iter, const OptTensor& iter_dev, int64_t limit) {
+  const at::Device dev = require_cuda(s2h_in, score_in, thres, checkin, h2f, f2h, iter_dev);
+  HC_ON(dev);
+  const Tensor s2h = i64c(s2h_in), score = score_in.contiguous();
+  HC_SPAN("hc_evict_both", dev);
+  check(lib.hc_evict_both(idata(s2h), fdata(score), fdata(thres), std::min(s2h.size(0), score.size(0)),
+                          data<int64_t>(checkin), data<int64_t>(h2f), data<int64_t>(f2h), checkin.size(0), glb_iter,
+                          iter_dev ? idata(*iter_dev) : nullptr, limit, stream_of(dev)),
+        "hc_evict_both");
+  ++g_launches;
+}
+
+// ---------------------------------------------------------------------------
+// receptive-field bookkeeping, lookup, row assembly
+// ---------------------------------------------------------------------------
+std::vector<Tensor> used_masks(const Tensor& ptr_in, const Tensor& idx_in, const OptTensor& maps, int64_t num_node,
+                               int64_t num_seed, int num_layer) {
+  const at::Device dev = require_cuda(ptr_in, idx_in);
+  HC_ON(dev);
+  const Tensor ptr = i64c(ptr_in, "ptr"), idx = i64c(idx_in, "idx"), hm = i64c(some_nonempty(maps), "history_maps");
+  Tensor buf = new_cuda({num_layer + 1, num_node}, at::kBool, dev);
+  Tensor sc = new_scratch(lib.hc_used_masks_scratch_bytes(), dev);
+  {
+    HC_SPAN("hc_used_masks", dev);
+    check(lib.hc_used_masks_together(idata(ptr), idata(idx), ptr.size(0) - 1, idata(hm), hm.defined() ? hm.size(0) : 0,
+                                     num_node, num_seed, num_layer, data<uint8_t>(buf), data(sc), stream_of(dev)),
+          "hc_used_masks");
+  }
+  ++g_launches;
+  return buf.unbind(0);
+}
+
+Tensor count_num(const Tensor& arr_in, int64_t mmax) {
+  const at::Device dev = require_cuda(arr_in);
+  HC_ON(dev);
+  const Tensor arr = i64c(arr_in, "arr");
+  Tensor out = new_cuda({mmax + 1}, at::kInt, dev);
+  HC_SPAN("hc_count_num", dev);
+  check(lib.hc_count_num(idata(arr), arr.size(0), mmax, data<int32_t>(out), stream_of(dev)), "hc_count_num");
+  ++g_launches;
+  return out;
+}
+
+Tensor map_lookup(const Tensor& map, const Tensor& ids_in, int64_t offset, int64_t force_miss_below,
+                  const OptTensor& out_in, const OptTensor& valid_in) {
+  const at::Device dev = require_cuda(map, ids_in);
+  HC_ON(dev);
+  const Tensor ids = i64c(ids_in, "ids");
+  const int64_t n = ids.size(0);
+  const Tensor valid = byte_mask(valid_in, n, "map_lookup: valid");
+  Tensor out = out_in ? *out_in : new_i64({n}, dev);
+  {
+    HC_SPAN("hc_map_lookup", dev);
+    if (valid.defined()) {
+      TORCH_CHECK(offset == 0, "map_lookup: a row mask needs offset 0");
+      check(lib.hc_map_lookup_masked(idata(map), map.size(0), idata(ids), n, force_miss_below, data<uint8_t>(valid),
+                                     data<int64_t>(out), stream_of(dev)), "hc_map_lookup_masked");
+    } else {
+      check(lib.hc_map_lookup(idata(map), map.size(0), idata(ids), n, offset, force_miss_below, data<int64_t>(out),
+                              stream_of(dev)), "hc_map_lookup");
+    }
+  }
+  ++g_launches;
+  return out;
+}
+
+// (sub2embed [n1], sub2feat [n])
+std::tuple<Tensor, Tensor> cache_lookup(const Tensor& map, const Tensor& ids_in, int64_t n1, int64_t offset) {
+  const at::Device dev = require_cuda(map, ids_in);
+  HC_ON(dev);
+  const Tensor ids = i64c(ids_in, "ids");
+  const int64_t n = ids.size(0);
+  Tensor embed = new_i64({n1}, dev), feat = new_i64({n}, dev);
+  {
+    HC_SPAN("hc_cache_lookup", dev);
+    check(lib.hc_cache_lookup(idata(map), map.size(0), idata(ids), n, n1, offset, data<int64_t>(embed), data<int64_t>(feat),
+                              stream_of(dev)), "hc_cache_lookup");
+  }
+  ++g_launches;
+  return {embed, feat};
+}
+
+Tensor gather_rows(const Tensor& table_in, const Tensor& rows_in, bool zero_missing, const std::optional<at::ScalarType>& type) {
+  const at::Device dev = require_cuda(table_in, rows_in);
+  HC_ON(dev);
+  at::NoGradGuard no_grad;
+  const Tensor table = rows2d(table_in), rows = i64c(rows_in, "rows");
+  const int64_t n = rows.size(0), F = table.size(1);
+  Tensor out = new_cuda({n, F}, type ? *type : table.scalar_type(), dev);
+  HC_SPAN("hc_gather_rows", dev);
+  check(lib.hc_gather_rows(data(table), dtype_code(table), table.size(0), row_stride(table, F), (int32_t)F, idata(rows), n,
+                           zero_missing ? 1 : 0, data(out), dtype_code(out), F, stream_of(dev)), "hc_gather_rows");
+  ++g_launches;
+  return out;
+}
+
+py::object load_rows(const Tensor& host_in, const OptTensor& cache_in, const Tensor& ids_in, const OptTensor& feat_in,
+                     const OptTensor& used_in, const std::optional<at::ScalarType>& type, bool want_mask,
+                     const OptTensor& stats, const OptTensor& out_in, const OptTensor& mask_out,
+                     const std::optional<std::tuple<Tensor, Tensor>>& staged) {
+  Where w;
+  w.add(ids_in).add(feat_in).add(used_in).add(cache_in).add(out_in).add(mask_out);
+  if (host_in.is_cuda()) w.add(host_in);
+  TORCH_CHECK(w.any, "hiscache_backend: no CUDA tensor given");
+  const at::Device dev = w.dev;
+  HC_ON(dev);
+  at::NoGradGuard no_grad;
+  TORCH_CHECK(host_in.is_cuda() || host_in.is_pinned(), "load_rows: a host feature table must be pinned memory");
+  const Tensor host = rows2d(host_in), ids = i64c(ids_in, "sub_to_full"), s2f = i64c(some(feat_in), "sub2feat");
+  const int64_t n = ids.size(0), F = host.size(1);
+  const at::ScalarType dt = type ? *type : host.scalar_type();
+  Tensor x = some(out_in), mask = some(mask_out), used = some(used_in), cache = some(cache_in);
+  if (x.defined()) {
+    if (x.dim() != 2 || x.size(0) != n || x.size(1) != F || x.scalar_type() != dt || !x.is_contiguous())
+      throw py::value_error("load_rows: out must be a contiguous [" + std::to_string(n) + ", " + std::to_string(F) +
+                            "] tensor of the batch's type");
+  } else {
+    x = new_cuda({n, F}, dt, dev);
+  }
+  if (mask.defined()) {
+    if (mask.scalar_type() != at::kByte || mask.size(0) != n || !mask.is_contiguous())
+      throw py::value_error("load_rows: mask_out must be a contiguous uint8 tensor of " + std::to_string(n) + " entries");
+  } else if (want_mask) {
+    mask = new_cuda({n}, at::kByte, dev);
+  }
+  if (used.defined()) {
+    used = used.contiguous();
+    if (used.size(0) != n || used.element_size() != 1)
+      throw py::value_error("load_rows: used must have " + std::to_string(n) + " one-byte entries");
+  }
+  int cd = HC_F32;
+  int64_t cr = 0, cs = 0;
+  if (cache.defined()) {
+    cache = rows2d(cache);
+    cd = dtype_code(cache);
+    cr = cache.size(0);
+    cs = row_stride(cache, F);
+  }
+  int64_t* st = stats ? data<int64_t>(*stats) : nullptr;
+  {
+    HC_SPAN("hc_load_rows", dev);
+    if (!staged) {
+      check(lib.hc_load_rows(data(host), dtype_code(host), host.size(0), row_stride(host, F), data(cache), cd, cr, cs,
+                             (int32_t)F, idata(ids), idata(s2f), data<uint8_t>(used), n, data(x), dtype_code(x), F,
+                             data<uint8_t>(mask), st, stream_of(dev)), "hc_load_rows");
+    } else {
+      const Tensor &sr = std::get<0>(*staged), &sm = std::get<1>(*staged);
+      require_cuda(sr, sm);
+      if (sr.dim() != 2 || sr.size(0) != n || sr.size(1) != F || sr.scalar_type() != x.scalar_type() ||
+          !sr.is_contiguous() || sm.scalar_type() != at::kByte || sm.size(0) != n || !sm.is_contiguous())
+        throw py::value_error("load_rows: staged must be ([" + std::to_string(n) + ", " + std::to_string(F) +
+                              "] rows of the batch's type, [" + std::to_string(n) + "] uint8 mask)");
+      if (stats && stats->numel() < 3) throw py::value_error("load_rows: stats needs three counters when rows are staged");
+      check(lib.hc_load_rows_staged(data(host), dtype_code(host), host.size(0), row_stride(host, F), data(cache), cd, cr, cs,
+                                    (int32_t)F, idata(ids), idata(s2f), data<uint8_t>(used), n, data(x), dtype_code(x), F,
+                                    data<uint8_t>(mask), st, data(sr), data<uint8_t>(sm), stream_of(dev)),
+            "hc_load_rows_staged");
+    }
+  }
+  ++g_launches;
+  if (want_mask) return py::make_tuple(x, mask.view(at::kBool));
+  return py::cast(x);
+}
+
+void stage_host_rows(const Tensor& host_in, const Tensor& ids_in, const OptTensor& feat_in, const OptTensor& consider_in,
+                     const Tensor& rows_out, const Tensor& mask_out, const OptTensor& stats, int64_t max_blocks) {
+  Where w;
+  w.add(ids_in).add(feat_in).add(consider_in).add(rows_out).add(mask_out);
+  if (host_in.is_cuda()) w.add(host_in);
+  TORCH_CHECK(w.any, "hiscache_backend: no CUDA tensor given");
+  const at::Device dev = w.dev;
+  HC_ON(dev);
+  TORCH_CHECK(host_in.is_cuda() || host_in.is_pinned(), "stage_host_rows: a host feature table must be pinned memory");
+  const Tensor host = rows2d(host_in), ids = i64c(ids_in, "ids"), s2f = i64c(some(feat_in), "sub2feat");
+  const int64_t n = ids.size(0), F = host.size(1);
+  if (s2f.defined() && s2f.size(0) != n)
+    throw py::value_error("stage_host_rows: sub2feat must have " + std::to_string(n) + " entries");
+  Tensor consider = some(consider_in);
+  if (consider.defined()) {
+    consider = consider.contiguous();
+    if (consider.size(0) != n || consider.element_size() != 1)
+      throw py::value_error("stage_host_rows: consider must have " + std::to_string(n) + " one-byte entries");
+  }
+  if (rows_out.dim() != 2 || rows_out.size(0) != n || rows_out.size(1) != F || rows_out.scalar_type() != host.scalar_type() ||
+      !rows_out.is_contiguous() || mask_out.scalar_type() != at::kByte || mask_out.size(0) != n || !mask_out.is_contiguous())
+    throw py::value_error("stage_host_rows: outputs must be [" + std::to_string(n) + ", " + std::to_string(F) +
+                          "] rows of the table's type and [" + std::to_string(n) + "] uint8 mask");
+  HC_SPAN("hc_stage_host_rows", dev);
+  check(lib.hc_stage_host_rows(data(host), dtype_code(host), host.size(0), row_stride(host, F), (int32_t)F, idata(ids),
+                               idata(s2f), data<uint8_t>(consider), n, data(rows_out), data<uint8_t>(mask_out),
+                               stats ? data<int64_t>(*stats) : nullptr, (int32_t)max_blocks, stream_of(dev)),
+        "hc_stage_host_rows");
+  ++g_launches;
+}
+
+// ---------------------------------------------------------------------------
+// sampling
+// ---------------------------------------------------------------------------
+void sample_batch(const Tensor& gptr, const Tensor& gidx, const Tensor& seeds_in, const Tensor& local_map, uint64_t seed,
+                  const Tensor& batch_no, const std::vector<int64_t>& fanouts, const std::vector<int64_t>& caps,
+                  int64_t edge_cap, const Tensor& ptr, const Tensor& idx, const Tensor& sub_to_full, const Tensor& mask,
+                  const Tensor& counters, const OptTensor& labels, const OptTensor& y) {
+  const at::Device dev = require_cuda(gptr, gidx, seeds_in, local_map, batch_no, ptr, idx, sub_to_full, mask, counters,
+                                      labels, y);
+  HC_ON(dev);
+  const Tensor seeds = i64c(seeds_in, "seeds");
+  hc_fixed_batch b{};
+  b.struct_size = sizeof(hc_fixed_batch);
+  const int64_t L = (int64_t)fanouts.size();
+  b.num_hops = (int32_t)L;
+  for (int64_t h = 0; h < L; ++h) b.fanout[h] = (int32_t)fanouts[h];
+  for (int64_t k = 0; k <= L; ++k) b.caps[k] = caps[k];
+  b.edge_cap = edge_cap;
+  TORCH_CHECK(ptr.numel() >= caps[L - 1] + 1 && idx.numel() >= edge_cap && sub_to_full.numel() >= caps[L] &&
+                  mask.numel() >= caps[L] && mask.element_size() == 1 && counters.numel() >= 4 &&
+                  (!y || y->numel() >= caps[0]),
+              "sample_fixed: an output is smaller than the batch's caps");
+  b.ptr = data<int64_t>(ptr);
+  b.idx = data<int64_t>(idx);
+  b.sub_to_full = data<int64_t>(sub_to_full);
+  b.mask = data<uint8_t>(mask);
+  b.counters = data<int64_t>(counters);
+  Tensor sc = new_scratch(lib.hc_sample_fixed_scratch_bytes(&b), dev);
+  HC_SPAN("hc_sample_fixed", dev);
+  check(lib.hc_sample_batch(idata(gptr), idata(gidx), idata(seeds), seeds.size(0), data<int32_t>(local_map), seed,
+                            data<int64_t>(batch_no), labels ? idata(*labels) : nullptr, y ? data<int64_t>(*y) : nullptr, &b,
+                            data(sc), stream_of(dev)),
+        "hc_sample_fixed");
+  ++g_launches;
+}
+
+py::tuple sample_hop(const Tensor& gptr, const Tensor& gidx, const Tensor& frontier_in, int64_t fanout, uint64_t seed,
+                     int64_t base) {
+  const at::Device dev = require_cuda(gptr, gidx, frontier_in);
+  HC_ON(dev);
+  const Tensor frontier = i64c(frontier_in, "frontier");
+  const int64_t nf = frontier.size(0);
+  Tensor out_ptr = at::zeros({nf + 1}, frontier.options());
+  Tensor counts = out_ptr.slice(0, 1);
+  {
+    HC_SPAN("hc_sample_counts", dev);
+    check(lib.hc_sample_counts(idata(gptr), idata(frontier), nf, (int32_t)fanout, data<int64_t>(counts), stream_of(dev)),
+          "hc_sample_counts");
+  }
+  at::cumsum_out(counts, counts, 0);
+  int64_t total = 0;
+  if (nf > 0) {
+    py::gil_scoped_release no_gil;
+    total = out_ptr[nf].item<int64_t>();
+  }
+  Tensor nbr = new_i64({total}, dev);
+  {
+    HC_SPAN("hc_sample_picks", dev);
+    check(lib.hc_sample_picks(idata(gptr), idata(gidx), idata(frontier), nf, (int32_t)fanout, idata(out_ptr), seed, base,
+                              data<int64_t>(nbr), stream_of(dev)), "hc_sample_picks");
+  }
+  g_launches += 2;
+  return py::make_tuple(out_ptr, nbr);
+}
+
+void relabel_seed(const Tensor& seeds_in, const Tensor& local_map) {
+  const at::Device dev = require_cuda(seeds_in, local_map);
+  HC_ON(dev);
+  const Tensor seeds = i64c(seeds_in);
+  check(lib.hc_relabel_seed(idata(seeds), seeds.size(0), data<int32_t>(local_map), stream_of(dev)), "hc_relabel_seed");
+  ++g_launches;
+}
+void relabel_reset(const Tensor& nodes_in, const Tensor& local_map) {
+  const at::Device dev = require_cuda(nodes_in, local_map);
+  HC_ON(dev);
+  const Tensor nodes = i64c(nodes_in);
+  check(lib.hc_relabel_reset(idata(nodes), nodes.size(0), data<int32_t>(local_map), stream_of(dev)), "hc_relabel_reset");
+  ++g_launches;
+}
+py::tuple relabel(const Tensor& nbr, const Tensor& local_map, int64_t n_total) {
+  const at::Device dev = require_cuda(nbr, local_map);
+  HC_ON(dev);
+  const int64_t m = nbr.size(0);
+  Tensor new_nodes = new_i64({std::max<int64_t>(m, 1)}, dev), n_new = at::zeros({1}, new_nodes.options());
+  Tensor out_idx = new_i64({m}, dev), sc = new_scratch(lib.hc_relabel_scratch_bytes(m), dev);
+  {
+    HC_SPAN("hc_relabel", dev);
+    check(lib.hc_relabel(idata(nbr), m, data<int32_t>(local_map), n_total, data<int64_t>(new_nodes), data<int64_t>(n_new),
+                         data<int64_t>(out_idx), data(sc), stream_of(dev)), "hc_relabel");
+  }
+  g_launches += 6;
+  int64_t n = 0;
+  {
+    py::gil_scoped_release no_gil;
+    n = n_new.item<int64_t>();
+  }
+  return py::make_tuple(new_nodes.slice(0, 0, n), out_idx);
+}
+
+// ---------------------------------------------------------------------------
+// heterogeneous layers
+// ---------------------------------------------------------------------------
+Tensor edge_types(const Tensor& ptr_in, const Tensor& idx_in, const Tensor& nodes_in, int64_t rows,
+                  const std::vector<int64_t>& bounds, const std::vector<int64_t>& rel_table) {
+  const at::Device dev = require_cuda(ptr_in, idx_in, nodes_in);
+  HC_ON(dev);
+  const int64_t T = (int64_t)bounds.size() - 1;
+  if (T < 1 || T > 8 || (int64_t)rel_table.size() != T * T)
+    throw py::value_error("edge_types: 1..8 node types, rel_table of n_types^2 entries");
+  const Tensor ptr = i64c(ptr_in), idx = i64c(idx_in), nodes = i64c(nodes_in);
+  Tensor out = new_i64({idx.size(0)}, dev);
+  if (idx.size(0) && rows < ptr.size(0) - 1) out.fill_(0);     // edges behind the rows asked for
+  const std::vector<int32_t> rel(rel_table.begin(), rel_table.end());
+  HC_SPAN("hc_edge_types", dev);
+  check(lib.hc_edge_types(idata(ptr), idata(idx), idata(nodes), rows, (int32_t)T, bounds.data(), rel.data(),
+                          data<int64_t>(out), stream_of(dev)), "hc_edge_types");
+  ++g_launches;
+  return out;
+}
+
+py::tuple rgcn_group(const Tensor& ptr_in, const Tensor& idx_in, const Tensor& etype_in, int64_t num_node, int64_t num_rel,
+                     const OptTensor& used_in, const OptTensor& hmap_in, bool want_perm, bool want_rel) {
+  const at::Device dev = require_cuda(ptr_in, idx_in, etype_in, used_in, hmap_in);
+  HC_ON(dev);
+  const Tensor ptr = i64c(ptr_in, "ptr"), idx = i64c(idx_in, "idx"), etype = i64c(etype_in, "edge_type"),
+               hmap = i64c(some(hmap_in));
+  const int64_t E = std::min(idx.size(0), etype.size(0)), room = std::max<int64_t>(E, 1);
+  TORCH_CHECK(ptr.size(0) >= num_node + 1, "rgcn_group: ptr shorter than num_node + 1");
+  TORCH_CHECK(!hmap.defined() || hmap.size(0) >= num_node, "rgcn_group: history map shorter than num_node");
+  Tensor used = some(used_in);
+  if (used.defined()) {
+    used = used.contiguous();
+    if (used.scalar_type() != at::kBool && used.scalar_type() != at::kByte)
+      throw py::type_error("rgcn_group: used mask must be bool");
+  }
+  Tensor ptr2 = new_i64({num_rel * num_node + 1}, dev), idx2 = new_i64({room}, dev), w2 = new_f32({room}, dev), perm, rel;
+  if (want_perm) perm = new_i64({room}, dev);
+  if (want_rel) rel = new_i64({room}, dev);
+  Tensor sc = new_scratch(lib.hc_rgcn_group_scratch_bytes(E), dev);
+  {
+    HC_SPAN("hc_rgcn_group", dev);
+    check(lib.hc_rgcn_group(idata(ptr), idata(idx), idata(etype), num_node, E, (int32_t)num_rel, data<uint8_t>(used),
+                            idata(hmap), data<int64_t>(ptr2), data<int64_t>(idx2), fdata(w2), data<int64_t>(perm),
+                            data<int64_t>(rel), data(sc), stream_of(dev)), "hc_rgcn_group");
+  }
+  g_launches += 7;
+  auto cut = [&](const Tensor& t) -> py::object { return t.defined() ? py::cast(t.slice(0, 0, E)) : py::none(); };
+  return py::make_tuple(ptr2, cut(idx2), cut(w2), cut(perm), cut(rel));
+}
 }  // namespace
 
 PYBIND11_MODULE(_native, m) {
@@ -648,4 +1168,75 @@ PYBIND11_MODULE(_native, m) {
     return py::make_tuple(t.t_ptr, t.t_dst, t.t_w, t.n_edges);
   });
   m.def("norm_act", &norm_act);
+  const py::object none = py::none();
+  m.def("score_rows", &score_rows, py::arg("x"), py::arg("kind") = HC_SCORE_L2, py::arg("out") = none,
+        "Per-row L2 / L1 norm in the library's fixed reduction order.");
+  m.def("select_threshold", &select_threshold, py::arg("score"), py::arg("q"), py::arg("out") = none,
+        py::arg("n_valid") = none, py::arg("valid") = none,
+        "torch.quantile(score, q) (linear interpolation) without leaving the device.  With n_valid (device int64[1]) "
+        "the quantile is over the n_valid smallest scores (padding rows carry +inf); with valid (one byte per row) "
+        "over the rows whose byte is set.");
+  m.def("record_history", &record_history, py::arg("buffer_new"), py::arg("buffer_all"), py::arg("used_mask"),
+        py::arg("sub_to_full"), py::arg("sub_to_history"), py::arg("history_to_full"), py::arg("full_to_history"),
+        py::arg("header"), py::arg("score"), py::arg("thres"), py::arg("checkin_iter"), py::arg("glb_iter"),
+        py::arg("n_admitted") = none, py::arg("valid") = none,
+        "src/cpp/src/grad_check.cu:48-68, same argument order; mutates buffer_all, both maps, header and checkin_iter "
+        "in place.  `thres` is a 1-element tensor.  valid: rows whose byte is 0 are never admitted.");
+  m.def("cache_admit", &cache_admit, py::arg("produced"), py::arg("buffer"), py::arg("hidden"), py::arg("in_feat"),
+        py::arg("embed_capacity"), py::arg("sub_to_full"), py::arg("sub2embed"), py::arg("score"), py::arg("thres"),
+        py::arg("full2embed"), py::arg("total_num_node"), py::arg("embed2full"), py::arg("feat2full"),
+        py::arg("header"), py::arg("reset_header") = false, py::arg("n_admitted") = none, py::arg("valid") = none,
+        "Device-side HistoryCache.update_history (hiscache/history_cache.py:211-254).");
+  m.def("evict_stale", &evict_stale, py::arg("checkin_iter"), py::arg("history_to_full"), py::arg("full_to_history"),
+        py::arg("glb_iter"), py::arg("limit"), "hiscache/history_table.py:189-200.");
+  m.def("evict_stale_dev", &evict_stale_dev, py::arg("checkin_iter"), py::arg("history_to_full"),
+        py::arg("full_to_history"), py::arg("iter_dev"), py::arg("limit"),
+        "evict_stale with the iteration number read from a device int64[1].");
+  m.def("stamp_checkin", &stamp_checkin, py::arg("checkin_iter"), py::arg("iter_dev"), py::arg("marker") = 1ll << 60,
+        "checkin_iter[checkin_iter == marker] = iter_dev[0].");
+  m.def("evict_by_score", &evict_by_score, py::arg("sub_to_history"), py::arg("score"), py::arg("thres"),
+        py::arg("checkin_iter"), py::arg("history_to_full"), py::arg("full_to_history"),
+        "hiscache/history_table.py:234-241.");
+  m.def("evict_both", &evict_both);
+  m.def("count_history_reconstruct", &used_masks, py::arg("ptr_t"), py::arg("idx_t"), py::arg("history_maps"),
+        py::arg("num_node"), py::arg("num_seed"), py::arg("num_layer"),
+        "src/cpp/src/grad_check.cu:103-130: list of num_layer+1 bool masks [num_node]; [num_layer] is the seed level, "
+        "[0] gates raw-feature loading.");
+  m.def("count_num", &count_num, py::arg("arr"), py::arg("mmax"),
+        "src/cpp/src/grad_check.cu:174-182: int32 histogram [mmax+1]; value 0 is not counted.");
+  m.def("map_lookup", &map_lookup, py::arg("map_t"), py::arg("ids"), py::arg("offset") = 0,
+        py::arg("force_miss_below") = 0, py::arg("out") = none, py::arg("valid") = none,
+        "out[i] = map[ids[i] + offset]; the first `force_miss_below` entries and rows whose byte of `valid` is 0 are -1.");
+  m.def("cache_lookup", &cache_lookup);
+  m.def("gather_rows", &gather_rows, py::arg("table"), py::arg("rows"), py::arg("zero_missing") = false,
+        py::arg("out_dtype") = none,
+        "table[rows] with torch's negative indexing (or zeros for -1 when zero_missing).");
+  m.def("load_rows", &load_rows, py::arg("host_table"), py::arg("feat_cache"), py::arg("sub_to_full"),
+        py::arg("sub2feat"), py::arg("used"), py::arg("out_dtype") = none, py::arg("want_mask") = false,
+        py::arg("stats") = none, py::arg("out") = none, py::arg("mask_out") = none, py::arg("staged") = none,
+        "One-pass batch.x assembly (hiscache/history_cache.py:327-350).  host_table may be a pinned host tensor (rows "
+        "are then read over the host link by the kernel) or a CUDA tensor.  Returns x, or (x, load_mask) when "
+        "want_mask.  out / mask_out: preallocated destinations ([n, F] rows, [n] uint8 mask).  staged = (rows [n, F], "
+        "mask [n] uint8): host rows fetched ahead of the step by `stage_host_rows`; a row whose mask is set is read "
+        "from there instead of host_table.  `stats` then needs three counters (host, cache, staged).");
+  m.def("stage_host_rows", &stage_host_rows);
+  m.def("sample_batch", &sample_batch);
+  m.def("sample_hop", &sample_hop, py::arg("gptr"), py::arg("gidx"), py::arg("frontier"), py::arg("fanout"),
+        py::arg("seed"), py::arg("base"),
+        "One hop of uniform sampling with replacement: (out_ptr [nf+1], nbr [total]) with min(fanout, degree) draws per "
+        "frontier node.  Reads one size back from the device.");
+  m.def("relabel_seed", &relabel_seed, py::arg("seeds"), py::arg("local_map"));
+  m.def("relabel_reset", &relabel_reset, py::arg("nodes"), py::arg("local_map"));
+  m.def("relabel", &relabel, py::arg("nbr"), py::arg("local_map"), py::arg("n_total"),
+        "(new_nodes [n_new], local ids of nbr): new nodes numbered from n_total in order of first occurrence.  Reads "
+        "n_new back from the device.");
+  m.def("edge_types", &edge_types, py::arg("ptr_t"), py::arg("idx_t"), py::arg("sub_to_full"), py::arg("rows"),
+        py::arg("type_bounds"), py::arg("rel_table"),
+        "etype[e] = rel_table[type(dst)][type(src)], node types being ranges of global ids: the counterpart of "
+        "cxgnncomp_backend.gen_edge_type_mag240m (hiscache/history_model.py:354-357).");
+  m.def("rgcn_group", &rgcn_group, py::arg("ptr_t"), py::arg("idx_t"), py::arg("etype"), py::arg("num_node"),
+        py::arg("num_rel"), py::arg("used_src") = none, py::arg("hmap") = none, py::arg("want_perm") = false,
+        py::arg("want_rel") = false,
+        "The relation-segmented block of one RGCN layer (hc_rgcn_group): (ptr2 [num_rel*num_node+1], idx2 [E], w2 [E], "
+        "perm or None, rel or None).");
 }

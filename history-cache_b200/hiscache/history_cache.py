@@ -196,9 +196,8 @@ class HistoryCache:
             self._cached_embedding = torch.tensor([])
             batch.x = self.uvm.get(batch.sub_to_full)
             return None
-        self.sub2embed = hb.map_lookup(self.full2embed, batch.sub_to_full[:n1])
+        self.sub2embed, self.sub2feat = hb.cache_lookup(self.full2embed, batch.sub_to_full, n1, N)
         self._cached_embedding = None
-        self.sub2feat = hb.map_lookup(self.full2embed, batch.sub_to_full, offset=N)
         self.used_masks = hb.count_history_reconstruct(batch.ptr, batch.idx, self.sub2embed,
                                                        batch.sub_to_full.shape[0], batch.y.shape[0],
                                                        num_layer)
@@ -266,16 +265,10 @@ class HistoryCache:
             score = torch.randn([num_node], device=self.device)
         self._sink = None
         prod.grad = None
-        valid = None
+        # fixed-shape batch: padding rows never count towards the quantile or get admitted
         mask = getattr(batch, "mask", None)
-        if mask is not None:
-            # fixed-shape batch: padding rows never count towards the quantile or get admitted
-            valid = mask[:num_node]
-            score = torch.where(valid, score, torch.full_like(score, float("inf")))
-            hb.select_threshold(score, self.rate, out=self._thres,
-                                n_valid=valid.sum(dtype=torch.int64).reshape(1))
-        else:
-            hb.select_threshold(score, self.rate, out=self._thres)
+        valid = None if mask is None else mask[:num_node]
+        hb.select_threshold(score, self.rate, out=self._thres, valid=valid)
         hb.cache_admit(prod.detach(), self.buffer, self.hidden_channels, self.in_channels,
                        self.overall_embed_num, batch.sub_to_full[:num_node], self.sub2embed, score,
                        self._thres, self.full2embed, self.total_num_node, self.embed2full,

@@ -101,11 +101,8 @@ class HistoryTable:
         num_seed = int(num_node_in_layer[0])
         for layer_id in range(self.num_layers):
             n = int(num_node_in_layer[self.num_layers_all - 1 - layer_id])
-            s2h = hb.map_lookup(self.full_to_history_layered[layer_id], sub_to_full[:n],
-                                force_miss_below=num_seed)
-            if valid is not None:
-                s2h = torch.where(valid[:n], s2h, torch.full_like(s2h, -1))
-            self.sub_to_history.append(s2h)
+            self.sub_to_history.append(hb.map_lookup(self.full_to_history_layered[layer_id], sub_to_full[:n],
+                                                     force_miss_below=num_seed, valid=valid))
 
     def _build_compact(self):
         bufs, maps = [], []
@@ -155,28 +152,21 @@ class HistoryTable:
             num_node = int(batch.num_node_in_layer[self.num_layers_all - 1 - layer_id])
             his = self.history_out[layer_id][:num_node]
             score = self._score(layer_id, batch, num_node)
-            used, thres = used_masks[layer_id + 1], self._threshold(score, self.rate, batch, num_node)
-            valid = getattr(batch, "mask", None)
-            if valid is not None:       # padding rows of a fixed-shape batch are never admitted
-                used = used[:num_node] & valid[:num_node]
+            thres = self._threshold(score, self.rate, batch)
             stamp = glb_iter if self.iter_dev is None else hb.CHECKIN_MARKER
             hb.record_history(his.detach(), self.history_buffer_layered[layer_id],
-                              used, sub_to_full, self.sub_to_history[layer_id],
+                              used_masks[layer_id + 1], sub_to_full, self.sub_to_history[layer_id],
                               self.history_to_full_layered[layer_id],
                               self.full_to_history_layered[layer_id],
                               self.cuda_header_layered[layer_id], score, thres,
-                              self.checkin_iter[layer_id], stamp)
+                              self.checkin_iter[layer_id], stamp,
+                              valid=getattr(batch, "mask", None))   # padding rows of a fixed-shape batch
             if self.iter_dev is not None:
                 hb.stamp_checkin(self.checkin_iter[layer_id], self.iter_dev)
 
-    def _threshold(self, score, q, batch, num_node):
+    def _threshold(self, score, q, batch):
         """torch.quantile(score, q) over the real rows of the batch (history_table.py:173,230)."""
-        valid = getattr(batch, "mask", None)
-        if valid is None:
-            return hb.select_threshold(score, q)
-        v = valid[:num_node]
-        padded = torch.where(v, score, torch.full_like(score, float("inf")))
-        return hb.select_threshold(padded, q, n_valid=v.sum(dtype=torch.int64).reshape(1))
+        return hb.select_threshold(score, q, valid=getattr(batch, "mask", None))
 
     def _evict_stale(self, layer_id, glb_iter, limit):
         if self.iter_dev is None:
@@ -204,11 +194,10 @@ class HistoryTable:
                 continue
             num_node = int(batch.num_node_in_layer[self.num_layers_all - 1 - layer_id])
             score = self._score(layer_id, batch, num_node)
-            thres = self._threshold(score, 1 - self.rate, batch, num_node)
-            hb.evict_by_score(self.sub_to_history[layer_id], score, thres, self.checkin_iter[layer_id],
-                              self.history_to_full_layered[layer_id],
-                              self.full_to_history_layered[layer_id])
-            self._evict_stale(layer_id, glb_iter, staleness_thres[layer_id])
+            thres = self._threshold(score, 1 - self.rate, batch)
+            hb.evict_both(self.sub_to_history[layer_id], score, thres, self.checkin_iter[layer_id],
+                          self.history_to_full_layered[layer_id], self.full_to_history_layered[layer_id],
+                          int(glb_iter), self.iter_dev, int(staleness_thres[layer_id]))
 
     def evict_history(self, batch, glb_iter):
         self.evict_by_both(batch, glb_iter, self.staleness_thres)

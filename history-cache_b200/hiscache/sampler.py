@@ -182,19 +182,17 @@ class NeighborSampler:
             out = {"ptr": pk.ptr, "idx": pk.idx, "sub_to_full": pk.sub_to_full, "mask": pk.mask, "y": pk.y,
                    "counters": torch.zeros(4, dtype=torch.int64, device=dev), "packed": pk.packed}
         o = hb.sample_fixed(g.ptr, g.idx, seeds, self.local, self.seed, self._batch_no_dev, self.fanouts,
-                            list(caps), int(edge_cap), out=out)
+                            list(caps), int(edge_cap), out=out, labels=g.labels)
         self.batch_no += 1
         self._batch_no_seen = int(self.batch_no)
         b = Batch()
         b.ptr, b.idx, b.sub_to_full, b.mask = o["ptr"], o["idx"][:int(edge_cap)], o["sub_to_full"], o["mask"]
-        if "y" not in o:
-            o["y"] = torch.full((caps[0],), -100, dtype=torch.int64, device=dev)
-        o["y"].fill_(-100)
-        o["y"][:seeds.shape[0]] = g.labels[seeds]
         b.y = o["y"]
         b.packed = o.get("packed")
-        b.num_node_in_layer = torch.tensor(list(caps), dtype=torch.int64)
-        b.num_edge_in_layer = torch.tensor([int(edge_cap)] * L, dtype=torch.int64)
+        if "layers" not in o:       # the sizes are the same for every batch of these buffers
+            o["layers"] = (torch.tensor(list(caps), dtype=torch.int64),
+                           torch.tensor([int(edge_cap)] * L, dtype=torch.int64))
+        b.num_node_in_layer, b.num_edge_in_layer = o["layers"]
         b.counters, b.fixed = o["counters"], o
         return b
 

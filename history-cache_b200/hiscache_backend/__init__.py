@@ -36,7 +36,7 @@ __all__ = [
     "aggr_forward", "score_rows", "record_history_noalloc", "select_threshold", "cache_admit", "evict_stale",
     "evict_by_score", "evict_stale_dev", "stamp_checkin", "CHECKIN_MARKER", "map_lookup", "gather_rows", "load_rows", "bucket_by_owner",
     "unpermute_rows", "owner_lookup", "bucket_pad", "unpad_hits", "last_occurrence", "sample_hop", "relabel", "relabel_seed",
-    "relabel_reset", "mix64", "launch_count", "ScoreSink", "KernelTimer",
+    "relabel_reset", "mix64", "cache_lookup", "evict_both", "launch_count", "ScoreSink", "KernelTimer",
     "set_kernel_timer", "prepare_aggr", "run_aggr_fwd", "run_aggr_bwd", "transpose_block", "run_aggr_bwd_gather",
     "PeerRegion", "peer_open", "peer_close", "peer_ptrs", "peer_lookup", "peer_publish", "peer_pull", "peer_admit", "make_shard",
 ]
@@ -279,9 +279,6 @@ def aggr_forward_history_edge_value(input, ptr, idx, edge_value, history_map, hi
 
 
 # ---------------------------------------------------------------------------
-# scores, threshold, admission, eviction
-# ---------------------------------------------------------------------------
-# ---------------------------------------------------------------------------
 # batch norm + ReLU + dropout in one forward pair / one backward pair
 # ---------------------------------------------------------------------------
 def norm_act(x, weight, bias, state, *, valid=None, running_mean=None, running_var=None, momentum=0.1,
@@ -297,84 +294,18 @@ def norm_act_supported(x) -> bool:
     return x.is_cuda and x.dtype == torch.float32 and x.dim() == 2 and x.shape[1] % 4 == 0 and x.shape[1] <= 1024
 
 
-def score_rows(x, kind=HC_SCORE_L2, out=None):
-    """Per-row L2 / L1 norm in the library's fixed reduction order."""
-    dev = require_cuda(x)
-    x = rows2d(x)
-    if x.dtype != torch.float32:
-        x = x.float()
-    n, F = x.shape
-    if out is None:
-        out = torch.empty(n, dtype=torch.float32, device=dev)
-    with on_device(dev), _span("hc_score_rows", dev):
-        check(lib.hc_score_rows(ptr(x), n, F, x.stride(0) if n > 1 else F, kind, ptr(out),
-                                stream_of(dev)), "hc_score_rows")
-    _called()
-    return out
-
-
-def select_threshold(score, q, out=None, n_valid=None):
-    """torch.quantile(score, q) (linear interpolation) without leaving the device.  With
-    n_valid (device int64[1]) the quantile is over the n_valid smallest scores (padding rows
-    carry +inf)."""
-    dev = require_cuda(score)
-    score = score.contiguous()
-    if score.dtype != torch.float32:
-        raise TypeError("select_threshold: scores must be float32")
-    if out is None:
-        out = torch.empty(1, dtype=torch.float32, device=dev)
-    n = score.shape[0]
-    nbytes = int(lib.hc_select_scratch_bytes(n))
-    sc = scratch(dev, nbytes, "select") if nbytes else None
-    with on_device(dev), _span("hc_select_threshold", dev):
-        if n_valid is None:
-            check(lib.hc_select_threshold(ptr(score), n, float(q), ptr(out), ptr(sc),
-                                          stream_of(dev)), "hc_select_threshold")
-        else:
-            check(lib.hc_select_threshold_counted(ptr(score), n, ptr(n_valid), float(q),
-                                                  ptr(out), ptr(sc), stream_of(dev)), "hc_select_threshold_counted")
-    _called(9 if nbytes else 1)
-    return out
-
-
-def record_history(buffer_new, buffer_all, used_mask, sub_to_full, sub_to_history,
-                   history_to_full, full_to_history, header, score, thres, checkin_iter, glb_iter,
-                   n_admitted=None):
-    """src/cpp/src/grad_check.cu:48-68, same argument order; mutates buffer_all, both maps,
-    header and checkin_iter in place.  `thres` is a 1-element tensor."""
-    dev = require_cuda(buffer_new, buffer_all, sub_to_full, sub_to_history, history_to_full,
-                       full_to_history, header, score, thres, checkin_iter)
-    buffer_new = rows2d(buffer_new)
-    if buffer_new.dtype != torch.float32:
-        buffer_new = buffer_new.float()
-    n, hs = buffer_new.shape
-    if not buffer_all.is_contiguous():
-        raise RuntimeError("record_history: buffer_all must be contiguous")
-    if buffer_all.shape[1] != hs:
-        raise RuntimeError("record_history: row widths differ")
-    for name, t in (("history_to_full", history_to_full), ("full_to_history", full_to_history),
-                    ("header", header), ("checkin_iter", checkin_iter)):
-        if t.dtype != torch.int64 or not t.is_contiguous():
-            raise TypeError(f"record_history: {name} must be contiguous int64")
-    if used_mask is not None:
-        if used_mask.dtype not in (torch.bool, torch.uint8):
-            raise TypeError("record_history: used_mask must be bool")
-        used_mask = used_mask.contiguous()
-        if used_mask.shape[0] < n:
-            raise RuntimeError("record_history: used_mask shorter than buffer_new")
-    if sub_to_full.shape[0] < n or sub_to_history.shape[0] < n or score.shape[0] < n:
-        raise RuntimeError("record_history: per-row arguments shorter than buffer_new")
-    thres = thres.reshape(-1).float()
-    sc = scratch(dev, lib.hc_admit_scratch_bytes(n), "admit")
-    with on_device(dev), _span("hc_record_history", dev):
-        check(lib.hc_record_history(
-            ptr(buffer_new), buffer_new.stride(0) if n > 1 else hs, n, ptr(buffer_all),
-            dtype_code(buffer_all), buffer_all.shape[0], hs, ptr(used_mask),
-            ptr(i64c(sub_to_full)), ptr(i64c(sub_to_history)), ptr(history_to_full),
-            ptr(full_to_history), ptr(header), ptr(score.contiguous().float()), ptr(thres),
-            ptr(checkin_iter), int(glb_iter), ptr(n_admitted), ptr(sc), stream_of(dev)),
-            "hc_record_history")
-    _called(4)
+# ---------------------------------------------------------------------------
+# scores, threshold, admission, eviction (csrc/torch_ops.cpp)
+# ---------------------------------------------------------------------------
+score_rows = _native.score_rows
+select_threshold = _native.select_threshold
+record_history = _native.record_history
+cache_admit = _native.cache_admit
+evict_stale = _native.evict_stale
+evict_stale_dev = _native.evict_stale_dev
+evict_by_score = _native.evict_by_score
+evict_both = _native.evict_both
+stamp_checkin = _native.stamp_checkin
 
 
 def record_history_noalloc(buffer_new, buffer_all, used_mask, sub_to_full, sub_to_history,
@@ -421,89 +352,14 @@ def record_history_noalloc(buffer_new, buffer_all, used_mask, sub_to_full, sub_t
     _called(4)
 
 
-def cache_admit(produced, buffer, hidden, in_feat, embed_capacity, sub_to_full, sub2embed, score,
-                thres, full2embed, total_num_node, embed2full, feat2full, header,
-                reset_header=False, n_admitted=None, valid=None):
-    """Device-side HistoryCache.update_history (hiscache/history_cache.py:211-254)."""
-    dev = require_cuda(produced, buffer, sub_to_full, sub2embed, score, thres, full2embed,
-                       embed2full, header)
-    produced = rows2d(produced)
-    if produced.dtype != torch.float32:
-        produced = produced.float()
-    n = produced.shape[0]
-    sc = scratch(dev, lib.hc_admit_scratch_bytes(n), "admit")
-    f2f_len = 0 if feat2full is None else feat2full.shape[0]
-    with on_device(dev), _span("hc_cache_admit", dev):
-        check(lib.hc_cache_admit(
-            ptr(produced), produced.stride(0) if n > 1 else hidden, n, ptr(buffer),
-            dtype_code(buffer), hidden, in_feat, embed_capacity, ptr(i64c(sub_to_full)),
-            ptr(i64c(sub2embed)), ptr(score), ptr(thres), ptr(full2embed), total_num_node,
-            ptr(embed2full), ptr(feat2full), f2f_len, ptr(header), 1 if reset_header else 0,
-            ptr(valid), ptr(n_admitted), ptr(sc), stream_of(dev)), "hc_cache_admit")
-    _called(4)
-
-
-def evict_stale(checkin_iter, history_to_full, full_to_history, glb_iter, limit):
-    """hiscache/history_table.py:189-200."""
-    dev = require_cuda(checkin_iter, history_to_full, full_to_history)
-    with on_device(dev), _span("hc_evict_stale", dev):
-        check(lib.hc_evict_stale(ptr(checkin_iter), ptr(history_to_full), ptr(full_to_history),
-                                 checkin_iter.shape[0], int(glb_iter), int(limit),
-                                 stream_of(dev)), "hc_evict_stale")
-    _called()
-
-
 CHECKIN_MARKER = 1 << 60   # a glb_iter no iteration takes
-
-
-def evict_stale_dev(checkin_iter, history_to_full, full_to_history, iter_dev, limit):
-    """evict_stale with the iteration number read from a device int64[1]."""
-    dev = require_cuda(checkin_iter, history_to_full, full_to_history, iter_dev)
-    with on_device(dev), _span("hc_evict_stale", dev):
-        check(lib.hc_evict_stale_dev(ptr(checkin_iter), ptr(history_to_full), ptr(full_to_history),
-                                     checkin_iter.shape[0], ptr(iter_dev), int(limit), stream_of(dev)),
-              "hc_evict_stale_dev")
-    _called()
-
-
-def stamp_checkin(checkin_iter, iter_dev, marker=CHECKIN_MARKER):
-    """checkin_iter[checkin_iter == marker] = iter_dev[0]."""
-    dev = require_cuda(checkin_iter, iter_dev)
-    with on_device(dev), _span("hc_stamp_checkin", dev):
-        check(lib.hc_stamp_checkin(ptr(checkin_iter), checkin_iter.shape[0], int(marker), ptr(iter_dev),
-                                   stream_of(dev)), "hc_stamp_checkin")
-    _called()
-
-
-def evict_by_score(sub_to_history, score, thres, checkin_iter, history_to_full, full_to_history):
-    """hiscache/history_table.py:234-241."""
-    dev = require_cuda(sub_to_history, score, thres, checkin_iter)
-    n = min(sub_to_history.shape[0], score.shape[0])
-    with on_device(dev), _span("hc_evict_by_score", dev):
-        check(lib.hc_evict_by_score(ptr(i64c(sub_to_history)), ptr(score.contiguous()),
-                                    ptr(thres.reshape(-1)), n, ptr(checkin_iter),
-                                    ptr(history_to_full), ptr(full_to_history), stream_of(dev)),
-              "hc_evict_by_score")
-    _called()
 
 
 # ---------------------------------------------------------------------------
 # receptive-field bookkeeping
 # ---------------------------------------------------------------------------
-def count_history_reconstruct(ptr_t, idx_t, history_maps, num_node, num_seed, num_layer):
-    """src/cpp/src/grad_check.cu:103-130: list of num_layer+1 bool masks [num_node];
-    [num_layer] is the seed level, [0] gates raw-feature loading."""
-    dev = require_cuda(ptr_t, idx_t)
-    ptr_t, idx_t = i64c(ptr_t, "ptr"), i64c(idx_t, "idx")
-    hm = None if _empty(history_maps) else i64c(history_maps, "history_maps")
-    buf = torch.empty((num_layer + 1, num_node), dtype=torch.uint8, device=dev)
-    with on_device(dev), _span("hc_used_masks", dev):
-        check(lib.hc_used_masks(ptr(ptr_t), ptr(idx_t), ptr_t.shape[0] - 1, ptr(hm),
-                                0 if hm is None else hm.shape[0], num_node, num_seed, num_layer,
-                                ptr(buf), stream_of(dev)), "hc_used_masks")
-    _called(num_layer)
-    b = buf.view(torch.bool)
-    return [b[k] for k in range(num_layer + 1)]
+count_history_reconstruct = _native.count_history_reconstruct
+count_num = _native.count_num
 
 
 def get_graph_structure_score(ptr_t, idx_t, num_node, num_seed, num_layer):
@@ -520,111 +376,13 @@ def get_graph_structure_score(ptr_t, idx_t, num_node, num_seed, num_layer):
     return out
 
 
-def count_num(arr, mmax):
-    """src/cpp/src/grad_check.cu:174-182: int32 histogram [mmax+1]; value 0 is not counted."""
-    dev = require_cuda(arr)
-    arr = i64c(arr, "arr")
-    out = torch.empty(int(mmax) + 1, dtype=torch.int32, device=dev)
-    with on_device(dev), _span("hc_count_num", dev):
-        check(lib.hc_count_num(ptr(arr), arr.shape[0], int(mmax), ptr(out), stream_of(dev)),
-              "hc_count_num")
-    _called()
-    return out
-
-
 # ---------------------------------------------------------------------------
 # lookup and row assembly
 # ---------------------------------------------------------------------------
-def map_lookup(map_t, ids, offset=0, force_miss_below=0, out=None):
-    """out[i] = map[ids[i] + offset]; first `force_miss_below` entries forced to -1."""
-    dev = require_cuda(map_t, ids)
-    ids = i64c(ids, "ids")
-    n = ids.shape[0]
-    if out is None:
-        out = torch.empty(n, dtype=torch.int64, device=dev)
-    with on_device(dev), _span("hc_map_lookup", dev):
-        check(lib.hc_map_lookup(ptr(map_t), map_t.shape[0], ptr(ids), n, int(offset),
-                                int(force_miss_below), ptr(out), stream_of(dev)), "hc_map_lookup")
-    _called()
-    return out
-
-
-def gather_rows(table, rows, zero_missing=False, out_dtype=None):
-    """table[rows] with torch's negative indexing (or zeros for -1 when zero_missing)."""
-    dev = require_cuda(table, rows)
-    table = rows2d(table)
-    rows = i64c(rows, "rows")
-    n, F = rows.shape[0], table.shape[1]
-    out = torch.empty((n, F), dtype=out_dtype or table.dtype, device=dev)
-    with on_device(dev), _span("hc_gather_rows", dev):
-        check(lib.hc_gather_rows(ptr(table), dtype_code(table), table.shape[0],
-                                 table.stride(0) if table.shape[0] > 1 else F, F, ptr(rows), n,
-                                 1 if zero_missing else 0, ptr(out), dtype_code(out), F,
-                                 stream_of(dev)), "hc_gather_rows")
-    _called()
-    return out
-
-
-def load_rows(host_table, feat_cache, sub_to_full, sub2feat, used, out_dtype=None,
-              want_mask=False, stats=None, out=None, mask_out=None, staged=None):
-    """One-pass batch.x assembly (hiscache/history_cache.py:327-350).  host_table may be a
-    pinned host tensor (rows are then read over the host link by the kernel) or a CUDA
-    tensor.  Returns x, or (x, load_mask) when want_mask.
-
-    out / mask_out: preallocated destinations ([n, F] rows, [n] uint8 mask).
-    staged = (rows [n, F], mask [n] uint8): host rows fetched ahead of the step by
-    `stage_host_rows`; a row whose mask is set is read from there instead of host_table.  `stats` then needs three counters (host, cache, staged)."""
-    dev = require_cuda(sub_to_full, sub2feat, used, feat_cache, out, mask_out,
-                       host_table if host_table.is_cuda else None)
-    if not host_table.is_cuda and not host_table.is_pinned():
-        raise RuntimeError("load_rows: a host feature table must be pinned memory")
-    host_table = rows2d(host_table)
-    sub_to_full = i64c(sub_to_full, "sub_to_full")
-    sub2feat = i64c(sub2feat, "sub2feat")
-    n, F = sub_to_full.shape[0], host_table.shape[1]
-    dt = out_dtype or host_table.dtype
-    if out is None:
-        x = torch.empty((n, F), dtype=dt, device=dev)
-    else:
-        if tuple(out.shape) != (n, F) or out.dtype != dt or not out.is_contiguous():
-            raise ValueError(f"load_rows: out must be a contiguous [{n}, {F}] {dt} tensor")
-        x = out
-    if mask_out is not None:
-        if mask_out.dtype != torch.uint8 or mask_out.shape[0] != n or not mask_out.is_contiguous():
-            raise ValueError(f"load_rows: mask_out must be a contiguous uint8 tensor of {n} entries")
-        mask = mask_out
-    else:
-        mask = torch.empty(n, dtype=torch.uint8, device=dev) if want_mask else None
-    if used is not None:
-        used = used.contiguous()
-        if used.shape[0] != n or used.element_size() != 1:
-            raise ValueError(f"load_rows: used must have {n} one-byte entries")
-    cd, cr, cs = HC_F32, 0, 0
-    if feat_cache is not None:
-        feat_cache = rows2d(feat_cache)
-        cd, cr = dtype_code(feat_cache), feat_cache.shape[0]
-        cs = feat_cache.stride(0) if cr > 1 else F
-    common = (ptr(host_table), dtype_code(host_table), host_table.shape[0],
-              host_table.stride(0) if host_table.shape[0] > 1 else F,
-              ptr(feat_cache), cd, cr, cs, F, ptr(sub_to_full), ptr(sub2feat),
-              ptr(used), n, ptr(x), dtype_code(x), F, ptr(mask), ptr(stats))
-    if staged is None:
-        with on_device(dev), _span("hc_load_rows", dev):
-            check(lib.hc_load_rows(*common, stream_of(dev)), "hc_load_rows")
-    else:
-        s_rows, s_mask = staged
-        require_cuda(s_rows, s_mask)
-        if (tuple(s_rows.shape) != (n, F) or s_rows.dtype != x.dtype or not s_rows.is_contiguous()
-                or s_mask.dtype != torch.uint8 or s_mask.shape[0] != n or not s_mask.is_contiguous()):
-            raise ValueError(f"load_rows: staged must be ([{n}, {F}] {x.dtype} rows, [{n}] uint8 mask)")
-        if stats is not None and stats.numel() < 3:
-            raise ValueError("load_rows: stats needs three counters when rows are staged")
-        with on_device(dev), _span("hc_load_rows", dev):
-            check(lib.hc_load_rows_staged(*common, ptr(s_rows), ptr(s_mask), stream_of(dev)),
-                  "hc_load_rows_staged")
-    _called()
-    return (x, mask.view(torch.bool)) if want_mask else x
-
+map_lookup = _native.map_lookup
+cache_lookup = _native.cache_lookup
+gather_rows = _native.gather_rows
+load_rows = _native.load_rows
 
 # thread blocks of a staging call; non-zero overrides every caller's choice (a knob for measurements)
 STAGE_BLOCKS = int(os.environ.get("HISCACHE_STAGE_BLOCKS", "0"))
@@ -634,30 +392,8 @@ def stage_host_rows(host_table, ids, sub2feat, consider, rows_out, mask_out, sta
     """Copies host_table[ids[i]] into rows_out[i] and sets mask_out[i] for every i that is to be
     considered and is not in the feature cache (sub2feat[i] == -1); other rows of rows_out are
     unspecified.  The result feeds `load_rows(..., staged=(rows_out, mask_out))` of a later step."""
-    dev = require_cuda(ids, sub2feat, consider, rows_out, mask_out, host_table if host_table.is_cuda else None)
-    if not host_table.is_cuda and not host_table.is_pinned():
-        raise RuntimeError("stage_host_rows: a host feature table must be pinned memory")
-    host_table = rows2d(host_table)
-    ids = i64c(ids, "ids")
-    n, F = ids.shape[0], host_table.shape[1]
-    if sub2feat is not None:
-        sub2feat = i64c(sub2feat, "sub2feat")
-        if sub2feat.shape[0] != n:
-            raise ValueError(f"stage_host_rows: sub2feat must have {n} entries")
-    if consider is not None:
-        consider = consider.contiguous()
-        if consider.shape[0] != n or consider.element_size() != 1:
-            raise ValueError(f"stage_host_rows: consider must have {n} one-byte entries")
-    if (tuple(rows_out.shape) != (n, F) or rows_out.dtype != host_table.dtype or not rows_out.is_contiguous()
-            or mask_out.dtype != torch.uint8 or mask_out.shape[0] != n or not mask_out.is_contiguous()):
-        raise ValueError(f"stage_host_rows: outputs must be [{n}, {F}] {host_table.dtype} rows and [{n}] uint8 mask")
-    with on_device(dev), _span("hc_stage_host_rows", dev):
-        check(lib.hc_stage_host_rows(ptr(host_table), dtype_code(host_table), host_table.shape[0],
-                                     host_table.stride(0) if host_table.shape[0] > 1 else F, F, ptr(ids),
-                                     ptr(sub2feat), ptr(consider), n, ptr(rows_out), ptr(mask_out), ptr(stats),
-                                     int(STAGE_BLOCKS or (max_blocks or 0)),
-                                     stream_of(dev)), "hc_stage_host_rows")
-    _called()
+    _native.stage_host_rows(host_table, ids, sub2feat, consider, rows_out, mask_out, stats,
+                            int(STAGE_BLOCKS or (max_blocks or 0)))
 
 
 # ---------------------------------------------------------------------------
@@ -932,153 +668,44 @@ def peer_admit(shard, pub_ids, pub_rows, pub_n, world, me, max_ids, got_ids, got
 # ---------------------------------------------------------------------------
 ABSENT = -(1 << 31)  # local_map value of a node outside the batch
 
-
-def sample_hop(gptr, gidx, frontier, fanout, seed, base):
-    """One hop of uniform sampling with replacement: (out_ptr [nf+1], nbr [total]) with
-    min(fanout, degree) draws per frontier node.  Reads one size back from the device."""
-    dev = require_cuda(gptr, gidx, frontier)
-    frontier = i64c(frontier, "frontier")
-    nf = frontier.shape[0]
-    out_ptr = torch.zeros(nf + 1, dtype=torch.int64, device=dev)
-    with on_device(dev), _span("hc_sample_counts", dev):
-        check(lib.hc_sample_counts(ptr(gptr), ptr(frontier), nf, int(fanout), ptr(out_ptr[1:]),
-                                   stream_of(dev)), "hc_sample_counts")
-    torch.cumsum(out_ptr[1:], 0, out=out_ptr[1:])
-    total = int(out_ptr[-1]) if nf > 0 else 0
-    nbr = torch.empty(total, dtype=torch.int64, device=dev)
-    with on_device(dev), _span("hc_sample_picks", dev):
-        check(lib.hc_sample_picks(ptr(gptr), ptr(gidx), ptr(frontier), nf, int(fanout), ptr(out_ptr),
-                                  C.c_uint64(seed & 0xFFFFFFFFFFFFFFFF), int(base), ptr(nbr),
-                                  stream_of(dev)), "hc_sample_picks")
-    _called(2)
-    return out_ptr, nbr
+sample_hop = _native.sample_hop
+relabel_seed = _native.relabel_seed
+relabel_reset = _native.relabel_reset
+relabel = _native.relabel
 
 
-def relabel_seed(seeds, local_map):
-    dev = require_cuda(seeds, local_map)
-    with torch.cuda.device(dev):
-        check(lib.hc_relabel_seed(ptr(i64c(seeds)), seeds.shape[0], ptr(local_map), stream_of(dev)),
-              "hc_relabel_seed")
-    _called()
-
-
-def relabel_reset(nodes, local_map):
-    dev = require_cuda(nodes, local_map)
-    with torch.cuda.device(dev):
-        check(lib.hc_relabel_reset(ptr(i64c(nodes)), nodes.shape[0], ptr(local_map), stream_of(dev)),
-              "hc_relabel_reset")
-    _called()
-
-
-def relabel(nbr, local_map, n_total):
-    """(new_nodes [n_new], local ids of nbr): new nodes numbered from n_total in order of first
-    occurrence.  Reads n_new back from the device."""
-    dev = require_cuda(nbr, local_map)
-    m = nbr.shape[0]
-    new_nodes = torch.empty(max(m, 1), dtype=torch.int64, device=dev)
-    n_new = torch.zeros(1, dtype=torch.int64, device=dev)
-    out_idx = torch.empty(m, dtype=torch.int64, device=dev)
-    sc = scratch(dev, lib.hc_relabel_scratch_bytes(m), "relabel")
-    with on_device(dev), _span("hc_relabel", dev):
-        check(lib.hc_relabel(ptr(nbr), m, ptr(local_map), int(n_total), ptr(new_nodes), ptr(n_new),
-                             ptr(out_idx), ptr(sc), stream_of(dev)), "hc_relabel")
-    _called(6)
-    return new_nodes[:int(n_new)], out_idx
-
-
-def sample_fixed(gptr, gidx, seeds, local_map, seed, batch_no, fanouts, caps, edge_cap, out=None):
+def sample_fixed(gptr, gidx, seeds, local_map, seed, batch_no, fanouts, caps, edge_cap, out=None, labels=None):
     """A whole batch in the fixed shape (caps, edge_cap) without any device->host read
     (hc_sample_fixed).  `batch_no`: device int64[1], advanced by the call.  Returns the dict of
-    output tensors (ptr, idx, sub_to_full, mask, counters); `out` reuses a previous one."""
-    dev = require_cuda(gptr, gidx, seeds, local_map, batch_no)
+    output tensors (ptr, idx, sub_to_full, mask, counters); `out` reuses a previous one.  With `labels`
+    (int64 per node) out["y"] is filled too: the seeds' labels, -100 in padding rows."""
     L = len(fanouts)
     if len(caps) != L + 1 or L < 1 or L > 8:
         raise ValueError("sample_fixed: one cap per layer (hops + 1), 1..8 hops")
     if local_map.dtype != torch.int32 or batch_no.dtype != torch.int64:
         raise TypeError("sample_fixed: local_map int32, batch_no int64")
-    seeds = i64c(seeds, "seeds")
     if seeds.shape[0] > caps[0]:
         raise RuntimeError("sample_fixed: more seeds than caps[0]")
     if out is None:
+        dev = require_cuda(gptr)
         out = {"ptr": torch.empty(caps[L - 1] + 1, dtype=torch.int64, device=dev),
                "idx": torch.empty(max(int(edge_cap), 1), dtype=torch.int64, device=dev),
                "sub_to_full": torch.empty(caps[L], dtype=torch.int64, device=dev),
                "mask": torch.empty(caps[L], dtype=torch.bool, device=dev),
                "counters": torch.zeros(4, dtype=torch.int64, device=dev)}
-    b = _capi.FixedBatch()
-    b.struct_size = C.sizeof(_capi.FixedBatch)
-    b.num_hops = L
-    for h in range(L):
-        b.fanout[h] = int(fanouts[h])
-    for k in range(L + 1):
-        b.caps[k] = int(caps[k])
-    b.edge_cap = int(edge_cap)
-    b.ptr, b.idx, b.sub_to_full = ptr(out["ptr"]), ptr(out["idx"]), ptr(out["sub_to_full"])
-    b.mask, b.counters = ptr(out["mask"]), ptr(out["counters"])
-    sc = scratch(dev, int(lib.hc_sample_fixed_scratch_bytes(C.byref(b))), "sample_fixed")
-    with on_device(dev), _span("hc_sample_fixed", dev):
-        check(lib.hc_sample_fixed(ptr(gptr), ptr(gidx), ptr(seeds), seeds.shape[0], ptr(local_map),
-                                  C.c_uint64(int(seed) & 0xFFFFFFFFFFFFFFFF), ptr(batch_no), C.byref(b),
-                                  ptr(sc), stream_of(dev)), "hc_sample_fixed")
-    _called(2 + 11 * L)
+    if labels is not None and "y" not in out:
+        out["y"] = torch.empty(caps[0], dtype=torch.int64, device=gptr.device)
+    _native.sample_batch(gptr, gidx, seeds, local_map, int(seed) & 0xFFFFFFFFFFFFFFFF, batch_no, fanouts, caps,
+                         int(edge_cap), out["ptr"], out["idx"], out["sub_to_full"], out["mask"], out["counters"],
+                         labels, None if labels is None else out["y"])
     return out
 
 
 # ---------------------------------------------------------------------------
 # heterogeneous layers
 # ---------------------------------------------------------------------------
-def edge_types(ptr_t, idx_t, sub_to_full, rows, type_bounds, rel_table):
-    """etype[e] = rel_table[type(dst)][type(src)], node types being ranges of global ids:
-    the counterpart of cxgnncomp_backend.gen_edge_type_mag240m (hiscache/history_model.py:354-357)."""
-    dev = require_cuda(ptr_t, idx_t, sub_to_full)
-    T = len(type_bounds) - 1
-    if T < 1 or T > 8 or len(rel_table) != T * T:
-        raise ValueError("edge_types: 1..8 node types, rel_table of n_types^2 entries")
-    out = torch.empty(idx_t.shape[0], dtype=torch.int64, device=dev)
-    rows = int(rows)
-    if idx_t.shape[0] and rows < ptr_t.shape[0] - 1:
-        out.fill_(0)     # edges behind the rows asked for
-    b = (C.c_int64 * (T + 1))(*[int(v) for v in type_bounds])
-    r = (C.c_int32 * (T * T))(*[int(v) for v in rel_table])
-    with on_device(dev), _span("hc_edge_types", dev):
-        check(lib.hc_edge_types(ptr(i64c(ptr_t)), ptr(i64c(idx_t)), ptr(i64c(sub_to_full)), rows, T, b, r,
-                                ptr(out), stream_of(dev)), "hc_edge_types")
-    _called()
-    return out
-
-
-def rgcn_group(ptr_t, idx_t, etype, num_node, num_rel, used_src=None, hmap=None, want_perm=False,
-               want_rel=False):
-    """The relation-segmented block of one RGCN layer (hc_rgcn_group): (ptr2 [num_rel*num_node+1],
-    idx2 [E], w2 [E], perm or None, rel or None)."""
-    dev = require_cuda(ptr_t, idx_t, etype, used_src, hmap)
-    ptr_t, idx_t, etype, hmap = i64c(ptr_t, "ptr"), i64c(idx_t, "idx"), i64c(etype, "edge_type"), i64c(hmap)
-    n_edges = min(int(idx_t.shape[0]), int(etype.shape[0]))
-    num_node, num_rel = int(num_node), int(num_rel)
-    if ptr_t.shape[0] < num_node + 1:
-        raise RuntimeError("rgcn_group: ptr shorter than num_node + 1")
-    if hmap is not None and hmap.shape[0] < num_node:
-        raise RuntimeError("rgcn_group: history map shorter than num_node")
-    if used_src is not None:
-        used_src = used_src.contiguous()
-        if used_src.dtype == torch.bool:
-            used_src = used_src.view(torch.uint8)
-        elif used_src.dtype != torch.uint8:
-            raise TypeError("rgcn_group: used mask must be bool")
-    ptr2 = torch.empty(num_rel * num_node + 1, dtype=torch.int64, device=dev)
-    idx2 = torch.empty(max(n_edges, 1), dtype=torch.int64, device=dev)
-    w2 = torch.empty(max(n_edges, 1), dtype=torch.float32, device=dev)
-    perm = torch.empty(max(n_edges, 1), dtype=torch.int64, device=dev) if want_perm else None
-    rel = torch.empty(max(n_edges, 1), dtype=torch.int64, device=dev) if want_rel else None
-    sc = scratch(dev, lib.hc_rgcn_group_scratch_bytes(n_edges), "rgcn")
-    with on_device(dev), _span("hc_rgcn_group", dev):
-        check(lib.hc_rgcn_group(ptr(ptr_t), ptr(idx_t), ptr(etype), num_node, n_edges, num_rel, ptr(used_src),
-                                ptr(hmap), ptr(ptr2), ptr(idx2), ptr(w2), ptr(perm), ptr(rel), ptr(sc),
-                                stream_of(dev)), "hc_rgcn_group")
-    _called(7)
-    return ptr2, idx2[:n_edges], w2[:n_edges], None if perm is None else perm[:n_edges], \
-        None if rel is None else rel[:n_edges]
-
+edge_types = _native.edge_types
+rgcn_group = _native.rgcn_group
 
 # ---------------------------------------------------------------------------
 # peer copies (kept for API compatibility; the multi-GPU path uses NCCL)

@@ -117,6 +117,15 @@ _SIGS = {
     "hc_rgcn_group": (C.c_int, [vp, vp, vp, i64, i64, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
     "hc_sample_fixed_scratch_bytes": (i64, [C.POINTER(FixedBatch)]),
     "hc_sample_fixed": (C.c_int, [vp, vp, vp, i64, vp, C.c_uint64, vp, C.POINTER(FixedBatch), vp, vp]),
+    "hc_sample_batch": (C.c_int, [vp, vp, vp, i64, vp, C.c_uint64, vp, vp, vp, C.POINTER(FixedBatch), vp, vp]),
+    "hc_evict_both": (C.c_int, [vp, vp, vp, i64, vp, vp, vp, i64, i64, vp, i64, vp]),
+    "hc_used_masks_scratch_bytes": (i64, []),
+    "hc_used_masks_together": (C.c_int, [vp, vp, i64, vp, i64, i64, i64, i32, vp, vp, vp]),
+    "hc_map_lookup_masked": (C.c_int, [vp, i64, vp, i64, i64, vp, vp, vp]),
+    "hc_cache_lookup": (C.c_int, [vp, i64, vp, i64, i64, i64, vp, vp, vp]),
+    "hc_select_threshold_masked": (C.c_int, [vp, vp, i64, f32, vp, vp, vp]),
+    "hc_record_history_masked": (C.c_int, [vp, i64, i64, vp, i32, i64, i32, vp, vp, vp, vp, vp, vp, vp,
+                                           vp, vp, vp, i64, vp, vp, vp]),
     "hc_mix64": (C.c_uint64, [C.c_uint64]),
     "hc_bucket_scratch_bytes": (i64, [i64, i32]),
     "hc_bucket_by_owner": (C.c_int, [vp, vp, i64, i32, vp, vp, vp, vp, vp]),

@@ -249,6 +249,9 @@ int hc_select_threshold(const float* score, int64_t n, float q, float* thres,
  */
 int hc_select_threshold_counted(const float* score, int64_t n, const int64_t* n_valid, float q,
                                 float* thres, void* scratch, void* stream);
+/* The same quantile over the rows whose byte of `valid` ([n]) is not 0. */
+int hc_select_threshold_masked(const float* score, const uint8_t* valid, int64_t n, float q,
+                               float* thres, void* scratch, void* stream);
 
 /* ------------------------------------------------------------------------ */
 /* Admission and eviction                                                   */
@@ -279,6 +282,16 @@ int hc_record_history(const float* buffer_new, int64_t new_stride, int64_t n,
                       int64_t* header, const float* score, const float* thres,
                       int64_t* checkin_iter, int64_t glb_iter,
                       int64_t* n_admitted, void* scratch, void* stream);
+/* hc_record_history that admits only rows whose byte of `valid` ([n], may be
+ * NULL) is not 0 besides used_mask. */
+int hc_record_history_masked(const float* buffer_new, int64_t new_stride, int64_t n,
+                             void* buffer_all, int32_t table_dtype, int64_t capacity,
+                             int32_t history_size, const uint8_t* used_mask,
+                             const uint8_t* valid, const int64_t* sub_to_full,
+                             const int64_t* sub_to_history, int64_t* history_to_full,
+                             int64_t* full_to_history, int64_t* header, const float* score,
+                             const float* thres, int64_t* checkin_iter, int64_t glb_iter,
+                             int64_t* n_admitted, void* scratch, void* stream);
 
 /*
  * hc_record_history for callers that cannot allocate device memory.  (No
@@ -288,7 +301,7 @@ int hc_record_history(const float* buffer_new, int64_t new_stride, int64_t n,
  * framework's device allocator for the scratch argument, and loops whose
  * device memory is wholly owned by a caching allocator, where a raw
  * cudaMalloc / cudaFree would fail or stall the device.  Same arguments and
- * result as hc_record_history minus `scratch`: the scratch is a 16 KB array
+ * result as hc_record_history minus `scratch`: the scratch is a small array
  * inside the library image (each GPU that loads the library holds it until
  * exit).  Limits and rules:
  *   - n <= HC_NOALLOC_MAX_ROWS (hc_noalloc_max_rows()); more returns
@@ -372,6 +385,17 @@ int hc_evict_by_score(const int64_t* sub_to_history, const float* score,
                       int64_t* history_to_full, int64_t* full_to_history,
                       void* stream);
 
+/*
+ * Both evictions of HistoryTable.evict_by_both (history_table.py:234-251) in
+ * one launch: hc_evict_by_score over n rows and hc_evict_stale over capacity
+ * slots, the iteration taken from glb_iter_dev (device int64) when that is
+ * not NULL.
+ */
+int hc_evict_both(const int64_t* sub_to_history, const float* score, const float* thres,
+                  int64_t n, int64_t* checkin_iter, int64_t* history_to_full,
+                  int64_t* full_to_history, int64_t capacity, int64_t glb_iter,
+                  const int64_t* glb_iter_dev, int64_t limit, void* stream);
+
 /* ------------------------------------------------------------------------ */
 /* Receptive-field bookkeeping                                              */
 /* ------------------------------------------------------------------------ */
@@ -389,6 +413,16 @@ int hc_used_masks(const int64_t* ptr, const int64_t* idx, int64_t ptr_rows,
                   const int64_t* history_map, int64_t history_map_len,
                   int64_t num_node, int64_t num_seed, int32_t num_layer,
                   uint8_t* masks, void* stream);
+/*
+ * The same as one cooperative launch (batches of up to 256 K rows; larger
+ * ones fall back to one launch per step).  scratch: device, 8-byte aligned,
+ * >= hc_used_masks_scratch_bytes().
+ */
+int64_t hc_used_masks_scratch_bytes(void);
+int hc_used_masks_together(const int64_t* ptr, const int64_t* idx, int64_t ptr_rows,
+                           const int64_t* history_map, int64_t history_map_len,
+                           int64_t num_node, int64_t num_seed, int32_t num_layer,
+                           uint8_t* masks, void* scratch, void* stream);
 
 /*
  * Level-synchronous form of get_graph_structure_score (grad_check.cu:132-163):
@@ -423,6 +457,16 @@ int hc_count_num(const int64_t* arr, int64_t n, int64_t mmax, int32_t* output,
 int hc_map_lookup(const int64_t* map, int64_t map_len, const int64_t* ids,
                   int64_t n, int64_t offset, int64_t force_miss_below,
                   int64_t* out, void* stream);
+/* hc_map_lookup with offset 0 in which rows whose byte of `valid` ([n]) is 0
+ * also give -1 (padding rows of fixed-shape batches). */
+int hc_map_lookup_masked(const int64_t* map, int64_t map_len, const int64_t* ids,
+                         int64_t n, int64_t force_miss_below, const uint8_t* valid,
+                         int64_t* out, void* stream);
+/* Both lookups of lookup_and_load in one launch: sub2embed[i] = map[ids[i]]
+ * for i < n1, sub2feat[i] = map[ids[i] + offset] for i < n. */
+int hc_cache_lookup(const int64_t* map, int64_t map_len, const int64_t* ids, int64_t n,
+                    int64_t n1, int64_t offset, int64_t* sub2embed, int64_t* sub2feat,
+                    void* stream);
 
 /*
  * out[i, :] = table[rows[i], :] for i < n; rows[i] == -1 reads the last row
@@ -731,6 +775,10 @@ int64_t hc_sample_fixed_scratch_bytes(const hc_fixed_batch* b);
 int hc_sample_fixed(const int64_t* gptr, const int64_t* gidx, const int64_t* seeds, int64_t n_seeds,
                     int32_t* local_map, uint64_t seed, int64_t* batch_no, const hc_fixed_batch* b,
                     void* scratch, void* stream);
+/* The same, and y [caps[0]]: labels[seed] of the real seed rows, -100 in padding rows. */
+int hc_sample_batch(const int64_t* gptr, const int64_t* gidx, const int64_t* seeds, int64_t n_seeds,
+                    int32_t* local_map, uint64_t seed, int64_t* batch_no, const int64_t* labels,
+                    int64_t* y, const hc_fixed_batch* b, void* scratch, void* stream);
 
 /* ---------------------------------------------------------------------------
  * Dense epilogue of a layer: batch norm (training statistics) + ReLU + dropout.

@@ -178,3 +178,48 @@ def test_evictions_bit_exact(backend, oracle):
     backend.evict_by_score(cu(s2h), cu(score), cu(np.array([0.8], dtype=np.float32)), g[0], g[1], g[2])
     oracle.evict_by_score(s2h, score, 0.8, chk, h2f, f2h)
     assert same(g[0], chk) and same(g[1], h2f) and same(g[2], f2h)
+
+
+@pytest.mark.parametrize("n", [1, 2, 1000, 1025, 16_000, 49_152, 70_000])
+@pytest.mark.parametrize("kind", ["spread", "ties", "one value"])
+def test_masked_threshold_is_the_quantile_of_the_valid_rows(backend, n, kind):
+    rng = np.random.default_rng(n)
+    s = rng.standard_normal(n, dtype=np.float32)
+    if kind == "ties":
+        s = np.round(s * 2) / 2 + np.float32(0)      # thousands of equal keys, no negative zeros
+    elif kind == "one value":
+        s[:] = 0.25
+    valid = rng.random(n) < 0.7
+    valid[0] = True
+    dirty = np.where(valid, s, np.float32(np.nan))      # what padding rows hold does not matter
+    t, m = torch.from_numpy(dirty).cuda(), torch.from_numpy(valid).cuda()
+    for q in (0.0, 0.37, 0.5, 1.0):
+        got = backend.select_threshold(t, q, valid=m)
+        want = torch.quantile(torch.from_numpy(s[valid]), q)
+        assert got.cpu().numpy().tobytes() == want.reshape(1).numpy().tobytes(), (n, kind, q)
+
+
+def test_both_evictions_at_once_equal_one_after_the_other(backend):
+    rng = np.random.default_rng(5)
+    cap, N, n = 3000, 9000, 700
+    h2f = np.full(cap, -1, np.int64)
+    live = rng.permutation(cap)[:2000]
+    h2f[live] = rng.permutation(N)[:2000]
+    f2h = np.full(N, -1, np.int64)
+    f2h[h2f[live]] = live
+    checkin = np.full(cap, -1, np.int64)
+    checkin[live] = rng.integers(0, 20, 2000)
+    s2h = np.where(rng.random(n) < 0.6, live[rng.permutation(2000)[:n]], -1)
+    score, thres = rng.random(n, dtype=np.float32), np.array([0.5], np.float32)
+    runs = []
+    for both in (False, True):
+        c, h, f = (torch.from_numpy(v.copy()).cuda() for v in (checkin, h2f, f2h))
+        args = [torch.from_numpy(v).cuda() for v in (s2h, score, thres)]
+        if both:
+            backend.evict_both(*args, c, h, f, 15, None, 4)
+        else:
+            backend.evict_by_score(*args, c, h, f)
+            backend.evict_stale(c, h, f, 15, 4)
+        runs.append((c.cpu(), h.cpu(), f.cpu()))
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
+    assert 0 < int((runs[0][1] != -1).sum()) < 2000
