@@ -49,6 +49,7 @@ namespace {
   X(hc_stage_host_rows) X(hc_sample_fixed_scratch_bytes) X(hc_sample_batch) X(hc_sample_counts)    \
   X(hc_sample_picks) X(hc_relabel_scratch_bytes) X(hc_relabel) X(hc_relabel_seed)                  \
   X(hc_relabel_reset) X(hc_edge_types) X(hc_rgcn_group_scratch_bytes) X(hc_rgcn_group)             \
+  X(hc_rgcn_rows_scratch_bytes) X(hc_rgcn_rows) X(hc_override_rows)                                \
   X(hc_norm_act_fwd) X(hc_norm_act_bwd)
 
 struct Lib {
@@ -1138,6 +1139,125 @@ py::tuple rgcn_group(const Tensor& ptr_in, const Tensor& idx_in, const Tensor& e
   auto cut = [&](const Tensor& t) -> py::object { return t.defined() ? py::cast(t.slice(0, 0, E)) : py::none(); };
   return py::make_tuple(ptr2, cut(idx2), cut(w2), cut(perm), cut(rel));
 }
+
+// One RGCN layer (MyRGCNConvHistory2): relation-segmented rows by destination, their weighted sums as
+// [num_node, num_rel * feat], one product with the stacked weights, history rows over it.  Destinations
+// served from history have no edges here, so they add nothing to either gradient.
+struct RgcnBackward : public torch::autograd::Node {
+  SavedVariable x, weight;
+  Tensor ptr2, idx2, w2, sums;
+  int64_t num_node = 0, num_rel = 0;
+  BwdRule rule;
+  bool released = false;
+
+  std::string name() const override { return "RgcnBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    x.reset_data();
+    weight.reset_data();
+    ptr2 = idx2 = w2 = sums = Tensor();
+    released = true;
+  }
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+    at::NoGradGuard no_grad;
+    variable_list out(2);
+    if (!grads[0].defined()) return out;
+    const Tensor xt = x.unpack(), w = weight.unpack();
+    const at::Device dev = xt.device();
+    c10::cuda::CUDAGuard guard(dev);
+    const int64_t F = xt.size(1), H = w.size(2);
+    const Tensor g = grads[0].contiguous(), wide = sums.view({num_node, num_rel * F});
+    if (task_should_compute_output(1)) out[1] = at::mm(wide.t(), g).view({num_rel, F, H});
+    if (task_should_compute_output(0)) {
+      const Tensor go = at::mm(g, w.reshape({num_rel * F, H}).t());      // [num_node, num_rel * F] = its rows
+      Block b;
+      b.inp = xt; b.ptr = ptr2; b.idx = idx2; b.ev = w2;
+      b.num_node = num_node * num_rel;
+      const hc_aggr_args a = aggr_args(b);
+      Tensor gx = new_f32(xt.sizes(), dev);
+      int64_t bytes = -1;
+      if (!rule.deterministic && F >= rule.gather_min_feat && a.n_src * F * 4 >= rule.gather_min_bytes)
+        bytes = lib.hc_aggr_bwd_source_scratch_bytes(&a, idx2.numel(), 0);
+      if (bytes >= 0) {
+        Tensor sc = new_scratch(bytes, dev);
+        HC_SPAN_ROWS("hc_aggr_bwd_source", xt, dev);
+        check(lib.hc_aggr_bwd_source(&a, idx2.numel(), fdata(go), fdata(gx), nullptr, data(sc), stream_of(dev)),
+              "hc_aggr_bwd_source");
+        g_launches += 5;
+      } else {
+        HC_SPAN_ROWS("hc_aggr_bwd", xt, dev);
+        check(lib.hc_aggr_bwd(&a, fdata(go), fdata(gx), 1, nullptr, nullptr, nullptr, HC_SCORE_L2, stream_of(dev)),
+              "hc_aggr_bwd");
+        ++g_launches;
+      }
+      out[0] = xt.scalar_type() == at::kFloat ? gx : gx.to(xt.scalar_type());
+    }
+    return out;
+  }
+};
+
+// (out [num_node, hidden], edges per relation)
+py::tuple rgcn_layer(const Tensor& x_in, const Tensor& ptr_in, const Tensor& idx_in, const Tensor& etype_in,
+                     int64_t num_node, const OptTensor& used_in, const OptTensor& hmap_in, const OptTensor& hbuf_in,
+                     bool indexed, const Tensor& weight, bool deterministic, int64_t gather_min_bytes,
+                     int64_t gather_min_feat) {
+  const int64_t R = weight.size(0), F = weight.size(1), H = weight.size(2);
+  const Tensor hm = i64c(some_nonempty(hmap_in), "history_map"), hbuf = rows2d(some_nonempty(hbuf_in));
+  const at::Device dev = require_cuda(x_in, ptr_in, idx_in, etype_in, weight, hm, hbuf, used_in);
+  std::shared_ptr<RgcnBackward> node;
+  if (torch::autograd::compute_requires_grad(x_in, weight)) {
+    node = std::shared_ptr<RgcnBackward>(new RgcnBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(x_in, weight));
+  }
+  at::NoGradGuard no_grad;
+  HC_ON(dev);
+  const Tensor x = rows2d(x_in), ptr = i64c(ptr_in, "ptr"), idx = i64c(idx_in, "idx"), etype = i64c(etype_in, "edge_type");
+  TORCH_CHECK(x.size(1) == F, "rgcn_layer: the weights take ", F, " columns, the rows have ", x.size(1));
+  TORCH_CHECK(ptr.size(0) >= num_node + 1, "rgcn_layer: ptr shorter than num_node + 1");
+  TORCH_CHECK(!hm.defined() || (hm.size(0) >= num_node && hbuf.defined() && (indexed || hbuf.size(0) >= num_node)),
+              "rgcn_layer: history shorter than num_node");
+  const int64_t E = std::min(idx.size(0), etype.size(0)), room = std::max<int64_t>(E, 1);
+  const Tensor used = some(used_in).defined() ? some(used_in).contiguous() : Tensor();
+  Tensor ptr2 = new_i64({num_node * R + 1}, dev), idx2 = new_i64({room}, dev), w2 = new_f32({room}, dev);
+  Tensor count = new_cuda({R + 1}, at::kInt, dev), sc = new_scratch(lib.hc_rgcn_rows_scratch_bytes(), dev);
+  {
+    HC_SPAN("hc_rgcn_rows", dev);
+    check(lib.hc_rgcn_rows(idata(ptr), idata(idx), idata(etype), num_node, E, (int32_t)R, data<uint8_t>(used), idata(hm),
+                           data<int64_t>(ptr2), data<int64_t>(idx2), fdata(w2), data<int32_t>(count), data(sc),
+                           stream_of(dev)), "hc_rgcn_rows");
+  }
+  Tensor sums = new_f32({num_node * R, F}, dev);
+  Block b;
+  b.inp = x; b.ptr = ptr2; b.idx = idx2; b.ev = w2;
+  b.num_node = num_node * R;
+  const hc_aggr_args a = aggr_args(b);
+  {
+    HC_SPAN_ROWS("hc_aggr_fwd", x, dev);
+    check(lib.hc_aggr_fwd(&a, fdata(sums), stream_of(dev)), "hc_aggr_fwd");
+  }
+  g_launches += 2;
+  Tensor out = at::mm(sums.view({num_node, R * F}), weight.reshape({R * F, H}));
+  if (hm.defined()) {
+    TORCH_CHECK(hbuf.size(-1) == H, "rgcn_layer: history rows have another width");
+    HC_SPAN("hc_override_rows", dev);
+    check(lib.hc_override_rows(idata(hm), num_node, data(hbuf), dtype_code(hbuf), row_stride(hbuf, H), indexed ? 1 : 0,
+                               (int32_t)H, fdata(out), stream_of(dev)), "hc_override_rows");
+    ++g_launches;
+  }
+  if (node) {
+    node->x = SavedVariable(x, false);
+    node->weight = SavedVariable(weight, false);
+    node->ptr2 = ptr2; node->idx2 = idx2; node->w2 = w2; node->sums = sums;
+    node->num_node = num_node;
+    node->num_rel = R;
+    node->rule = {deterministic, gather_min_bytes, gather_min_feat};
+    torch::autograd::set_history(out, node);
+  }
+  return py::make_tuple(out, count);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_native, m) {
@@ -1239,4 +1359,5 @@ PYBIND11_MODULE(_native, m) {
         py::arg("want_rel") = false,
         "The relation-segmented block of one RGCN layer (hc_rgcn_group): (ptr2 [num_rel*num_node+1], idx2 [E], w2 [E], "
         "perm or None, rel or None).");
+  m.def("rgcn_layer", &rgcn_layer);
 }

@@ -276,13 +276,15 @@ class MyRGCNConvHistory2(torch.nn.Module):
 
     The reference gives edges with an unused source the relation num_rel (:250), sorts the edges
     by relation (torch.sort), counts them per relation (count_num, :260) and calls
-    cxgnncomp.RGCNOP_sorted, which is not part of the project.  Here hc_rgcn_group does the
-    pruning, the sort (one stable radix pass) and builds a CSR over (relation, destination)
-    rows; ONE pass of the aggregation kernel then reads every source row once per kept edge and
-    leaves the per-(relation, destination) sums, and the typed transform is one product per
-    relation accumulated in place: out = sum_r A[r] @ W[r].  Normalisation is by the total
-    in-degree, as in the reference (:245,272).  Edges into destinations that are served from
-    history are pruned as well (their result is overwritten, :273-274)."""
+    cxgnncomp.RGCNOP_sorted, which is not part of the project.  Here hc_rgcn_rows prunes and orders
+    the edges by relation inside each destination, ONE pass of the aggregation kernel reads every
+    source row once per kept edge and leaves the per-(destination, relation) sums, and the typed
+    transform is one product with the stacked weights.  With more than RGCN_ROWS_MAX_REL relations
+    hc_rgcn_group sorts the edges by relation (stable radix passes) into rows by (relation,
+    destination), and the transform is one product per relation: out = sum_r A[r] @ W[r].
+    Normalisation is by the total in-degree, as in the reference (:245,272).  Edges into
+    destinations that are served from history are pruned as well (their result is overwritten,
+    :273-274)."""
 
     def __init__(self, in_channels, hidden_channels, num_rel, need_grad):
         super().__init__()
@@ -306,23 +308,28 @@ class MyRGCNConvHistory2(torch.nn.Module):
         R = self.num_rel
         has_hist = history_size > 0 and history_map is not None and history_map.numel() > 0
         hmap = history_map[:num_node] if has_hist else None
-        ptr2, idx2, w2, _, rel = hb.rgcn_group(ptr, idx, edge_types, num_node, R, used_src=used_mask,
-                                               hmap=hmap, want_rel=True)
-        # segment sizes per relation, as the reference computes them (:260); value 0 is never
-        # counted there (grad_check.cu:169), so relation 0's size comes from the grouped CSR
-        self.last_count = hb.count_num(rel, R)
         xf = x if x.dtype in (torch.float32, torch.float16) else x.float()
-        agg = hb.aggr_forward(xf, ptr2, idx2, R * num_node, edge_value=w2, force_grad=False)
-        agg = agg.view(R, num_node, -1)
-        out = agg[0] @ self.linear[0]
-        for r in range(1, R):
-            out = torch.addmm(out, agg[r], self.linear[r])
-        if has_hist:
-            hit = hmap != -1
-            rows = hb.gather_rows(history_buffer, hmap if indexed else
-                                  torch.where(hit, torch.arange(num_node, device=x.device), -1),
-                                  zero_missing=True, out_dtype=torch.float32)
-            out = torch.where(hit.unsqueeze(-1), rows, out)
+        if R <= hb.RGCN_ROWS_MAX_REL and self.linear.dtype == torch.float32 and not torch.is_autocast_enabled():
+            out, self.last_count = hb.rgcn_layer(xf, ptr, idx, edge_types, num_node, self.linear, used_src=used_mask,
+                                                 history_map=hmap, history_buffer=history_buffer if has_hist else None,
+                                                 indexed=indexed)
+        else:
+            ptr2, idx2, w2, _, rel = hb.rgcn_group(ptr, idx, edge_types, num_node, R, used_src=used_mask,
+                                                   hmap=hmap, want_rel=True)
+            # segment sizes per relation, as the reference computes them (:260); value 0 is never
+            # counted there (grad_check.cu:169), so relation 0's size comes from the grouped CSR
+            self.last_count = hb.count_num(rel, R)
+            agg = hb.aggr_forward(xf, ptr2, idx2, R * num_node, edge_value=w2, force_grad=False)
+            agg = agg.view(R, num_node, -1)
+            out = agg[0] @ self.linear[0]
+            for r in range(1, R):
+                out = torch.addmm(out, agg[r], self.linear[r])
+            if has_hist:
+                hit = hmap != -1
+                rows = hb.gather_rows(history_buffer, hmap if indexed else
+                                      torch.where(hit, torch.arange(num_node, device=x.device), -1),
+                                      zero_missing=True, out_dtype=torch.float32)
+                out = torch.where(hit.unsqueeze(-1), rows, out)
         his = out
         if self.need_grad and self.training and history_size > 0:
             his.retain_grad()

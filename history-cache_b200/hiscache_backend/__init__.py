@@ -706,6 +706,17 @@ def sample_fixed(gptr, gidx, seeds, local_map, seed, batch_no, fanouts, caps, ed
 # ---------------------------------------------------------------------------
 edge_types = _native.edge_types
 rgcn_group = _native.rgcn_group
+RGCN_ROWS_MAX_REL = 8
+
+
+def rgcn_layer(x, ptr, idx, edge_type, num_node, weight, *, used_src=None, history_map=None, history_buffer=None,
+               indexed=False):
+    """One RGCN layer: out[d] = (1/deg(d)) * sum_e x[src_e] @ weight[rel_e], history rows over it.
+    Returns (out, edges per relation [num_rel + 1] with value 0 never counted, pruned slots last).
+    weight [num_rel, feat, hidden] fp32, at most RGCN_ROWS_MAX_REL relations."""
+    return _native.rgcn_layer(x, ptr, idx, edge_type, int(num_node), used_src, history_map, history_buffer, indexed,
+                              weight, DETERMINISTIC_BWD, GATHER_MIN_BYTES, GATHER_MIN_FEAT)
+
 
 # ---------------------------------------------------------------------------
 # peer copies (kept for API compatibility; the multi-GPU path uses NCCL)

@@ -126,6 +126,9 @@ _SIGS = {
     "hc_select_threshold_masked": (C.c_int, [vp, vp, i64, f32, vp, vp, vp]),
     "hc_record_history_masked": (C.c_int, [vp, i64, i64, vp, i32, i64, i32, vp, vp, vp, vp, vp, vp, vp,
                                            vp, vp, vp, i64, vp, vp, vp]),
+    "hc_rgcn_rows_scratch_bytes": (i64, []),
+    "hc_rgcn_rows": (C.c_int, [vp, vp, vp, i64, i64, i32, vp, vp, vp, vp, vp, vp, vp, vp]),
+    "hc_override_rows": (C.c_int, [vp, i64, vp, i32, i64, i32, i32, vp, vp]),
     "hc_mix64": (C.c_uint64, [C.c_uint64]),
     "hc_bucket_scratch_bytes": (i64, [i64, i32]),
     "hc_bucket_by_owner": (C.c_int, [vp, vp, i64, i32, vp, vp, vp, vp, vp]),

@@ -866,6 +866,23 @@ int hc_rgcn_group(const int64_t* ptr, const int64_t* idx, const int64_t* etype, 
                   int64_t n_edges, int32_t num_rel, const uint8_t* used_src, const int64_t* hmap,
                   int64_t* ptr2, int64_t* idx2, float* w2, int64_t* perm, int64_t* rel_out,
                   void* scratch, void* stream);
+/*
+ * The same block with its rows by destination: row d*num_rel + r of ptr2
+ * ([num_node*num_rel + 1]) lists d's relation-r edges in their order; pruned
+ * edges are in no row.  idx2 / w2 [n_edges].  count [num_rel + 1]: edges per
+ * relation (value 0 is not counted, as in hc_count_num), all slots in no row
+ * last.  num_rel <= 8, else -HC_ERR_UNSUPPORTED.  One cooperative launch.
+ * scratch: device, 8-byte aligned, >= hc_rgcn_rows_scratch_bytes().
+ */
+int64_t hc_rgcn_rows_scratch_bytes(void);
+int hc_rgcn_rows(const int64_t* ptr, const int64_t* idx, const int64_t* etype,
+                 int64_t num_node, int64_t n_edges, int32_t num_rel,
+                 const uint8_t* used_src, const int64_t* hmap, int64_t* ptr2,
+                 int64_t* idx2, float* w2, int32_t* count, void* scratch, void* stream);
+/* out[d, 0:feat] (fp32, dense) = row hmap[d] (indexed) or d of table where
+ * hmap[d] != -1 (hiscache/history_model.py:273-274); other rows stay. */
+int hc_override_rows(const int64_t* hmap, int64_t n, const void* table, int32_t table_dtype,
+                     int64_t stride, int32_t indexed, int32_t feat, float* out, void* stream);
 
 #ifdef __cplusplus
 }
