@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(256)
     aggr_bwd_vec_kernel(const hc_aggr_args a, const float* __restrict__ grad_out,
                         float* __restrict__ grad_input, float* __restrict__ grad_history,
                         float* __restrict__ row_score_out, const int score_kind, const int nvec,
-                        const int64_t gi_stride, float* __restrict__ edge_grad) {
+                        const int64_t gi_stride, float* __restrict__ edge_grad, const int64_t go_stride) {
   HC_BAIL_IF_BAD()
   constexpr int EPW = kWarp / G;
   const int lane = threadIdx.x & 31;
@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
   for (int k = 0; k < V; ++k) {
     const int v = gl + k * G;
-    g[k] = v < nvec ? __ldg(reinterpret_cast<const float4*>(grad_out + t * F) + v)
+    g[k] = v < nvec ? __ldg(reinterpret_cast<const float4*>(grad_out + t * go_stride) + v)
                     : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 
@@ -815,6 +815,18 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// grad_input before the scatter: row r < rooted starts from root[r], the others from zero
+__global__ void __launch_bounds__(256)
+    start_rows_kernel(float* __restrict__ grad_input, const int64_t rows, const int64_t nvec,
+                      const float* __restrict__ root, const int64_t root_stride, const int64_t rooted) {
+  const int64_t total = rows * nvec;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = i / nvec;
+    reinterpret_cast<float4*>(grad_input)[i] =
+        r < rooted ? *reinterpret_cast<const float4*>(root + r * root_stride + 4 * (i - r * nvec)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
@@ -954,12 +966,12 @@ static bool launch_fwd(const FwdLaunch& l, int vb) {
 template <bool EV>
 static void launch_bwd_vec(int G, int V, dim3 grid, cudaStream_t st, const hc_aggr_args& a,
                            const float* grad_out, float* grad_input, float* grad_history,
-                           float* row_score, int score_kind, int nvec, int64_t gi_stride) {
+                           float* row_score, int score_kind, int nvec, int64_t gi_stride, int64_t go_stride) {
 #define HC_BWD_CASE(g, v)                                                                  \
   if (G == g && V == v) {                                                                  \
     aggr_bwd_vec_kernel<g, v, EV><<<grid, 256, 0, st>>>(a, grad_out, grad_input,           \
                                                         grad_history, row_score,           \
-                                                        score_kind, nvec, gi_stride, nullptr); \
+                                                        score_kind, nvec, gi_stride, nullptr, go_stride); \
     return;                                                                                \
   }
   HC_BWD_CASE(8, 1) HC_BWD_CASE(16, 1) HC_BWD_CASE(32, 1) HC_BWD_CASE(32, 2)
@@ -978,7 +990,7 @@ static void launch_bwd_heads(int G, int V, dim3 grid, cudaStream_t st, const hc_
     aggr_bwd_vec_kernel<g, v, true, MH, EG><<<grid, 256, 0, st>>>(a, grad_out, grad_input,         \
                                                                   grad_history, row_score,         \
                                                                   score_kind, nvec, gi_stride,     \
-                                                                  edge_grad);                      \
+                                                                  edge_grad, a.feat);              \
     return;                                                                                        \
   }
   HC_BWD_CASE(8, 1) HC_BWD_CASE(16, 1) HC_BWD_CASE(32, 1) HC_BWD_CASE(32, 2)
@@ -1065,17 +1077,30 @@ extern "C" int hc_aggr_fwd(const hc_aggr_args* args, float* out, void* stream) {
   return 0;
 }
 
-extern "C" int hc_aggr_bwd(const hc_aggr_args* args, const float* grad_out, float* grad_input,
-                           int32_t zero_grad_input, float* grad_history, float* edge_grad,
-                           float* row_score, int32_t score_kind, void* stream) {
+extern "C" int hc_aggr_bwd_rooted(const hc_aggr_args* args, const float* grad_out, int64_t go_stride, const float* root,
+                                  int64_t root_stride, float* grad_input, int32_t zero_grad_input,
+                                  float* grad_history, float* edge_grad, float* row_score, int32_t score_kind,
+                                  void* stream) {
   hc_aggr_args a;
   int rc = validate(args, &a);
   if (rc) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int64_t row = (int64_t)a.num_head * a.feat;
   const int64_t gi_stride = row;  // grad_input is dense [n_src, num_head, feat]
-  if (grad_input && zero_grad_input && a.n_src > 0)
-    HC_CUDA(cudaMemsetAsync(grad_input, 0, (size_t)a.n_src * row * sizeof(float), st));
+  if (go_stride == 0) go_stride = row;
+  if (root && root_stride == 0) root_stride = row;
+  HC_REQUIRE(go_stride >= row && (!root || root_stride >= row), HC_ERR_SIZE);
+  HC_REQUIRE(!root || (grad_input && a.num_node <= a.n_src), HC_ERR_UNSUPPORTED);
+  if (grad_input && zero_grad_input && a.n_src > 0) {
+    if (root) {
+      HC_REQUIRE(row % 4 == 0 && root_stride % 4 == 0 && aligned16(root) && aligned16(grad_input), HC_ERR_UNSUPPORTED);
+      const int64_t blocks = ceil_div(a.n_src * row / 4, 256 * 4);
+      start_rows_kernel<<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, st>>>(grad_input, a.n_src, row / 4, root,
+                                                                                         root_stride, a.num_node);
+    } else {
+      HC_CUDA(cudaMemsetAsync(grad_input, 0, (size_t)a.n_src * row * sizeof(float), st));
+    }
+  }
   if (a.num_node == 0) return 0;
   HC_REQUIRE(grad_out != nullptr, HC_ERR_NULL);
   HC_REQUIRE(score_kind == HC_SCORE_L2 || score_kind == HC_SCORE_L1, HC_ERR_SIZE);
@@ -1087,7 +1112,7 @@ extern "C" int hc_aggr_bwd(const hc_aggr_args* args, const float* grad_out, floa
     HC_CUDA(cudaMemsetAsync(grad_history, 0, (size_t)a.num_node * a.hsize * sizeof(float), st));
 
   const bool heads = a.num_head > 1;
-  bool vec = a.feat % 4 == 0 && aligned16(grad_out) && (grad_input == nullptr || aligned16(grad_input)) &&
+  bool vec = a.feat % 4 == 0 && aligned16(grad_out) && go_stride % 4 == 0 && (grad_input == nullptr || aligned16(grad_input)) &&
              (grad_history == nullptr || (aligned16(grad_history) && a.hsize % 4 == 0));
   // several heads / the gradient of the edge values: vector path for edge-weighted sums over fp32
   // rows, with per-head (or single-head) history rows
@@ -1101,6 +1126,7 @@ extern "C" int hc_aggr_bwd(const hc_aggr_args* args, const float* grad_out, floa
   int G = 0, V = 0;
   const int nvec = a.feat / 4;
   if (vec) vec = vec_shape(nvec, &G, &V) != 0;
+  HC_REQUIRE(go_stride == row || (vec && !special), HC_ERR_UNSUPPORTED);
   const int64_t targets = a.num_node * a.num_head;
   const int64_t blocks = ceil_div(targets, 8);
   HC_REQUIRE(blocks <= 0x7fffffffLL, HC_ERR_SIZE);
@@ -1118,10 +1144,10 @@ extern "C" int hc_aggr_bwd(const hc_aggr_args* args, const float* grad_out, floa
   } else if (vec) {
     if (a.edge_value)
       launch_bwd_vec<true>(G, V, grid, st, a, grad_out, grad_input, grad_history, row_score,
-                           score_kind, nvec, gi_stride);
+                           score_kind, nvec, gi_stride, go_stride);
     else
       launch_bwd_vec<false>(G, V, grid, st, a, grad_out, grad_input, grad_history, row_score,
-                            score_kind, nvec, gi_stride);
+                            score_kind, nvec, gi_stride, go_stride);
   } else if (!special && a.feat <= 512 && (grad_input == nullptr || aligned16(grad_input))) {
     // four copies of a row per warp: up to 66 KB of shared memory at 512 columns
     const int smem = 8 * 16 * shift_words(a.feat) * 4;
@@ -1141,4 +1167,11 @@ extern "C" int hc_aggr_bwd(const hc_aggr_args* args, const float* grad_out, floa
   }
   HC_LAUNCH_OK();
   return 0;
+}
+
+extern "C" int hc_aggr_bwd(const hc_aggr_args* args, const float* grad_out, float* grad_input,
+                           int32_t zero_grad_input, float* grad_history, float* edge_grad,
+                           float* row_score, int32_t score_kind, void* stream) {
+  return hc_aggr_bwd_rooted(args, grad_out, 0, nullptr, 0, grad_input, zero_grad_input, grad_history, edge_grad, row_score,
+                            score_kind, stream);
 }

@@ -49,7 +49,7 @@ namespace {
   X(hc_stage_host_rows) X(hc_sample_fixed_scratch_bytes) X(hc_sample_batch) X(hc_sample_counts)    \
   X(hc_sample_picks) X(hc_relabel_scratch_bytes) X(hc_relabel) X(hc_relabel_seed)                  \
   X(hc_relabel_reset) X(hc_edge_types) X(hc_rgcn_group_scratch_bytes) X(hc_rgcn_group)             \
-  X(hc_rgcn_rows_scratch_bytes) X(hc_rgcn_rows) X(hc_override_rows)                                \
+  X(hc_aggr_bwd_rooted) X(hc_rgcn_rows_scratch_bytes) X(hc_rgcn_rows) X(hc_override_rows)          \
   X(hc_norm_act_fwd) X(hc_norm_act_bwd)
 
 struct Lib {
@@ -337,6 +337,13 @@ void aggr_bwd_gather(const hc_aggr_args& a, const Transposed& t, const Tensor& g
   g_launches += t.n_edges > 64 ? 4 : 1;
 }
 
+// What the layer behind an aggregation leaves for its backward pass: the gradient of the destination rows
+// that the layer read directly ([num_node, feat], rows may be part of a wider product).  The aggregation's
+// gradient then starts from it, instead of autograd padding it to all sources and adding it up.
+struct RootGrad {
+  Tensor rows;
+};
+
 // which backward a call takes (see the Python module for the measured limits)
 struct BwdRule {
   bool deterministic = false;
@@ -354,6 +361,8 @@ struct AggrBackward : public torch::autograd::Node {
   Tensor score;
   int score_kind = HC_SCORE_L2;
   BwdRule rule;
+  const c10::TensorImpl* source = nullptr;       // the input tensor (only compared)
+  std::shared_ptr<RootGrad> root;
 
   std::string name() const override { return "AggrBackward"; }
   void release_variables() override {
@@ -382,7 +391,8 @@ variable_list AggrBackward::apply(variable_list&& grads) {
                : at::zeros({num_node, b.inp.size(1)}, b.inp.options().dtype(at::kFloat));
   }
   if (go.scalar_type() != at::kFloat) go = go.to(at::kFloat);
-  go = go.contiguous();
+  Tensor root_rows;
+  if (root) std::swap(root_rows, root->rows);
   const bool need_in = task_should_compute_output(0);
   const bool need_ev = b.ev.defined() && task_should_compute_output(1);
   const bool need_h = b.hbuf.defined() && task_should_compute_output(2);
@@ -395,6 +405,15 @@ variable_list AggrBackward::apply(variable_list&& grads) {
   Tensor g_in, g_ev, g_h;
   if (need_in) g_in = new_f32(b.inp.sizes(), dev);
   if (need_ev) g_ev = new_f32(b.ev.sizes(), dev);
+  // one scatter takes rows that are part of a wider product as they lie
+  const bool by_source = (need_in || need_ev) && !rule.deterministic &&
+                         (int64_t)a.feat * a.num_head >= rule.gather_min_feat &&
+                         a.n_src * (int64_t)a.feat * a.num_head * 4 >= rule.gather_min_bytes;
+  const bool plain = !multi && !b.ev.defined() && a.feat % 4 == 0 && !by_source && !rule.deterministic;
+  if (!(plain && go.stride(-1) == 1 && go.stride(0) % 4 == 0 && ((uintptr_t)go.data_ptr() & 15) == 0)) go = go.contiguous();
+  Tensor root_start = plain && root_rows.defined() && need_in && root_rows.stride(-1) == 1 && root_rows.stride(0) % 4 == 0 &&
+                              ((uintptr_t)root_rows.data_ptr() & 15) == 0
+                          ? root_rows : Tensor();
   // Three forms.  A reproducible backward gathers over the sorted transposition.  Otherwise blocks
   // that gather enough are differentiated by source, and the rest scatter.
   bool gathered = false, edges_done = false;
@@ -404,8 +423,7 @@ variable_list AggrBackward::apply(variable_list&& grads) {
       t = transpose_block(a, b.idx.numel(), dev);
     aggr_bwd_gather(a, t, go, g_in, dev, b.inp);
     gathered = true;
-  } else if ((need_in || need_ev) && !rule.deterministic && (int64_t)a.feat * a.num_head >= rule.gather_min_feat &&
-             a.n_src * (int64_t)a.feat * a.num_head * 4 >= rule.gather_min_bytes) {
+  } else if (by_source) {
     const int64_t bytes = lib.hc_aggr_bwd_source_scratch_bytes(&a, b.idx.numel(), g_ev.defined());
     if (bytes >= 0) {
       Tensor sc = new_scratch(bytes, dev);
@@ -422,11 +440,14 @@ variable_list AggrBackward::apply(variable_list&& grads) {
   }
   if (!gathered || need_h || row_score.defined()) {
     HC_SPAN_ROWS("hc_aggr_bwd", b.inp, dev);
-    check(lib.hc_aggr_bwd(&a, fdata(go), gathered ? nullptr : fdata(g_in), 1, fdata(g_h), edges_done ? nullptr : fdata(g_ev),
-                          fdata(row_score), score_kind, stream_of(dev)),
+    check(lib.hc_aggr_bwd_rooted(&a, fdata(go), multi ? 0 : go.stride(0), fdata(root_start),
+                                 root_start.defined() ? root_start.stride(0) : 0, gathered ? nullptr : fdata(g_in), 1,
+                                 fdata(g_h), edges_done ? nullptr : fdata(g_ev), fdata(row_score), score_kind,
+                                 stream_of(dev)),
           "hc_aggr_bwd");
     ++g_launches;
   }
+  if (g_in.defined() && root_rows.defined() && !root_start.defined()) g_in.slice(0, 0, num_node).add_(root_rows);
   if (row_score.defined() && sink) sink->fresh = true;
   if (g_in.defined()) out[0] = g_in.scalar_type() == b.inp.scalar_type() ? g_in : g_in.to(b.inp.scalar_type());
   if (g_ev.defined()) out[1] = g_ev;
@@ -506,6 +527,7 @@ Tensor aggr(const Tensor& input, const Tensor& ptr, const Tensor& idx, int64_t n
     }
     node->score_kind = score_kind;
     node->rule = {deterministic, gather_min_bytes, gather_min_feat};
+    node->source = input.unsafeGetTensorImpl();
     torch::autograd::set_history(out, node);
   } else if (force_grad) {
     out.set_requires_grad(true);
@@ -1258,6 +1280,107 @@ py::tuple rgcn_layer(const Tensor& x_in, const Tensor& ptr_in, const Tensor& idx
   return py::make_tuple(out, count);
 }
 
+// ---------------------------------------------------------------------------
+// dense part of a SAGE layer: lin_l(aggregate) + lin_r(x[:num_node]) as one product over
+// [aggregate | root].  The weight gradient of such tall, narrow products has a very long reduction and a
+// small output, which the library runs on a few dozen blocks: the rows are cut into slabs, one batched
+// product gives the slabs' weight gradients, a batched ones-row product their bias gradients, and a sum over
+// the slabs finishes both.  The order of the additions is fixed.
+// ---------------------------------------------------------------------------
+struct SageLinearBackward : public torch::autograd::Node {
+  SavedVariable weight;      // [wl | wr]
+  Tensor rows;               // [aggregate | root]
+  std::shared_ptr<RootGrad> root;
+  int64_t K = 0, n_src = 0, slabs = 8;
+  bool has_bias = false, released = false;
+  at::ScalarType root_type = at::kFloat;
+
+  std::string name() const override { return "SageLinearBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    weight.reset_data();
+    rows = Tensor();
+    released = true;
+  }
+  variable_list apply(variable_list&& grads) override {      // his, wl, bias, wr, x
+    std::lock_guard<std::mutex> lock(mutex_);
+    TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+    at::NoGradGuard no_grad;
+    variable_list out(5);
+    if (!grads[0].defined()) return out;
+    c10::cuda::CUDAGuard guard(rows.device());
+    const Tensor g = grads[0].contiguous(), w = weight.unpack();
+    const int64_t n = rows.size(0);
+    const bool want_x = task_should_compute_output(4);
+    if (task_should_compute_output(0) || want_x || root) {
+      const Tensor g2 = at::mm(g, w);
+      out[0] = g2.narrow(1, 0, K);
+      if (root) root->rows = g2.narrow(1, K, K);
+      if (want_x) {
+        out[4] = at::zeros({n_src, K}, rows.options().dtype(root_type));
+        out[4].slice(0, 0, n).copy_(g2.narrow(1, K, K));
+      }
+    }
+    int64_t s = slabs;
+    while (s > 1 && (n % s || n / s < 256)) s /= 2;
+    const bool want_l = task_should_compute_output(1), want_r = task_should_compute_output(3),
+               want_b = has_bias && task_should_compute_output(2);
+    if (s > 1) {
+      const Tensor gs = g.view({s, n / s, -1}), rs = rows.view({s, n / s, -1});
+      if (want_l || want_r) {
+        const Tensor parts = at::bmm(gs.transpose(1, 2), rs);
+        if (want_l) out[1] = parts.narrow(2, 0, K).sum(0);
+        if (want_r) out[3] = parts.narrow(2, K, K).sum(0);
+      }
+      if (want_b) out[2] = at::bmm(at::ones({s, 1, n / s}, g.options()), gs).sum(0).reshape({-1});
+    } else {
+      if (want_l) out[1] = at::mm(g.t(), rows.narrow(1, 0, K));
+      if (want_r) out[3] = at::mm(g.t(), rows.narrow(1, K, K));
+      if (want_b) out[2] = g.sum(0);
+    }
+    return out;
+  }
+};
+
+Tensor sage_linear(const Tensor& his, const Tensor& x, int64_t num_node, const Tensor& wl, const OptTensor& bias_in,
+                   const Tensor& wr, int64_t slabs) {
+  const Tensor bias = some(bias_in);
+  const at::Device dev = require_cuda(his, x, wl, bias, wr);
+  const int64_t K = his.size(1);
+  TORCH_CHECK(his.size(0) == num_node && x.size(0) >= num_node && x.size(1) == K && wl.size(1) == K && wr.sizes() == wl.sizes(),
+              "sage_linear: shapes do not match");
+  std::shared_ptr<SageLinearBackward> node;
+  if (torch::autograd::compute_requires_grad(his, wl, bias, wr, x)) {
+    node = std::shared_ptr<SageLinearBackward>(new SageLinearBackward(), torch::autograd::deleteNode);
+    auto edges = torch::autograd::collect_next_edges(his, wl, bias, wr, x);
+    // when `his` is the aggregation of this very x, its backward pass takes x's second gradient along
+    auto* aggr = dynamic_cast<AggrBackward*>(his.grad_fn().get());
+    if (aggr && aggr->source == x.unsafeGetTensorImpl() && x.requires_grad() && aggr->num_node == num_node && !aggr->root) {
+      node->root = aggr->root = std::make_shared<RootGrad>();
+      edges[4] = torch::autograd::Edge();
+    }
+    node->set_next_edges(std::move(edges));
+  }
+  at::NoGradGuard no_grad;
+  HC_ON(dev);
+  Tensor rows = new_f32({num_node, 2 * K}, dev);
+  rows.narrow(1, 0, K).copy_(his);
+  rows.narrow(1, K, K).copy_(x.slice(0, 0, num_node));
+  const Tensor w = at::cat({wl, wr}, 1);
+  Tensor out = bias.defined() ? at::addmm(bias, rows, w.t()) : at::mm(rows, w.t());
+  if (node) {
+    node->weight = SavedVariable(w, false);
+    node->rows = rows;
+    node->K = K;
+    node->n_src = x.size(0);
+    node->slabs = slabs;
+    node->has_bias = bias.defined();
+    node->root_type = x.scalar_type();
+    torch::autograd::set_history(out, node);
+  }
+  return out;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_native, m) {
@@ -1360,4 +1483,5 @@ PYBIND11_MODULE(_native, m) {
         "The relation-segmented block of one RGCN layer (hc_rgcn_group): (ptr2 [num_rel*num_node+1], idx2 [E], w2 [E], "
         "perm or None, rel or None).");
   m.def("rgcn_layer", &rgcn_layer);
+  m.def("sage_linear", &sage_linear);
 }

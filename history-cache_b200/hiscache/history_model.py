@@ -17,56 +17,10 @@ from .util import cfg_get
 
 import os
 
+# lin_l(aggregate) + lin_r(root) as one product (hiscache_backend.sage_linear)
 FUSE_ROOT_PRODUCT = os.environ.get("HISCACHE_FUSE_ROOT_PRODUCT", "1") not in ("", "0")
-
-
+# row slabs of its weight gradient
 SPLIT_WGRAD = int(os.environ.get("HISCACHE_SPLIT_WGRAD", "8"))
-
-
-class _TallLinear(torch.autograd.Function):
-    """y = x @ w.T + b for tall, narrow x (tens of thousands of rows, a few hundred columns).
-
-    The forward product is cuBLAS as usual.  The weight gradient x.T @ g of such a shape is a
-    product with a very long reduction and a small output, which the library runs on a few dozen
-    thread blocks (measured: 80 us per layer, the largest dense kernel of a step), and the bias
-    gradient is a column sum that torch's generic reduction does at a fraction of the bandwidth.
-    Here the rows are cut into SPLIT_WGRAD slabs: one batched product gives the slabs' weight
-    gradients, a batched ones-row product their bias gradients, and a small sum over the slabs
-    finishes both.  The order of the additions is fixed, so the result is reproducible."""
-
-    @staticmethod
-    def forward(ctx, x, w, b):
-        ctx.save_for_backward(x, w)
-        ctx.has_bias = b is not None
-        return torch.addmm(b, x, w.t()) if b is not None else x @ w.t()
-
-    @staticmethod
-    def backward(ctx, g):
-        x, w = ctx.saved_tensors
-        g = g.contiguous()
-        n = x.shape[0]
-        gx = g @ w if ctx.needs_input_grad[0] else None
-        s = SPLIT_WGRAD
-        while s > 1 and (n % s or n // s < 256):
-            s //= 2
-        gw = gb = None
-        if s > 1 and x.is_contiguous():
-            gs, xs = g.view(s, n // s, -1), x.view(s, n // s, -1)
-            if ctx.needs_input_grad[1]:
-                gw = torch.bmm(gs.transpose(1, 2), xs).sum(0)
-            if ctx.has_bias and ctx.needs_input_grad[2]:
-                ones = torch.ones((s, 1, n // s), dtype=g.dtype, device=g.device)
-                gb = torch.bmm(ones, gs).sum(0).reshape(-1)
-        else:
-            if ctx.needs_input_grad[1]:
-                gw = g.t() @ x
-            if ctx.has_bias and ctx.needs_input_grad[2]:
-                gb = g.sum(0)
-        return gx, gw, gb
-
-
-def tall_linear(x, w, b):
-    return _TallLinear.apply(x, w, b) if SPLIT_WGRAD > 1 else F.linear(x, w, b)
 
 
 class MaskedBatchNorm1d(torch.nn.BatchNorm1d):
@@ -165,14 +119,14 @@ class MySageConvHistory(torch.nn.Module):
         if self.need_grad and self.training and history_size > 0:
             his.retain_grad()
         if self.root_weight:
-            root = x[:num_node] if num_node != 0 else x
-            root = root if root.dtype == out.dtype else root.to(out.dtype)
-            if FUSE_ROOT_PRODUCT:
+            if FUSE_ROOT_PRODUCT and self.lin_l.weight.dtype == torch.float32:
                 # lin_l(aggr) + lin_r(root) as ONE product over [aggr | root]: half the GEMM launches of
                 # the layer in forward and backward (their shapes are small and launch-bound)
-                w = torch.cat([self.lin_l.weight, self.lin_r.weight], dim=1)
-                out = tall_linear(torch.cat([out, root], dim=1), w, self.lin_l.bias)
+                out = hb.sage_linear(out, x, num_node, self.lin_l.weight, self.lin_l.bias, self.lin_r.weight,
+                                     SPLIT_WGRAD)
             else:
+                root = x[:num_node] if num_node != 0 else x
+                root = root if root.dtype == out.dtype else root.to(out.dtype)
                 out = self.lin_l(out) + self.lin_r(root)
         else:
             out = self.lin_l(out)

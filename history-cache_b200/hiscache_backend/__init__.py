@@ -719,6 +719,11 @@ def rgcn_layer(x, ptr, idx, edge_type, num_node, weight, *, used_src=None, histo
 
 
 # ---------------------------------------------------------------------------
+# dense part of a SAGE layer
+# ---------------------------------------------------------------------------
+sage_linear = _native.sage_linear       # (his, x, num_node, w_l, bias, w_r, slabs)
+
+# ---------------------------------------------------------------------------
 # peer copies (kept for API compatibility; the multi-GPU path uses NCCL)
 # ---------------------------------------------------------------------------
 def p2psend(tsrc, tdst, num_element, target_device):

@@ -138,6 +138,18 @@ int hc_aggr_fwd(const hc_aggr_args* a, float* out, void* stream);
 int hc_aggr_bwd(const hc_aggr_args* a, const float* grad_out, float* grad_input,
                 int32_t zero_grad_input, float* grad_history, float* edge_grad,
                 float* row_score, int32_t score_kind, void* stream);
+/*
+ * hc_aggr_bwd for a layer that also reads its destination rows directly:
+ * grad_out has go_stride elements between rows (0 = dense; rows need not be
+ * dense, e.g. half of a wider product), and row r < num_node of grad_input
+ * starts from root[r, :] (stride root_stride, NULL = zeros).  Strides other
+ * than dense, and root, need feat % 4 == 0, 16-byte aligned rows, one head and
+ * no edge_grad, else -HC_ERR_UNSUPPORTED.
+ */
+int hc_aggr_bwd_rooted(const hc_aggr_args* a, const float* grad_out, int64_t go_stride,
+                       const float* root, int64_t root_stride, float* grad_input,
+                       int32_t zero_grad_input, float* grad_history, float* edge_grad,
+                       float* row_score, int32_t score_kind, void* stream);
 
 /*
  * Index checks (a library built with -DHC_CHECK_BOUNDS, libhiscache_b200_checked.so).

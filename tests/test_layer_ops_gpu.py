@@ -63,3 +63,56 @@ def test_rgcn_layer(backend, oracle, seeds, rel, feat, hidden, dt, used, hist):
     c[0] = 0
     assert np.array_equal(count.cpu().numpy()[:rel], c)
     assert int(count[rel]) == len(idx) - keep
+
+
+@pytest.mark.parametrize("feat,hidden,seeds,bias", [(8, 12, 3, True), (100, 256, 40, True), (33, 7, 9, False),
+                                                    (256, 47, 200, True)])
+@pytest.mark.parametrize("mode", ["scatter", "source", "deterministic"])
+@pytest.mark.parametrize("dt", [torch.float32, torch.float16])
+def test_sage_linear_takes_both_gradients_along(backend, monkeypatch, feat, hidden, seeds, bias, mode, dt):
+    monkeypatch.setattr(backend, "DETERMINISTIC_BWD", mode == "deterministic")
+    monkeypatch.setattr(backend, "GATHER_MIN_BYTES", 0 if mode == "source" else 1 << 60)
+    monkeypatch.setattr(backend, "GATHER_MIN_FEAT", 0)
+    ptr, idx, nn = block(seeds, seeds, [10, 5], 5000)
+    n, n_all = nn[1], nn[-1]
+    x = (torch.randn(n_all, feat, device="cuda")).to(dt).requires_grad_()
+    wl = (torch.randn(hidden, feat, device="cuda") * 0.1).requires_grad_()
+    wr = (torch.randn(hidden, feat, device="cuda") * 0.1).requires_grad_()
+    b = torch.randn(hidden, device="cuda").requires_grad_() if bias else None
+    his = backend.aggr_forward(x, cu(ptr), cu(idx), n)
+    his.retain_grad()
+    out = backend.sage_linear(his, x, n, wl, b, wr, 8)
+    g = torch.randn_like(out)
+    params = [p for p in (x, wl, wr, b) if p is not None]
+    out.backward(g, retain_graph=True)
+    first = [p.grad.clone() for p in params]
+    for p in params:
+        p.grad = None
+    out.backward(g)                       # a second pass over the same graph gives the same
+    d = [p.detach().double().requires_grad_() for p in params]
+    deg = np.diff(ptr)[:n]
+    e = int(ptr[n])
+    dst = cu(np.repeat(np.arange(n), deg))
+    hd = torch.zeros(n, feat, dtype=torch.float64, device="cuda").index_add(0, dst, d[0][cu(idx[:e])])
+    hd = hd / cu(np.maximum(deg, 1)).double()[:, None]
+    hd.retain_grad()
+    want = hd @ d[1].t() + d[0][:n] @ d[2].t() + (d[3] if bias else 0)
+    want.backward(g.double())
+    assert (out.double() - want).abs().max() <= 2e-5 * (1 + want.abs().max())
+    assert (his.grad.double() / 2 - hd.grad).abs().max() <= 2e-5 * (1 + hd.grad.abs().max())
+    for got, again, w in zip(first, params, d):
+        tol = 2e-3 if got.dtype == torch.float16 else 3e-5
+        assert (got.double() - w.grad).abs().max() <= tol * (1 + w.grad.abs().max())
+        assert (again.grad.double() - w.grad).abs().max() <= tol * (1 + w.grad.abs().max())
+
+
+def test_sage_linear_with_an_unrelated_aggregate(backend):
+    x = torch.randn(50, 12, device="cuda", requires_grad=True)
+    his = torch.randn(20, 12, device="cuda", requires_grad=True)
+    wl, wr = (torch.randn(5, 12, device="cuda", requires_grad=True) for _ in range(2))
+    out = backend.sage_linear(his, x, 20, wl, None, wr, 8)
+    g = torch.randn_like(out)
+    out.backward(g)
+    assert torch.allclose(out, his @ wl.t() + x[:20] @ wr.t(), atol=1e-4)
+    assert torch.allclose(his.grad, g @ wl, atol=1e-4)
+    assert torch.allclose(x.grad[:20], g @ wr, atol=1e-4) and not x.grad[20:].any()
