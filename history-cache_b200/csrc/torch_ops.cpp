@@ -50,6 +50,7 @@ namespace {
   X(hc_sample_picks) X(hc_relabel_scratch_bytes) X(hc_relabel) X(hc_relabel_seed)                  \
   X(hc_relabel_reset) X(hc_edge_types) X(hc_rgcn_group_scratch_bytes) X(hc_rgcn_group)             \
   X(hc_aggr_bwd_rooted) X(hc_rgcn_rows_scratch_bytes) X(hc_rgcn_rows) X(hc_override_rows)          \
+  X(hc_adam_step)                                                                                  \
   X(hc_norm_act_fwd) X(hc_norm_act_bwd)
 
 struct Lib {
@@ -1381,6 +1382,38 @@ Tensor sage_linear(const Tensor& his, const Tensor& x, int64_t num_node, const T
   return out;
 }
 
+// ---------------------------------------------------------------------------
+// optimiser
+// ---------------------------------------------------------------------------
+void adam_step(const std::vector<Tensor>& params, const std::vector<Tensor>& grads, const std::vector<Tensor>& avgs,
+               const std::vector<Tensor>& avg_sqs, const std::vector<Tensor>& steps, double lr, double beta1, double beta2,
+               double eps) {
+  if (params.empty()) return;
+  at::NoGradGuard no_grad;
+  const at::Device dev = params[0].device();
+  HC_ON(dev);
+  const size_t n = params.size();
+  std::vector<void*> p(n), m(n), v(n), t(n);
+  std::vector<const void*> g(n);
+  std::vector<int64_t> numel(n);
+  std::vector<Tensor> keep;
+  for (size_t k = 0; k < n; ++k) {
+    Tensor gr = grads[k];
+    if (!gr.is_contiguous()) keep.push_back(gr = gr.contiguous());
+    p[k] = params[k].data_ptr();
+    g[k] = gr.data_ptr();
+    m[k] = avgs[k].data_ptr();
+    v[k] = avg_sqs[k].data_ptr();
+    t[k] = steps[k].data_ptr();
+    numel[k] = params[k].numel();
+  }
+  HC_SPAN("hc_adam_step", dev);
+  check(lib.hc_adam_step(p.data(), g.data(), m.data(), v.data(), t.data(), numel.data(), (int32_t)n, lr, beta1, beta2, eps,
+                         stream_of(dev)), "hc_adam_step");
+  g_launches += 2;
+  for (const auto* list : {&params, &avgs, &avg_sqs, &steps})
+    for (const Tensor& x : *list) torch::autograd::impl::bump_version(x);
+}
 }  // namespace
 
 PYBIND11_MODULE(_native, m) {
@@ -1484,4 +1517,5 @@ PYBIND11_MODULE(_native, m) {
         "perm or None, rel or None).");
   m.def("rgcn_layer", &rgcn_layer);
   m.def("sage_linear", &sage_linear);
+  m.def("adam_step", &adam_step);
 }

@@ -18,6 +18,7 @@ from .feature_store import HostFeatureStore
 from .history_cache import HistoryCache
 from .history_model import get_model
 from .sampler import get_loader, wait_ready
+from .optim import Adam
 from .util import cfg_get, log
 
 
@@ -43,8 +44,8 @@ class HistoryTableTrainer:
         self.uvm = uvm
         self.table = HistoryTable(config, total_num_node=g.num_nodes, storage_dtype=storage_dtype)
         self.model = get_model(config, self.table).to(self.device)
-        self.optimizer = torch.optim.Adam(self.model.parameters(), lr=cfg_get(config, "train.optimizer.lr", 1e-3),
-                                          fused=True, capturable=True)
+        self.optimizer = Adam(self.model.parameters(), lr=cfg_get(config, "train.optimizer.lr", 1e-3),
+                              fused=True, capturable=True)
         self.loss_fn = F.nll_loss
         self.num_layer = len(self.model.convs)
         self.glb_iter = 0
@@ -124,8 +125,8 @@ class HistoryTrainer:
                                   sorted_indices=self.loader.graph.sorted_indices,
                                   storage_dtype=storage_dtype)
         self.model = get_model(config, self.table).to(self.device)
-        self.optimizer = torch.optim.Adam(self.model.parameters(), lr=cfg_get(config, "train.optimizer.lr", 1e-3),
-                                          fused=True, capturable=True)
+        self.optimizer = Adam(self.model.parameters(), lr=cfg_get(config, "train.optimizer.lr", 1e-3),
+                              fused=True, capturable=True)
         self.scheduler = torch.optim.lr_scheduler.LambdaLR(self.optimizer, lambda _: 1.0)
         self.loss_fn = F.nll_loss
         self.type = config.train.type.lower()

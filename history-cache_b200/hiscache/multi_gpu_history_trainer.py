@@ -20,6 +20,7 @@ from .history_cache import HistoryCache
 from .history_model import get_model
 from .sampler import get_loader, wait_ready
 from .sharded import PeerHistoryTable, ShardedHistoryTable
+from .optim import Adam
 from .util import cfg_get, log
 
 
@@ -172,8 +173,8 @@ class MultiGpuHistoryTrainer:
         self.model = get_model(config, self.table).to(self.device)
         self.models = [self.model]
         self.num_layer = len(self.model.convs)
-        self.optimizer = torch.optim.Adam(self.model.parameters(), lr=cfg_get(config, "train.optimizer.lr", 1e-3),
-                                          fused=True, capturable=True)
+        self.optimizer = Adam(self.model.parameters(), lr=cfg_get(config, "train.optimizer.lr", 1e-3),
+                              fused=True, capturable=True)
         # enable_cuda_graph() replays the step as two captured segments with the collectives
         # issued eagerly between them (hiscache/graphed.py); no collective is ever captured.
         self.graphed = None

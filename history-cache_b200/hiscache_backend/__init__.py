@@ -719,9 +719,10 @@ def rgcn_layer(x, ptr, idx, edge_type, num_node, weight, *, used_src=None, histo
 
 
 # ---------------------------------------------------------------------------
-# dense part of a SAGE layer
+# dense part of a SAGE layer, optimiser
 # ---------------------------------------------------------------------------
 sage_linear = _native.sage_linear       # (his, x, num_node, w_l, bias, w_r, slabs)
+adam_step = _native.adam_step           # (params, grads, exp_avgs, exp_avg_sqs, steps, lr, beta1, beta2, eps)
 
 # ---------------------------------------------------------------------------
 # peer copies (kept for API compatibility; the multi-GPU path uses NCCL)

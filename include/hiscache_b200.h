@@ -792,6 +792,16 @@ int hc_sample_batch(const int64_t* gptr, const int64_t* gidx, const int64_t* see
                     int32_t* local_map, uint64_t seed, int64_t* batch_no, const int64_t* labels,
                     int64_t* y, const hc_fixed_batch* b, void* scratch, void* stream);
 
+/*
+ * One Adam step over n fp32 tensors (host arrays of device pointers): steps[k]
+ * (float, one per tensor) is advanced, then with t = steps[k]
+ *   m = beta1 m + (1 - beta1) g;  v = beta2 v + (1 - beta2) g^2
+ *   p -= lr / (1 - beta1^t) * m / (sqrt(v) / sqrt(1 - beta2^t) + eps).
+ */
+int hc_adam_step(void* const* params, const void* const* grads, void* const* avgs,
+                 void* const* avg_sqs, void* const* steps, const int64_t* numels, int32_t n,
+                 double lr, double beta1, double beta2, double eps, void* stream);
+
 /* ---------------------------------------------------------------------------
  * Dense epilogue of a layer: batch norm (training statistics) + ReLU + dropout.
  *

@@ -116,3 +116,29 @@ def test_sage_linear_with_an_unrelated_aggregate(backend):
     assert torch.allclose(out, his @ wl.t() + x[:20] @ wr.t(), atol=1e-4)
     assert torch.allclose(his.grad, g @ wl, atol=1e-4)
     assert torch.allclose(x.grad[:20], g @ wr, atol=1e-4) and not x.grad[20:].any()
+
+
+@pytest.mark.parametrize("sizes", [[1], [3, 1024, 1025, 5000], [64] * 49 + [70000]])
+def test_adam_step_matches_torch(backend, sizes):
+    from hiscache.optim import Adam
+    init = [torch.randn(n, device="cuda") for n in sizes]
+    a, b = ([t.clone().requires_grad_() for t in init] for _ in range(2))
+    ours = Adam(a, lr=3e-3, betas=(0.8, 0.95), fused=True, capturable=True)
+    theirs = torch.optim.Adam(b, lr=3e-3, betas=(0.8, 0.95), fused=True, capturable=True)
+    for step in range(4):
+        for k, (p, q) in enumerate(zip(a, b)):
+            p.grad = torch.randn_like(p) if (k + step) % 3 or len(sizes) == 1 else None
+            q.grad = None if p.grad is None else p.grad.clone()
+        version = a[0]._version
+        ours.step()
+        theirs.step()
+        assert a[0].grad is None or a[0]._version > version
+    for p, q in zip(a, b):
+        assert torch.allclose(p, q, rtol=1e-6, atol=1e-8)
+    so, st = ours.state_dict(), theirs.state_dict()
+    assert so["state"].keys() == st["state"].keys()
+    for k in so["state"]:
+        for name in ("step", "exp_avg", "exp_avg_sq"):
+            assert torch.allclose(so["state"][k][name], st["state"][k][name], rtol=1e-5, atol=1e-7)
+    ours.load_state_dict(st)
+    assert isinstance(ours, torch.optim.Adam)
