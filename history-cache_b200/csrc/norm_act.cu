@@ -10,7 +10,7 @@
 // batches): they do not enter the statistics and produce zeros.
 //
 // The statistics of a batch's 16 K rows are bound by that last block's walk over the partial sums, so its
-// loads are all in flight at once (23 -> 14 us alone at 8 K rows).
+// loads are all in flight at once.
 // Column statistics are reproducible: every block writes its partial sums, the block that
 // finishes last adds them in block order in double precision.
 #include "common.cuh"
@@ -43,46 +43,44 @@ __device__ __forceinline__ unsigned dropout_keep4(uint64_t seed, int64_t step, i
   return m;
 }
 
-// Sum over blocks b of p[b * stride + c] in a fixed order, by the whole block: thread t takes
-// column t % feat and the blocks b = t / feat, t / feat + parts, ... (eight loads in flight), the
-// `parts` partial sums of a column are then added in part order.  red: shared double [2][parts * feat].
-// Returns the two column sums (p and p + feat) to the threads with t < feat; all threads must call.
+// Sum over blocks b of p[b][0:2 * feat] in a fixed order, by the whole block: thread t takes four columns of
+// the 2 * feat and the blocks b = t / (feat / 2), ... + parts (ten 16-byte loads in flight: two rounds for
+// 148 blocks of 256 columns, where single words of both halves took four), the `parts` sums of a column are
+// then added in part order.  red: shared double [parts][2 * feat].  Threads with t < feat get column t's two
+// sums; all threads must call.  feat <= 2 * blockDim.x.
 __device__ __forceinline__ void column_sums(const float* p, int feat, unsigned nb, double* red, double* s0,
                                             double* s1) {
-  const int parts = blockDim.x / feat > 0 ? blockDim.x / feat : 1;
-  const int64_t stride = 2 * (int64_t)feat;
-  for (int base = 0; base < feat; base += blockDim.x) {      // feat > blockDim.x: several rounds
-    const int t = threadIdx.x;
-    const int c = base + (parts > 1 ? t % feat : t);
-    const int part = parts > 1 ? t / feat : 0;
-    double a0 = 0.0, a1 = 0.0;
-    if (c < feat && part < parts) {
-      constexpr int B = 10;      // blocks in flight per thread (two loads each)
-      for (unsigned b0 = part; b0 < nb; b0 += (unsigned)(B * parts)) {
-        float v[B], q[B];
+  const int nv = feat / 2, parts = blockDim.x / nv;
+  const int part = threadIdx.x / nv, cv = threadIdx.x - part * nv;
+  if (part < parts) {
+    constexpr int B = 10;
+    double4 acc = make_double4(0.0, 0.0, 0.0, 0.0);
+    for (unsigned b0 = part; b0 < nb; b0 += (unsigned)(B * parts)) {
+      float4 v[B];
 #pragma unroll
-        for (int j = 0; j < B; ++j) {
-          const unsigned b = b0 + (unsigned)(j * parts);
-          v[j] = b < nb ? __ldcg(p + (int64_t)b * stride + c) : 0.f;
-          q[j] = b < nb ? __ldcg(p + (int64_t)b * stride + feat + c) : 0.f;
-        }
+      for (int j = 0; j < B; ++j) {
+        const unsigned b = b0 + (unsigned)(j * parts);
+        v[j] = b < nb ? __ldcg(reinterpret_cast<const float4*>(p + (int64_t)b * 2 * feat) + cv)
+                      : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
 #pragma unroll
-        for (int j = 0; j < B; ++j) { a0 += (double)v[j]; a1 += (double)q[j]; }
+      for (int j = 0; j < B; ++j) {
+        acc.x += (double)v[j].x; acc.y += (double)v[j].y;
+        acc.z += (double)v[j].z; acc.w += (double)v[j].w;
       }
-      red[part * feat + (c - base)] = a0;
-      red[(parts + part) * feat + (c - base)] = a1;
     }
-    __syncthreads();
-    if (c < feat && part == 0) {
-      double t0 = 0.0, t1 = 0.0;
-      for (int k = 0; k < parts; ++k) {
-        t0 += red[k * feat + (c - base)];
-        t1 += red[(parts + k) * feat + (c - base)];
-      }
-      s0[base / blockDim.x] = t0;
-      s1[base / blockDim.x] = t1;
+    double* to = red + part * 2 * feat + 4 * cv;
+    to[0] = acc.x; to[1] = acc.y; to[2] = acc.z; to[3] = acc.w;
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < feat) {
+    double t0 = 0.0, t1 = 0.0;
+    for (int k = 0; k < parts; ++k) {
+      t0 += red[k * 2 * feat + threadIdx.x];
+      t1 += red[k * 2 * feat + feat + threadIdx.x];
     }
-    __syncthreads();
+    *s0 = t0;
+    *s1 = t1;
   }
 }
 
@@ -179,9 +177,9 @@ __global__ void __launch_bounds__(kStatsBlock) norm_stats_kernel(const NormArgs 
     a.partial_count[blockIdx.x] = c;
   }
   // the block that takes the last ticket reduces all partials in block order
-  __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
+    __threadfence();
     const unsigned t = atomicAdd(a.ticket, 1u);
     is_last = (t == gridDim.x - 1);
   }
@@ -191,6 +189,11 @@ __global__ void __launch_bounds__(kStatsBlock) norm_stats_kernel(const NormArgs 
   // counts are whole numbers below 2^24 per block: their sum is exact in any order
   __shared__ double counted[kStatsBlock / 32];
   double n_valid = threadIdx.x < gridDim.x ? (double)__ldcg(a.partial_count + threadIdx.x) : 0.0;
+  const int c = threadIdx.x;      // feat <= 1024 = blockDim.x: a column a thread
+  const bool run = a.running_mean && c < a.feat;
+  const double old_mean = run ? (double)a.running_mean[c] : 0.0, old_var = run ? (double)a.running_var[c] : 0.0;
+  double sum = 0.0, sq = 0.0;
+  column_sums(a.partial, a.feat, gridDim.x, reinterpret_cast<double*>(sh), &sum, &sq);
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) n_valid += __shfl_xor_sync(kFull, n_valid, off);
   if ((threadIdx.x & 31) == 0) counted[threadIdx.x >> 5] = n_valid;
@@ -198,20 +201,17 @@ __global__ void __launch_bounds__(kStatsBlock) norm_stats_kernel(const NormArgs 
   n_valid = 0.0;
 #pragma unroll
   for (int w = 0; w < (kNormMaxPartials + 31) / 32; ++w) n_valid += counted[w];
-  double cs0[1], cs1[1];
-  column_sums(a.partial, a.feat, gridDim.x, reinterpret_cast<double*>(sh), cs0, cs1);
-  for (int c = threadIdx.x; c < a.feat; c += blockDim.x) {   // feat <= 1024 = blockDim.x: one round
-    const double sum = cs0[0], sq = cs1[0];
+  if (c < a.feat) {
     const double nn = n_valid > 0.0 ? n_valid : 1.0;
     const double mean = sum / nn;
     double var = sq / nn - mean * mean;
     if (var < 0.0) var = 0.0;
     a.save_mean[c] = (float)mean;
     a.save_rstd[c] = (float)(1.0 / sqrt(var + (double)a.eps));
-    if (a.running_mean) {
+    if (run) {
       const double unb = n_valid > 1.0 ? var * (n_valid / (n_valid - 1.0)) : var;
-      a.running_mean[c] = (float)((1.0 - a.momentum) * (double)a.running_mean[c] + a.momentum * mean);
-      a.running_var[c] = (float)((1.0 - a.momentum) * (double)a.running_var[c] + a.momentum * unb);
+      a.running_mean[c] = (float)((1.0 - a.momentum) * old_mean + a.momentum * mean);
+      a.running_var[c] = (float)((1.0 - a.momentum) * old_var + a.momentum * unb);
     }
   }
   if (threadIdx.x == 0) {
@@ -326,19 +326,19 @@ __global__ void __launch_bounds__(kStatsBlock) norm_bwd_stats_kernel(const NormA
     *reinterpret_cast<float4*>(p + 4 * cv) = s;
     *reinterpret_cast<float4*>(p + a.feat + 4 * cv) = q;
   }
-  __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
+    __threadfence();
     const unsigned t = atomicAdd(a.ticket, 1u);
     is_last = (t == gridDim.x - 1);
   }
   __syncthreads();
   if (!is_last) return;
   __threadfence();
-  double cs0[1], cs1[1];
-  column_sums(a.partial, a.feat, gridDim.x, reinterpret_cast<double*>(sh), cs0, cs1);
-  for (int c = threadIdx.x; c < a.feat; c += blockDim.x) {
-    const double sum = cs0[0], sq = cs1[0];
+  double sum = 0.0, sq = 0.0;
+  column_sums(a.partial, a.feat, gridDim.x, reinterpret_cast<double*>(sh), &sum, &sq);
+  const int c = threadIdx.x;
+  if (c < a.feat) {
     bw.sum_dz[c] = (float)sum;
     bw.sum_dzx[c] = (float)sq;
     if (bw.grad_bias) bw.grad_bias[c] = (float)sum;
@@ -415,12 +415,13 @@ static void grids(const NormArgs& a, unsigned* stats_blocks, unsigned* apply_blo
   const NormGeom gs = norm_geom(a.feat, kStatsBlock), ga = norm_geom(a.feat, kNormBlock);
   const int64_t n = a.n > 0 ? a.n : 1;
   const int64_t si = ceil_div(n, gs.rpi), ai = ceil_div(n, ga.rpi);
-  *stats_blocks = (unsigned)(si < kNormMaxPartials ? si : kNormMaxPartials);
+  // a thread's four rows are in flight together: fewer rows a thread only make more partial sums
+  const int64_t sb = ceil_div(si, 4);
+  *stats_blocks = (unsigned)(sb < kNormMaxPartials ? sb : kNormMaxPartials);
   *apply_blocks = (unsigned)(ai < 148 * 8 ? ai : 148 * 8);
   // block partial sums (float4 x 2 per row slot), reused by the last block for the column sums
   size_t need = (size_t)2 * gs.rpi * gs.nvec * sizeof(float4);
-  const int parts = kStatsBlock / a.feat > 0 ? kStatsBlock / a.feat : 1;
-  const size_t fin = (size_t)2 * parts * a.feat * sizeof(double);
+  const size_t fin = (size_t)(kStatsBlock / (a.feat / 2)) * 2 * a.feat * sizeof(double);
   *smem = need > fin ? need : fin;
 }
 
