@@ -50,7 +50,8 @@ namespace {
   X(hc_sample_picks) X(hc_relabel_scratch_bytes) X(hc_relabel) X(hc_relabel_seed)                  \
   X(hc_relabel_reset) X(hc_edge_types) X(hc_rgcn_group_scratch_bytes) X(hc_rgcn_group)             \
   X(hc_aggr_bwd_rooted) X(hc_rgcn_rows_scratch_bytes) X(hc_rgcn_rows) X(hc_override_rows)          \
-  X(hc_adam_step)                                                                                  \
+  X(hc_adam_step) X(hc_sage_pack) X(hc_slab_sums_scratch_bytes) X(hc_slab_sums) X(hc_nll_fwd)      \
+  X(hc_nll_bwd)                                                                                    \
   X(hc_norm_act_fwd) X(hc_norm_act_bwd)
 
 struct Lib {
@@ -1163,9 +1164,49 @@ py::tuple rgcn_group(const Tensor& ptr_in, const Tensor& idx_in, const Tensor& e
   return py::make_tuple(ptr2, cut(idx2), cut(w2), cut(perm), cut(rel));
 }
 
+// g^T r for tall, narrow g [n, M] and r [n, N]: columns [0, split) of the result into left, the others into
+// right; column sums of g into bias (undefined = not wanted).  Such a product has a very long reduction and a
+// small output, which the library runs on a few dozen blocks: the rows are cut into slabs of at least 256, one
+// batched product gives the slabs' results, and hc_slab_sums adds them up, takes the few rows that fill no
+// slab along and finishes the bias.  The order of the additions is fixed.
+constexpr int64_t kSlabRows = 256;
+void tall_products(const Tensor& g, const Tensor& r, int64_t slabs, int64_t split, Tensor* left, Tensor* right, Tensor* bias) {
+  const at::Device dev = g.device();
+  const int64_t n = g.size(0), M = g.size(1), N = r.size(1);
+  int64_t s = std::max<int64_t>(slabs, 1);
+  while (s > 1 && n / s < kSlabRows) s /= 2;
+  const int64_t m = n / s, rest = n - m * s;
+  Tensor parts;
+  if (left || right) {
+    if (s > 1) {
+      parts = at::bmm(g.narrow(0, 0, m * s).view({s, m, M}).transpose(1, 2), r.narrow(0, 0, m * s).view({s, m, N}));
+    } else {
+      parts = at::mm(g.t(), r);
+      if (left && split == N) *left = parts;
+      if (!bias && left && split == N) return;
+    }
+    if (left && !left->defined()) *left = new_f32({M, split}, dev);
+    if (right) *right = new_f32({M, N - split}, dev);
+  }
+  Tensor sc;
+  if (bias) {
+    *bias = new_f32({M}, dev);
+    sc = new_scratch(lib.hc_slab_sums_scratch_bytes(M), dev);
+  }
+  const bool copied = s == 1 && split == N;      // the product is the result already
+  HC_SPAN("hc_slab_sums", dev);
+  check(lib.hc_slab_sums(fdata(parts), (int32_t)s, M, (int32_t)N, rest ? fdata(g) + m * s * M : nullptr,
+                         rest ? fdata(r) + m * s * N : nullptr, (int32_t)rest, (int32_t)split,
+                         left && !copied ? fdata(*left) : nullptr, right ? fdata(*right) : nullptr, fdata(g), n,
+                         bias ? fdata(*bias) : nullptr, data(sc), stream_of(dev)),
+        "hc_slab_sums");
+  g_launches += (bias ? 1 : 0) + 1;
+}
+
 // One RGCN layer (MyRGCNConvHistory2): relation-segmented rows by destination, their weighted sums as
 // [num_node, num_rel * feat], one product with the stacked weights, history rows over it.  Destinations
 // served from history have no edges here, so they add nothing to either gradient.
+constexpr int64_t kRgcnSlabs = 8;
 struct RgcnBackward : public torch::autograd::Node {
   SavedVariable x, weight;
   Tensor ptr2, idx2, w2, sums;
@@ -1192,7 +1233,11 @@ struct RgcnBackward : public torch::autograd::Node {
     c10::cuda::CUDAGuard guard(dev);
     const int64_t F = xt.size(1), H = w.size(2);
     const Tensor g = grads[0].contiguous(), wide = sums.view({num_node, num_rel * F});
-    if (task_should_compute_output(1)) out[1] = at::mm(wide.t(), g).view({num_rel, F, H});
+    if (task_should_compute_output(1)) {
+      Tensor gw;
+      tall_products(wide, g, kRgcnSlabs, H, &gw, nullptr, nullptr);
+      out[1] = gw.view({num_rel, F, H});
+    }
     if (task_should_compute_output(0)) {
       const Tensor go = at::mm(g, w.reshape({num_rel * F, H}).t());      // [num_node, num_rel * F] = its rows
       Block b;
@@ -1283,10 +1328,7 @@ py::tuple rgcn_layer(const Tensor& x_in, const Tensor& ptr_in, const Tensor& idx
 
 // ---------------------------------------------------------------------------
 // dense part of a SAGE layer: lin_l(aggregate) + lin_r(x[:num_node]) as one product over
-// [aggregate | root].  The weight gradient of such tall, narrow products has a very long reduction and a
-// small output, which the library runs on a few dozen blocks: the rows are cut into slabs, one batched
-// product gives the slabs' weight gradients, a batched ones-row product their bias gradients, and a sum over
-// the slabs finishes both.  The order of the additions is fixed.
+// [aggregate | root].
 // ---------------------------------------------------------------------------
 struct SageLinearBackward : public torch::autograd::Node {
   SavedVariable weight;      // [wl | wr]
@@ -1322,23 +1364,10 @@ struct SageLinearBackward : public torch::autograd::Node {
         out[4].slice(0, 0, n).copy_(g2.narrow(1, K, K));
       }
     }
-    int64_t s = slabs;
-    while (s > 1 && (n % s || n / s < 256)) s /= 2;
     const bool want_l = task_should_compute_output(1), want_r = task_should_compute_output(3),
                want_b = has_bias && task_should_compute_output(2);
-    if (s > 1) {
-      const Tensor gs = g.view({s, n / s, -1}), rs = rows.view({s, n / s, -1});
-      if (want_l || want_r) {
-        const Tensor parts = at::bmm(gs.transpose(1, 2), rs);
-        if (want_l) out[1] = parts.narrow(2, 0, K).sum(0);
-        if (want_r) out[3] = parts.narrow(2, K, K).sum(0);
-      }
-      if (want_b) out[2] = at::bmm(at::ones({s, 1, n / s}, g.options()), gs).sum(0).reshape({-1});
-    } else {
-      if (want_l) out[1] = at::mm(g.t(), rows.narrow(1, 0, K));
-      if (want_r) out[3] = at::mm(g.t(), rows.narrow(1, K, K));
-      if (want_b) out[2] = g.sum(0);
-    }
+    if (want_l || want_r || want_b)
+      tall_products(g, rows, slabs, K, want_l ? &out[1] : nullptr, want_r ? &out[3] : nullptr, want_b ? &out[2] : nullptr);
     return out;
   }
 };
@@ -1364,10 +1393,16 @@ Tensor sage_linear(const Tensor& his, const Tensor& x, int64_t num_node, const T
   }
   at::NoGradGuard no_grad;
   HC_ON(dev);
-  Tensor rows = new_f32({num_node, 2 * K}, dev);
-  rows.narrow(1, 0, K).copy_(his);
-  rows.narrow(1, K, K).copy_(x.slice(0, 0, num_node));
-  const Tensor w = at::cat({wl, wr}, 1);
+  const Tensor left = f32_rows(his), right = rows2d(x), wlc = wl.contiguous(), wrc = wr.contiguous();
+  const int64_t H = wl.size(0);
+  Tensor rows = new_f32({num_node, 2 * K}, dev), w = new_f32({H, 2 * K}, dev);
+  {
+    HC_SPAN("hc_sage_pack", dev);
+    check(lib.hc_sage_pack(fdata(left), row_stride(left, K), data(right), dtype_code(right), row_stride(right, K), num_node,
+                           (int32_t)K, fdata(rows), fdata(wlc), fdata(wrc), (int32_t)H, fdata(w), stream_of(dev)),
+          "hc_sage_pack");
+  }
+  ++g_launches;
   Tensor out = bias.defined() ? at::addmm(bias, rows, w.t()) : at::mm(rows, w.t());
   if (node) {
     node->weight = SavedVariable(w, false);
@@ -1380,6 +1415,70 @@ Tensor sage_linear(const Tensor& his, const Tensor& x, int64_t num_node, const T
     torch::autograd::set_history(out, node);
   }
   return out;
+}
+
+// ---------------------------------------------------------------------------
+// loss
+// ---------------------------------------------------------------------------
+struct NllBackward : public torch::autograd::Node {
+  SavedVariable y;
+  Tensor count;
+  int64_t classes = 0, ignore = -100;
+  bool released = false;
+
+  std::string name() const override { return "NllBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    y.reset_data();
+    count = Tensor();
+    released = true;
+  }
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+    at::NoGradGuard no_grad;
+    variable_list out(1);
+    if (!grads[0].defined() || !task_should_compute_output(0)) return out;
+    const Tensor yt = y.unpack();
+    const at::Device dev = yt.device();
+    c10::cuda::CUDAGuard guard(dev);
+    const Tensor g = grads[0].to(at::kFloat);
+    out[0] = new_f32({yt.size(0), classes}, dev);
+    HC_SPAN("hc_nll_bwd", dev);
+    check(lib.hc_nll_bwd(fdata(g), idata(yt), ignore, fdata(count), yt.size(0), (int32_t)classes, fdata(out[0]),
+                         stream_of(dev)), "hc_nll_bwd");
+    ++g_launches;
+    return out;
+  }
+};
+
+Tensor nll_loss(const Tensor& logp_in, const Tensor& y_in, int64_t ignore) {
+  const at::Device dev = require_cuda(logp_in, y_in);
+  TORCH_CHECK(logp_in.dim() == 2 && y_in.dim() == 1 && y_in.size(0) == logp_in.size(0), "nll_loss: logp [n, classes], y [n]");
+  if (logp_in.scalar_type() != at::kFloat) throw py::type_error("nll_loss: logp must be float32");
+  std::shared_ptr<NllBackward> node;
+  if (torch::autograd::compute_requires_grad(logp_in)) {
+    node = std::shared_ptr<NllBackward>(new NllBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(logp_in));
+  }
+  at::NoGradGuard no_grad;
+  HC_ON(dev);
+  const Tensor logp = rows2d(logp_in), y = i64c(y_in, "y");
+  Tensor loss = new_f32({}, dev), count = new_f32({1}, dev);
+  {
+    HC_SPAN("hc_nll_fwd", dev);
+    check(lib.hc_nll_fwd(fdata(logp), row_stride(logp, logp.size(1)), logp.size(0), (int32_t)logp.size(1), idata(y), ignore,
+                         fdata(loss), fdata(count), stream_of(dev)), "hc_nll_fwd");
+  }
+  ++g_launches;
+  if (node) {
+    node->y = SavedVariable(y, false);
+    node->count = count;
+    node->classes = logp.size(1);
+    node->ignore = ignore;
+    torch::autograd::set_history(loss, node);
+  }
+  return loss;
 }
 
 // ---------------------------------------------------------------------------
@@ -1517,5 +1616,6 @@ PYBIND11_MODULE(_native, m) {
         "perm or None, rel or None).");
   m.def("rgcn_layer", &rgcn_layer);
   m.def("sage_linear", &sage_linear);
+  m.def("nll_loss", &nll_loss);
   m.def("adam_step", &adam_step);
 }

@@ -12,7 +12,8 @@ import time
 
 import numpy as np
 import torch
-import torch.nn.functional as F
+
+import hiscache_backend as hb
 
 from .feature_store import HostFeatureStore
 from .history_cache import HistoryCache
@@ -46,7 +47,7 @@ class HistoryTableTrainer:
         self.model = get_model(config, self.table).to(self.device)
         self.optimizer = Adam(self.model.parameters(), lr=cfg_get(config, "train.optimizer.lr", 1e-3),
                               fused=True, capturable=True)
-        self.loss_fn = F.nll_loss
+        self.loss_fn = hb.nll_loss
         self.num_layer = len(self.model.convs)
         self.glb_iter = 0
         self.graphed = None
@@ -65,7 +66,6 @@ class HistoryTableTrainer:
         """One iteration on the device.  Once the table keeps its iteration counter on the device
         (enable_cuda_graph) the body contains no host-side value that changes from step to step
         and can be captured in a CUDA graph."""
-        import hiscache_backend as hb
         t = self.table
         self.optimizer.zero_grad(set_to_none=True)
         nn = [int(v) for v in batch.num_node_in_layer]
@@ -128,7 +128,7 @@ class HistoryTrainer:
         self.optimizer = Adam(self.model.parameters(), lr=cfg_get(config, "train.optimizer.lr", 1e-3),
                               fused=True, capturable=True)
         self.scheduler = torch.optim.lr_scheduler.LambdaLR(self.optimizer, lambda _: 1.0)
-        self.loss_fn = F.nll_loss
+        self.loss_fn = hb.nll_loss
         self.type = config.train.type.lower()
         self.load_type = config.dl.type.lower()
         self.glb_iter = 0

@@ -11,7 +11,6 @@ import time
 
 import torch
 import torch.distributed as dist
-import torch.nn.functional as F
 
 import hiscache_backend as hb
 
@@ -179,7 +178,7 @@ class MultiGpuHistoryTrainer:
         # issued eagerly between them (hiscache/graphed.py); no collective is ever captured.
         self.graphed = None
         self.scheduler = torch.optim.lr_scheduler.LambdaLR(self.optimizer, lambda _: 1.0)
-        self.loss_fn = F.nll_loss
+        self.loss_fn = hb.nll_loss
         self.glb_iter = 0
         # gradients travel in one flat bucket: autograd leaves fresh per-parameter gradients
         # (no accumulation kernels), one concatenation packs them, one all-reduce averages them

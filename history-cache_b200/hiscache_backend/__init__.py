@@ -719,8 +719,15 @@ def rgcn_layer(x, ptr, idx, edge_type, num_node, weight, *, used_src=None, histo
 
 
 # ---------------------------------------------------------------------------
-# dense part of a SAGE layer, optimiser
+# dense part of a SAGE layer, loss, optimiser
 # ---------------------------------------------------------------------------
+def nll_loss(logp, y, ignore_index=-100):
+    """torch.nn.functional.nll_loss (mean over the labelled rows), one kernel per direction."""
+    if logp.dim() == 2 and y.dim() == 1 and logp.dtype == torch.float32 and y.dtype == torch.int64:
+        return _native.nll_loss(logp, y, ignore_index)
+    return torch.nn.functional.nll_loss(logp, y, ignore_index=ignore_index)
+
+
 sage_linear = _native.sage_linear       # (his, x, num_node, w_l, bias, w_r, slabs)
 adam_step = _native.adam_step           # (params, grads, exp_avgs, exp_avg_sqs, steps, lr, beta1, beta2, eps)
 

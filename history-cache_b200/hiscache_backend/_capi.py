@@ -130,6 +130,11 @@ _SIGS = {
     "hc_rgcn_rows": (C.c_int, [vp, vp, vp, i64, i64, i32, vp, vp, vp, vp, vp, vp, vp, vp]),
     "hc_override_rows": (C.c_int, [vp, i64, vp, i32, i64, i32, i32, vp, vp]),
     "hc_aggr_bwd_rooted": (C.c_int, [C.POINTER(AggrArgs), vp, i64, vp, i64, vp, i32, vp, vp, vp, i32, vp]),
+    "hc_sage_pack": (C.c_int, [vp, i64, vp, i32, i64, i64, i32, vp, vp, vp, i32, vp, vp]),
+    "hc_slab_sums_scratch_bytes": (i64, [i64]),
+    "hc_slab_sums": (C.c_int, [vp, i32, i64, i32, vp, vp, i32, i32, vp, vp, vp, i64, vp, vp, vp]),
+    "hc_nll_fwd": (C.c_int, [vp, i64, i64, i32, vp, i64, vp, vp, vp]),
+    "hc_nll_bwd": (C.c_int, [vp, vp, i64, vp, i64, i32, vp, vp]),
     "hc_adam_step": (C.c_int, [vp, vp, vp, vp, vp, vp, i32, C.c_double, C.c_double, C.c_double, C.c_double, vp]),
     "hc_mix64": (C.c_uint64, [C.c_uint64]),
     "hc_bucket_scratch_bytes": (i64, [i64, i32]),

@@ -793,6 +793,33 @@ int hc_sample_batch(const int64_t* gptr, const int64_t* gidx, const int64_t* see
                     int64_t* y, const hc_fixed_batch* b, void* scratch, void* stream);
 
 /*
+ * Around the dense products of a layer.
+ * hc_sage_pack: rows [n, 2*feat] = [his | x[:n]] in fp32 (x fp32 or fp16) and
+ * w [hidden, 2*feat] = [wl | wr].
+ * hc_slab_sums: out[i, j] = sum_s parts[s, i, j] + sum_k a[k, i] * b[k, j] over
+ * `rest` rows k of a [rest, rows] and b [rest, cols]; columns [0, split) go to
+ * left [rows, split], the others to right [rows, cols - split] (either may be
+ * NULL).  bias (NULL = none) [rows] = column sums of g [n, rows].  Fixed order
+ * of additions.  scratch (for bias): >= hc_slab_sums_scratch_bytes(rows), 4-byte aligned.
+ */
+int hc_sage_pack(const float* his, int64_t his_stride, const void* x, int32_t x_dtype,
+                 int64_t x_stride, int64_t n, int32_t feat, float* rows, const float* wl,
+                 const float* wr, int32_t hidden, float* w, void* stream);
+int64_t hc_slab_sums_scratch_bytes(int64_t rows);
+int hc_slab_sums(const float* parts, int32_t slabs, int64_t rows, int32_t cols, const float* a,
+                 const float* b, int32_t rest, int32_t split, float* left, float* right,
+                 const float* g, int64_t n, float* bias, void* scratch, void* stream);
+/*
+ * Negative log likelihood, mean over the rows with y[i] != ignore: loss [1],
+ * count [1] = number of such rows (NaN loss when there are none, or when a label is outside
+ * [0, classes)).  Backward: grad_logp [n, classes] dense, written whole.
+ */
+int hc_nll_fwd(const float* logp, int64_t stride, int64_t n, int32_t classes, const int64_t* y,
+               int64_t ignore, float* loss, float* count, void* stream);
+int hc_nll_bwd(const float* grad, const int64_t* y, int64_t ignore, const float* count, int64_t n,
+               int32_t classes, float* grad_logp, void* stream);
+
+/*
  * One Adam step over n fp32 tensors (host arrays of device pointers): steps[k]
  * (float, one per tensor) is advanced, then with t = steps[k]
  *   m = beta1 m + (1 - beta1) g;  v = beta2 v + (1 - beta2) g^2

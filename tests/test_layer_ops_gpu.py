@@ -142,3 +142,38 @@ def test_adam_step_matches_torch(backend, sizes):
             assert torch.allclose(so["state"][k][name], st["state"][k][name], rtol=1e-5, atol=1e-7)
     ours.load_state_dict(st)
     assert isinstance(ours, torch.optim.Adam)
+
+
+@pytest.mark.parametrize("n,hidden,feat", [(1, 3, 5), (255, 47, 100), (512, 64, 33), (2051, 256, 128), (5000, 1100, 8)])
+def test_weight_and_bias_gradients_from_slabs(backend, n, hidden, feat):
+    """Row counts that are no multiple of the slabs, outputs wider than a block, one slab."""
+    x, his = (torch.randn(n + 3, feat, device="cuda"), torch.randn(n, feat, device="cuda"))
+    wl, wr = (torch.randn(hidden, feat, device="cuda", requires_grad=True) for _ in range(2))
+    b = torch.randn(hidden, device="cuda", requires_grad=True)
+    g = torch.randn(n, hidden, device="cuda")
+    for slabs in (1, 8):
+        out = backend.sage_linear(his, x, n, wl, b, wr, slabs)
+        want = his.double() @ wl.double().t() + x[:n].double() @ wr.double().t() + b.double()
+        assert (out - want).abs().max() <= 1e-5 * (1 + want.abs().max())
+        got = torch.autograd.grad(out, (wl, wr, b), g)
+        for a, w in zip(got, (g.double().t() @ his.double(), g.double().t() @ x[:n].double(), g.double().sum(0))):
+            assert (a - w).abs().max() <= 1e-5 * (1 + w.abs().max())
+        only = torch.autograd.grad(backend.sage_linear(his, x, n, wl.detach(), b, wr, slabs), (b, wr), g)
+        assert torch.equal(only[0], got[2]) and torch.equal(only[1], got[1])
+
+
+@pytest.mark.parametrize("n,classes", [(1, 2), (1000, 172), (1025, 47), (9000, 153)])
+@pytest.mark.parametrize("ignored", [0.0, 0.3, 1.0])
+def test_nll_loss(backend, n, classes, ignored):
+    logp = torch.randn(n, classes + 1, device="cuda").log_softmax(-1)[:, :classes].requires_grad_()
+    y = torch.randint(0, classes, (n,), device="cuda")
+    y[torch.rand(n, device="cuda") < ignored] = -100
+    loss = backend.nll_loss(logp, y)
+    want = torch.nn.functional.nll_loss(logp.double(), y)
+    if bool((y == -100).all()):
+        assert torch.isnan(loss) and torch.isnan(want)
+        return
+    assert loss.shape == want.shape and abs(float(loss) - float(want)) <= 1e-6 * abs(float(want))
+    got, = torch.autograd.grad(loss * 3, logp)
+    ref, = torch.autograd.grad(want * 3, logp)
+    assert torch.allclose(got, ref.float(), rtol=1e-6, atol=0)
