@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(256) load_rows_kernel(const LoadArgs a) {
 constexpr int kBulkWarps = 4;      // warps per block
 constexpr int kBulkTile = 32;      // rows per tile = one row per lane
 constexpr int kBulkSpin = 1 << 22; // bound of every wait loop
-constexpr int kStageBlocks = 16;   // grid of a staging call (hc_stage_host_rows), see stage_rows_kernel
+constexpr int kStageBlocks = 24;   // grid of a staging call (hc_stage_host_rows), see stage_rows_kernel
 
 __global__ void __launch_bounds__(kBulkWarps * 32)
     load_rows_bulk_kernel(const LoadArgs a, const int row_bytes, const int64_t tiles) {
@@ -382,11 +382,11 @@ using namespace hc;
 // shared memory, no polling.  A batch is seen as a list of 16-byte units (unit u belongs to row
 // u / units_per_row); consecutive lanes take consecutive units, every thread issues kStageUnroll
 // independent 16-byte loads before it stores the first, and a warp that waits for the host link
-// is simply stalled on its loads.  The grid is deliberately small: measured inside a training
-// step of 0.8 ms, 16 blocks (about 0.6 ms alone for 20 K rows of 256 B, 9 GB/s) leave the step's
-// own kernels undisturbed, while 64 or 148 blocks (0.43 ms alone) slow them down by as much as
-// the call takes; the more read requests to host memory are outstanding, the more the step's
-// own memory traffic waits behind them.
+// is simply stalled on its loads.  The grid is deliberately small: the more
+// read requests to host memory are outstanding, the more the step's own memory traffic waits behind
+// them, and the call only has to finish within the step.  Measured beside a step whose own kernels
+// take 0.49 ms (us a step; table of 0.13 / 1 / 4 / 12.8 GB): 16 blocks 516 / 520 / 635 / 714,
+// 24 blocks 502 / 505 / 588 / 668, 32 blocks 502 / 506 / 615 / 720.
 // ---------------------------------------------------------------------------
 namespace hc {
 
