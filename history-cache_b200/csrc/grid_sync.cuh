@@ -15,10 +15,10 @@ struct GridSync {
   // true: every block has arrived, and what it wrote before is visible
   __device__ __forceinline__ bool wait() {
     __shared__ bool ok;
-    __threadfence();
     __syncthreads();
     ++round;
     if (threadIdx.x == 0) {
+      __threadfence();      // cumulative: covers what the barrier above ordered before it
       const unsigned want = round * gridDim.x;
       atomicAdd(word, 1u);
       int spins = 0;

@@ -13,6 +13,8 @@
 // loads are all in flight at once.
 // Column statistics are reproducible: every block writes its partial sums, the block that
 // finishes last adds them in block order in double precision.
+#include <stddef.h>
+
 #include "common.cuh"
 
 namespace hc {
@@ -91,6 +93,7 @@ struct NormArgs {
   float* running_mean; float* running_var; float momentum; float eps;
   float drop_p; uint64_t seed; int64_t* counter; int64_t* saved_step;   // state[0], state[1]
   float* save_mean; float* save_rstd; float* save_count;
+  int64_t* tracked;
   int relu;
   // scratch
   float* partial;          // [blocks][2][feat]  (+ [blocks] counts behind)
@@ -217,6 +220,7 @@ __global__ void __launch_bounds__(kStatsBlock) norm_stats_kernel(const NormArgs 
   if (threadIdx.x == 0) {
     a.save_count[0] = (float)n_valid;
     *a.ticket = 0;
+    if (a.tracked) a.tracked[0] += 1;
     if (a.counter) {      // this call's dropout stream; the next call gets the next one
       a.saved_step[0] = a.counter[0];
       a.counter[0] += 1;
@@ -384,7 +388,8 @@ __global__ void __launch_bounds__(kNormBlock)
 
 static int fill(const hc_norm_args* p, void* scratch, NormArgs* a, NormBwd* bw) {
   HC_REQUIRE(p != nullptr, HC_ERR_NULL);
-  HC_REQUIRE(p->struct_size == sizeof(hc_norm_args), HC_ERR_STRUCT);
+  constexpr uint32_t kWithoutTracked = offsetof(hc_norm_args, batches_tracked);
+  HC_REQUIRE(p->struct_size == sizeof(hc_norm_args) || p->struct_size == kWithoutTracked, HC_ERR_STRUCT);
   HC_REQUIRE(p->n >= 0 && p->feat > 0, HC_ERR_SIZE);
   HC_REQUIRE(p->feat % 4 == 0 && p->feat <= 1024, HC_ERR_UNSUPPORTED);
   HC_REQUIRE(p->drop_p >= 0.f && p->drop_p < 1.f && p->eps > 0.f, HC_ERR_SIZE);
@@ -401,6 +406,7 @@ static int fill(const hc_norm_args* p, void* scratch, NormArgs* a, NormBwd* bw) 
   a->counter = p->drop_p > 0.f ? p->state : nullptr;
   a->saved_step = p->state + 1;
   a->ticket = reinterpret_cast<unsigned int*>(p->state + 2);
+  a->tracked = p->struct_size == sizeof(hc_norm_args) ? p->batches_tracked : nullptr;
   a->save_mean = p->save_mean; a->save_rstd = p->save_rstd; a->save_count = p->save_count;
   a->relu = p->relu ? 1 : 0;
   float* f = reinterpret_cast<float*>(scratch);

@@ -130,6 +130,7 @@ struct RowsArgs {
   int32_t* count;          // [num_rel + 1] edges per relation (0 is not counted), pruned ones last
   unsigned* word;          // barrier
   int* block_edges;        // [blocks]
+  int* block_rel;          // [blocks][kRowsMaxRel] edges per relation
 };
 
 __global__ void __launch_bounds__(kRowsThreads) rgcn_rows_kernel(const RowsArgs a) {
@@ -177,7 +178,7 @@ __global__ void __launch_bounds__(kRowsThreads) rgcn_rows_kernel(const RowsArgs 
   int total;
   block_exclusive<kRowsThreads>(mine, &total);
   if (threadIdx.x == 0) a.block_edges[blockIdx.x] = total;
-  if (threadIdx.x > 0 && threadIdx.x < R && hist[threadIdx.x]) atomicAdd(a.count + threadIdx.x, hist[threadIdx.x]);
+  if (threadIdx.x < R) a.block_rel[blockIdx.x * kRowsMaxRel + threadIdx.x] = hist[threadIdx.x];
   if (!grid.wait()) return;
 
   int all, first;
@@ -185,6 +186,15 @@ __global__ void __launch_bounds__(kRowsThreads) rgcn_rows_kernel(const RowsArgs 
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.ptr2[a.num_node * R] = all;
     a.count[R] = (int32_t)(a.n_edges - all);
+    a.count[0] = 0;
+  }
+  // relation r's edges, by a warp of the last block
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x / 32 > 0 && threadIdx.x / 32 < R) {
+    const int r = threadIdx.x / 32;
+    int n = 0;
+    for (int b = threadIdx.x & 31; b < (int)gridDim.x; b += 32) n += __ldcg(a.block_rel + b * kRowsMaxRel + r);
+    n = __reduce_add_sync(kFull, n);
+    if ((threadIdx.x & 31) == 0) a.count[r] = n;
   }
   if (threadIdx.x == 0) kept_before = first;
   for (int64_t t0 = d0; t0 < d1; t0 += kGroups) {
@@ -251,7 +261,9 @@ __global__ void __launch_bounds__(256)
 
 using namespace hc;
 
-extern "C" int64_t hc_rgcn_rows_scratch_bytes(void) { return 16 + kRowsBlocks * (int64_t)sizeof(int); }
+extern "C" int64_t hc_rgcn_rows_scratch_bytes(void) {
+  return 16 + kRowsBlocks * (1 + kRowsMaxRel) * (int64_t)sizeof(int);
+}
 
 extern "C" int hc_rgcn_rows(const int64_t* ptr, const int64_t* idx, const int64_t* etype, int64_t num_node,
                             int64_t n_edges, int32_t num_rel, const uint8_t* used_src, const int64_t* hmap,
@@ -261,14 +273,15 @@ extern "C" int hc_rgcn_rows(const int64_t* ptr, const int64_t* idx, const int64_
   HC_REQUIRE(n_edges < 0x7fffffffLL && num_node < 0x7fffffffLL, HC_ERR_SIZE);
   HC_REQUIRE(ptr2 && count && scratch, HC_ERR_NULL);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  HC_CUDA(cudaMemsetAsync(count, 0, (num_rel + 1) * sizeof(int32_t), st));
   if (n_edges == 0 || num_node == 0) {
+    HC_CUDA(cudaMemsetAsync(count, 0, (num_rel + 1) * sizeof(int32_t), st));
     HC_CUDA(cudaMemsetAsync(ptr2, 0, (size_t)(num_rel * num_node + 1) * sizeof(int64_t), st));
     return 0;
   }
   HC_REQUIRE(ptr && idx && etype && idx2 && w2, HC_ERR_NULL);
   RowsArgs a{ptr, idx, etype, num_node, n_edges, num_rel, used_src, hmap, ptr2, idx2, w2, count,
-             reinterpret_cast<unsigned*>(scratch), reinterpret_cast<int*>(scratch) + 4};
+             reinterpret_cast<unsigned*>(scratch), reinterpret_cast<int*>(scratch) + 4,
+             reinterpret_cast<int*>(scratch) + 4 + kRowsBlocks};
   const int64_t blocks = ceil_div(num_node, 16);
   return launch_together(rgcn_rows_kernel, (unsigned)(blocks < kRowsBlocks ? blocks : kRowsBlocks), kRowsThreads, 0, a.word,
                          st, a);

@@ -612,8 +612,8 @@ struct NormActBackward : public torch::autograd::Node {
 
 Tensor norm_act(const Tensor& x_in, const OptTensor& weight, const OptTensor& bias, const Tensor& state,
                 const OptTensor& valid_in, const OptTensor& running_mean, const OptTensor& running_var,
-                double momentum, double eps, double p, bool relu, uint64_t seed) {
-  const Tensor w = some(weight), bi = some(bias), rm = some(running_mean), rv = some(running_var);
+                double momentum, double eps, double p, bool relu, uint64_t seed, const OptTensor& tracked_in) {
+  const Tensor w = some(weight), bi = some(bias), rm = some(running_mean), rv = some(running_var), tracked = some(tracked_in);
   Tensor valid = some(valid_in);
   const at::Device dev = require_cuda(x_in, w, bi, valid, rm, rv, state);
   std::shared_ptr<NormActBackward> node;
@@ -632,7 +632,17 @@ Tensor norm_act(const Tensor& x_in, const OptTensor& weight, const OptTensor& bi
   const int64_t F = x.size(1);
   Tensor y = new_f32({x.size(0), F}, dev), save = new_f32({2 * F + 4}, dev);
   const NormCfg cfg{momentum, eps, p, relu, seed};
-  const hc_norm_args a = norm_args(x, valid, w, bi, rm, rv, cfg, state, save);
+  hc_norm_args a = norm_args(x, valid, w, bi, rm, rv, cfg, state, save);
+  if (tracked.defined()) {
+    TORCH_CHECK(tracked.device() == dev && tracked.scalar_type() == at::kLong && tracked.numel() == 1,
+                "norm_act: num_batches_tracked must be an int64 CUDA scalar");
+    if (a.n) {
+      a.batches_tracked = data<int64_t>(tracked);
+      torch::autograd::impl::bump_version(tracked);
+    } else {
+      tracked.add_(1);
+    }
+  }
   Tensor sc = new_scratch(lib.hc_norm_scratch_bytes((int32_t)F), dev);
   {
     HC_SPAN("hc_norm_act_fwd", dev);
@@ -1182,8 +1192,10 @@ void tall_products(const Tensor& g, const Tensor& r, int64_t slabs, int64_t spli
       parts = at::bmm(g.narrow(0, 0, m * s).view({s, m, M}).transpose(1, 2), r.narrow(0, 0, m * s).view({s, m, N}));
     } else {
       parts = at::mm(g.t(), r);
-      if (left && split == N) *left = parts;
-      if (!bias && left && split == N) return;
+    }
+    if (s == 1 && left && split == N) {      // the product is the result already
+      *left = parts;
+      if (!bias) return;
     }
     if (left && !left->defined()) *left = new_f32({M, split}, dev);
     if (right) *right = new_f32({M, N - split}, dev);
@@ -1193,7 +1205,7 @@ void tall_products(const Tensor& g, const Tensor& r, int64_t slabs, int64_t spli
     *bias = new_f32({M}, dev);
     sc = new_scratch(lib.hc_slab_sums_scratch_bytes(M), dev);
   }
-  const bool copied = s == 1 && split == N;      // the product is the result already
+  const bool copied = s == 1 && split == N;
   HC_SPAN("hc_slab_sums", dev);
   check(lib.hc_slab_sums(fdata(parts), (int32_t)s, M, (int32_t)N, rest ? fdata(g) + m * s * M : nullptr,
                          rest ? fdata(r) + m * s * N : nullptr, (int32_t)rest, (int32_t)split,
@@ -1206,7 +1218,7 @@ void tall_products(const Tensor& g, const Tensor& r, int64_t slabs, int64_t spli
 // One RGCN layer (MyRGCNConvHistory2): relation-segmented rows by destination, their weighted sums as
 // [num_node, num_rel * feat], one product with the stacked weights, history rows over it.  Destinations
 // served from history have no edges here, so they add nothing to either gradient.
-constexpr int64_t kRgcnSlabs = 8;
+constexpr int64_t kRgcnSlabs = 16;
 struct RgcnBackward : public torch::autograd::Node {
   SavedVariable x, weight;
   Tensor ptr2, idx2, w2, sums;
@@ -1395,15 +1407,21 @@ Tensor sage_linear(const Tensor& his, const Tensor& x, int64_t num_node, const T
   HC_ON(dev);
   const Tensor left = f32_rows(his), right = rows2d(x), wlc = wl.contiguous(), wrc = wr.contiguous();
   const int64_t H = wl.size(0);
-  Tensor rows = new_f32({num_node, 2 * K}, dev), w = new_f32({H, 2 * K}, dev);
+  Tensor rows = new_f32({num_node, 2 * K}, dev), w = new_f32({H, 2 * K}, dev), out = new_f32({num_node, H}, dev);
+  const Tensor bc = bias.defined() ? bias.contiguous() : bias;
   {
     HC_SPAN("hc_sage_pack", dev);
     check(lib.hc_sage_pack(fdata(left), row_stride(left, K), data(right), dtype_code(right), row_stride(right, K), num_node,
-                           (int32_t)K, fdata(rows), fdata(wlc), fdata(wrc), (int32_t)H, fdata(w), stream_of(dev)),
+                           (int32_t)K, fdata(rows), fdata(wlc), fdata(wrc), (int32_t)H, fdata(w), fdata(bc),
+                           bias.defined() ? fdata(out) : nullptr, stream_of(dev)),
           "hc_sage_pack");
   }
   ++g_launches;
-  Tensor out = bias.defined() ? at::addmm(bias, rows, w.t()) : at::mm(rows, w.t());
+  if (bias.defined()) {
+    out.addmm_(rows, w.t());
+  } else {
+    at::mm_out(out, rows, w.t());
+  }
   if (node) {
     node->weight = SavedVariable(w, false);
     node->rows = rows;
@@ -1484,10 +1502,28 @@ Tensor nll_loss(const Tensor& logp_in, const Tensor& y_in, int64_t ignore) {
 // ---------------------------------------------------------------------------
 // optimiser
 // ---------------------------------------------------------------------------
-void adam_step(const std::vector<Tensor>& params, const std::vector<Tensor>& grads, const std::vector<Tensor>& avgs,
+// whether adam_step takes these tensors (device-side step counts, fp32, dense)
+bool adam_fits(const std::vector<Tensor>& params, const std::vector<Tensor>& grads, const std::vector<Tensor>& avgs,
+               const std::vector<Tensor>& avg_sqs, const std::vector<Tensor>& steps) {
+  const size_t n = params.size();
+  if (grads.size() != n || avgs.size() != n || avg_sqs.size() != n || steps.size() != n) return false;
+  for (size_t k = 0; k < n; ++k) {
+    const at::Device dev = params[0].device();
+    for (const Tensor* t : {&params[k], &grads[k], &avgs[k], &avg_sqs[k], &steps[k]})
+      if (!t->is_cuda() || t->device() != dev || t->scalar_type() != at::kFloat || t->layout() != at::kStrided) return false;
+    for (const Tensor* t : {&params[k], &avgs[k], &avg_sqs[k]})
+      if (!t->is_contiguous() || t->numel() != params[k].numel()) return false;
+    if (params[k].numel() == 0 || grads[k].numel() != params[k].numel() || steps[k].numel() != 1) return false;
+  }
+  return true;
+}
+
+// false: not a case for the kernel, nothing done
+bool adam_step(const std::vector<Tensor>& params, const std::vector<Tensor>& grads, const std::vector<Tensor>& avgs,
                const std::vector<Tensor>& avg_sqs, const std::vector<Tensor>& steps, double lr, double beta1, double beta2,
                double eps) {
-  if (params.empty()) return;
+  if (params.empty()) return true;
+  if (!adam_fits(params, grads, avgs, avg_sqs, steps)) return false;
   at::NoGradGuard no_grad;
   const at::Device dev = params[0].device();
   HC_ON(dev);
@@ -1512,6 +1548,7 @@ void adam_step(const std::vector<Tensor>& params, const std::vector<Tensor>& gra
   g_launches += 2;
   for (const auto* list : {&params, &avgs, &avg_sqs, &steps})
     for (const Tensor& x : *list) torch::autograd::impl::bump_version(x);
+  return true;
 }
 }  // namespace
 
@@ -1618,4 +1655,5 @@ PYBIND11_MODULE(_native, m) {
   m.def("sage_linear", &sage_linear);
   m.def("nll_loss", &nll_loss);
   m.def("adam_step", &adam_step);
+  m.def("adam_fits", &adam_fits);
 }

@@ -17,12 +17,22 @@ class Adam(torch.optim.Adam):
     @torch.no_grad()
     def step(self, closure=None):
         calls = self._native_calls() if closure is None else None
-        if calls is None:
+        # several groups: all of them or none, so that torch's step never follows half of ours
+        if calls is None or (len(calls) > 1 and not all(hb.adam_fits(*c[:5]) for c in calls)):
             return super().step(closure)
         for call in calls:
-            hb.adam_step(*call)
+            if not hb.adam_step(*call):
+                return super().step()
+
+    def zero_grad(self, set_to_none=True):
+        if not set_to_none:
+            return super().zero_grad(False)
+        for g in self.param_groups:
+            for p in g["params"]:
+                p.grad = None
 
     def _native_calls(self):
+        """Arguments of hb.adam_step per parameter group, or None when torch has to do the step."""
         if getattr(self, "grad_scale", None) is not None or getattr(self, "found_inf", None) is not None:
             return None
         calls = []
@@ -32,25 +42,17 @@ class Adam(torch.optim.Adam):
                     or not (g["capturable"] or g["fused"])
                     or any(isinstance(v, torch.Tensor) for v in (lr, b1, b2, eps))):
                 return None
-            params, grads, states = [], [], []
-            for p in g["params"]:
-                if p.grad is None:
+            params = [p for p in g["params"] if p.grad is not None]
+            states = [self.state[p] for p in params]
+            for p, s in zip(params, states):
+                if s:
                     continue
-                if not (p.is_cuda and p.dtype == torch.float32 and p.is_contiguous() and p.numel() > 0
-                        and p.grad.dtype == torch.float32 and p.grad.layout == torch.strided
-                        and (not params or p.device == params[0].device)):
+                if not p.is_cuda or p.dtype != torch.float32:
                     return None
-                params.append(p)
-                grads.append(p.grad)
-                s = self.state[p]
-                if not s:
-                    s["step"] = torch.zeros((), dtype=torch.float32, device=p.device)
-                    s["exp_avg"] = torch.zeros_like(p)
-                    s["exp_avg_sq"] = torch.zeros_like(p)
-                elif not (s["step"].is_cuda and s["step"].dtype == torch.float32
-                          and s["exp_avg"].is_contiguous() and s["exp_avg_sq"].is_contiguous()):
-                    return None
-                states.append(s)
-            calls.append((params, grads, [s["exp_avg"] for s in states], [s["exp_avg_sq"] for s in states],
-                          [s["step"] for s in states], lr, b1, b2, eps))
+                s["step"] = torch.zeros((), dtype=torch.float32, device=p.device)
+                s["exp_avg"] = torch.zeros_like(p)
+                s["exp_avg_sq"] = torch.zeros_like(p)
+            tensors = (params, [p.grad for p in params], [s["exp_avg"] for s in states],
+                       [s["exp_avg_sq"] for s in states], [s["step"] for s in states])
+            calls.append((*tensors, lr, b1, b2, eps))
         return calls

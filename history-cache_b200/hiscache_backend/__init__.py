@@ -282,12 +282,13 @@ def aggr_forward_history_edge_value(input, ptr, idx, edge_value, history_map, hi
 # batch norm + ReLU + dropout in one forward pair / one backward pair
 # ---------------------------------------------------------------------------
 def norm_act(x, weight, bias, state, *, valid=None, running_mean=None, running_var=None, momentum=0.1,
-             eps=1e-5, p=0.0, relu=True, seed=0):
+             eps=1e-5, p=0.0, relu=True, seed=0, num_batches_tracked=None):
     """y = dropout(relu(batch_norm(x))) with batch statistics (training mode), as two kernels
     forward and two backward (csrc/norm_act.cu).  `state`: int64[4] CUDA tensor, zero-initialised
-    once and private to the calling layer (dropout step counter).  `valid`: optional row mask."""
+    once and private to the calling layer (dropout step counter).  `valid`: optional row mask.
+    `num_batches_tracked`: BatchNorm1d's counter, advanced by the same kernel."""
     return _native.norm_act(x, weight, bias, state, valid, running_mean, running_var, momentum, eps, p, relu,
-                            seed & 0xFFFFFFFFFFFFFFFF)
+                            seed & 0xFFFFFFFFFFFFFFFF, num_batches_tracked)
 
 
 def norm_act_supported(x) -> bool:
@@ -729,7 +730,8 @@ def nll_loss(logp, y, ignore_index=-100):
 
 
 sage_linear = _native.sage_linear       # (his, x, num_node, w_l, bias, w_r, slabs)
-adam_step = _native.adam_step           # (params, grads, exp_avgs, exp_avg_sqs, steps, lr, beta1, beta2, eps)
+adam_step = _native.adam_step           # (params, grads, exp_avgs, exp_avg_sqs, steps, lr, beta1, beta2, eps) -> whether done
+adam_fits = _native.adam_fits           # (params, grads, exp_avgs, exp_avg_sqs, steps) -> bool
 
 # ---------------------------------------------------------------------------
 # peer copies (kept for API compatibility; the multi-GPU path uses NCCL)

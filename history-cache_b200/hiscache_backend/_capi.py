@@ -68,6 +68,7 @@ class NormArgs(C.Structure):
         ("weight", vp), ("bias", vp), ("running_mean", vp), ("running_var", vp),
         ("momentum", f32), ("eps", f32), ("drop_p", f32), ("relu", i32), ("seed", C.c_uint64),
         ("state", vp), ("save_mean", vp), ("save_rstd", vp), ("save_count", vp),
+        ("batches_tracked", vp),
     ]
 
 
@@ -130,7 +131,7 @@ _SIGS = {
     "hc_rgcn_rows": (C.c_int, [vp, vp, vp, i64, i64, i32, vp, vp, vp, vp, vp, vp, vp, vp]),
     "hc_override_rows": (C.c_int, [vp, i64, vp, i32, i64, i32, i32, vp, vp]),
     "hc_aggr_bwd_rooted": (C.c_int, [C.POINTER(AggrArgs), vp, i64, vp, i64, vp, i32, vp, vp, vp, i32, vp]),
-    "hc_sage_pack": (C.c_int, [vp, i64, vp, i32, i64, i64, i32, vp, vp, vp, i32, vp, vp]),
+    "hc_sage_pack": (C.c_int, [vp, i64, vp, i32, i64, i64, i32, vp, vp, vp, i32, vp, vp, vp, vp]),
     "hc_slab_sums_scratch_bytes": (i64, [i64]),
     "hc_slab_sums": (C.c_int, [vp, i32, i64, i32, vp, vp, i32, i32, vp, vp, vp, i64, vp, vp, vp]),
     "hc_nll_fwd": (C.c_int, [vp, i64, i64, i32, vp, i64, vp, vp, vp]),

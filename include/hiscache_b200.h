@@ -544,7 +544,7 @@ int hc_load_rows_staged(const void* host_table, int32_t host_dtype,
  * The call is meant to run beside a training step and therefore uses a small
  * grid (the more host reads are outstanding, the more the step's own kernels
  * are slowed down); max_blocks > 0 overrides the default number of thread
- * blocks (16).
+ * blocks (24).
  */
 int hc_stage_host_rows(const void* host_table, int32_t host_dtype,
                        int64_t host_rows, int64_t host_stride, int32_t feat,
@@ -795,7 +795,7 @@ int hc_sample_batch(const int64_t* gptr, const int64_t* gidx, const int64_t* see
 /*
  * Around the dense products of a layer.
  * hc_sage_pack: rows [n, 2*feat] = [his | x[:n]] in fp32 (x fp32 or fp16) and
- * w [hidden, 2*feat] = [wl | wr].
+ * w [hidden, 2*feat] = [wl | wr]; out (NULL = none) [n, hidden] = bias in every row.
  * hc_slab_sums: out[i, j] = sum_s parts[s, i, j] + sum_k a[k, i] * b[k, j] over
  * `rest` rows k of a [rest, rows] and b [rest, cols]; columns [0, split) go to
  * left [rows, split], the others to right [rows, cols - split] (either may be
@@ -804,7 +804,8 @@ int hc_sample_batch(const int64_t* gptr, const int64_t* gidx, const int64_t* see
  */
 int hc_sage_pack(const float* his, int64_t his_stride, const void* x, int32_t x_dtype,
                  int64_t x_stride, int64_t n, int32_t feat, float* rows, const float* wl,
-                 const float* wr, int32_t hidden, float* w, void* stream);
+                 const float* wr, int32_t hidden, float* w, const float* bias, float* out,
+                 void* stream);
 int64_t hc_slab_sums_scratch_bytes(int64_t rows);
 int hc_slab_sums(const float* parts, int32_t slabs, int64_t rows, int32_t cols, const float* a,
                  const float* b, int32_t rest, int32_t split, float* left, float* right,
@@ -873,6 +874,7 @@ typedef struct hc_norm_args {
   float* save_mean;
   float* save_rstd;
   float* save_count;
+  int64_t* batches_tracked; /* advanced by one in the forward pass, or NULL (a struct_size without it = NULL) */
 } hc_norm_args;
 int64_t hc_norm_scratch_bytes(int32_t feat);
 int hc_norm_act_fwd(const hc_norm_args* a, float* y, void* scratch, void* stream);

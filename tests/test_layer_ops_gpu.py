@@ -144,22 +144,29 @@ def test_adam_step_matches_torch(backend, sizes):
     assert isinstance(ours, torch.optim.Adam)
 
 
-@pytest.mark.parametrize("n,hidden,feat", [(1, 3, 5), (255, 47, 100), (512, 64, 33), (2051, 256, 128), (5000, 1100, 8)])
-def test_weight_and_bias_gradients_from_slabs(backend, n, hidden, feat):
+@pytest.mark.parametrize("n,hidden,feat", [
+    (1, 3, 5), (255, 47, 100), (512, 64, 33), (2051, 256, 128), (5000, 1100, 8), (9473, 47, 50)])
+def test_dense_part_of_a_layer(backend, n, hidden, feat):
     """Row counts that are no multiple of the slabs, outputs wider than a block, one slab."""
-    x, his = (torch.randn(n + 3, feat, device="cuda"), torch.randn(n, feat, device="cuda"))
+    x = torch.randn(n + 3, feat, device="cuda", requires_grad=True)
+    his = torch.randn(n, feat, device="cuda", requires_grad=True)
     wl, wr = (torch.randn(hidden, feat, device="cuda", requires_grad=True) for _ in range(2))
     b = torch.randn(hidden, device="cuda", requires_grad=True)
     g = torch.randn(n, hidden, device="cuda")
-    for slabs in (1, 8):
-        out = backend.sage_linear(his, x, n, wl, b, wr, slabs)
-        want = his.double() @ wl.double().t() + x[:n].double() @ wr.double().t() + b.double()
-        assert (out - want).abs().max() <= 1e-5 * (1 + want.abs().max())
-        got = torch.autograd.grad(out, (wl, wr, b), g)
-        for a, w in zip(got, (g.double().t() @ his.double(), g.double().t() @ x[:n].double(), g.double().sum(0))):
-            assert (a - w).abs().max() <= 1e-5 * (1 + w.abs().max())
-        only = torch.autograd.grad(backend.sage_linear(his, x, n, wl.detach(), b, wr, slabs), (b, wr), g)
-        assert torch.equal(only[0], got[2]) and torch.equal(only[1], got[1])
+    d = [t.detach().double() for t in (his, x, wl, wr, b, g)]
+    zero = torch.zeros(3, feat, dtype=torch.float64, device="cuda")
+    want_grads = (d[5] @ d[2], torch.cat([d[5] @ d[3], zero]), d[5].t() @ d[0], d[5].t() @ d[1][:n], d[5].sum(0))
+    for bias in (b, None):
+        for slabs in (1, 8):
+            out = backend.sage_linear(his, x, n, wl, bias, wr, slabs)
+            want = d[0] @ d[2].t() + d[1][:n] @ d[3].t() + (d[4] if bias is not None else 0)
+            assert (out - want).abs().max() <= 1e-5 * (1 + want.abs().max())
+            over = (his, x, wl, wr) + (() if bias is None else (b,))
+            for a, w in zip(torch.autograd.grad(out, over, g), want_grads):
+                assert (a - w).abs().max() <= 1e-5 * (1 + w.abs().max())
+    only = torch.autograd.grad(backend.sage_linear(his.detach(), x.detach(), n, wl.detach(), b, wr, 8), (b, wr), g)
+    assert (only[0] - want_grads[4]).abs().max() <= 1e-5 * (1 + want_grads[4].abs().max())
+    assert (only[1] - want_grads[3]).abs().max() <= 1e-5 * (1 + want_grads[3].abs().max())
 
 
 @pytest.mark.parametrize("n,classes", [(1, 2), (1000, 172), (1025, 47), (9000, 153)])
