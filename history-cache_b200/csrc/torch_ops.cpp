@@ -11,7 +11,9 @@
 //
 // The library's functions are looked up in the handle that the ctypes binding opened, so an
 // overridden library (the index-checking build) is the one that runs.
+#include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
@@ -20,6 +22,7 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/extension.h>
 
+#include <array>
 #include <atomic>
 #include <mutex>
 
@@ -1174,43 +1177,82 @@ py::tuple rgcn_group(const Tensor& ptr_in, const Tensor& idx_in, const Tensor& e
   return py::make_tuple(ptr2, cut(idx2), cut(w2), cut(perm), cut(rel));
 }
 
+// A branch beside the current stream, joined at the end of the scope.  Only while a step is being captured:
+// there the fork is two edges of the graph, while eager it would cost more host time than the overlap
+// brings.  The stream is this thread's own: a pooled one may belong to somebody who is not being captured.
+// What the branch writes is allocated before, on the main stream.
+class Branch {
+ public:
+  explicit Branch(const at::Device& dev, bool wanted)
+      : main_(c10::cuda::getCurrentCUDAStream(dev.index())), side_(main_) {
+    if (!wanted || c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) return;
+    thread_local std::array<cudaStream_t, 64> own{};
+    TORCH_CHECK(dev.index() >= 0 && dev.index() < 64, "hiscache_backend: device index");
+    cudaStream_t& st = own[dev.index()];
+    if (!st && cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) {
+      st = nullptr;
+      return;
+    }
+    side_ = c10::cuda::getStreamFromExternal(st, dev.index());
+    fork_.record(main_);
+    fork_.block(side_);
+    open_ = true;
+  }
+  Branch(const Branch&) = delete;
+  ~Branch() {
+    if (!open_) return;
+    try {
+      join_.record(side_);
+      join_.block(main_);
+    } catch (const std::exception&) {      // the capture is lost, its end reports it
+    }
+  }
+  c10::cuda::CUDAStream stream() const { return side_; }
+
+ private:
+  c10::cuda::CUDAStream main_, side_;
+  at::cuda::CUDAEvent fork_, join_;
+  bool open_ = false;
+};
+
 // g^T r for tall, narrow g [n, M] and r [n, N]: columns [0, split) of the result into left, the others into
 // right; column sums of g into bias (undefined = not wanted).  Such a product has a very long reduction and a
 // small output, which the library runs on a few dozen blocks: the rows are cut into slabs of at least 256, one
 // batched product gives the slabs' results, and hc_slab_sums adds them up, takes the few rows that fill no
 // slab along and finishes the bias.  The order of the additions is fixed.
 constexpr int64_t kSlabRows = 256;
-void tall_products(const Tensor& g, const Tensor& r, int64_t slabs, int64_t split, Tensor* left, Tensor* right, Tensor* bias) {
+void tall_products(const Tensor& g, const Tensor& r, int64_t slabs, int64_t split, Tensor* left, Tensor* right, Tensor* bias,
+                   const c10::cuda::CUDAStream& stream, variable_list& keep) {
   const at::Device dev = g.device();
   const int64_t n = g.size(0), M = g.size(1), N = r.size(1);
   int64_t s = std::max<int64_t>(slabs, 1);
   while (s > 1 && n / s < kSlabRows) s /= 2;
   const int64_t m = n / s, rest = n - m * s;
-  Tensor parts;
+  Tensor parts, sc;
+  const bool copied = s == 1 && split == N;      // the product is the result already
   if (left || right) {
-    if (s > 1) {
-      parts = at::bmm(g.narrow(0, 0, m * s).view({s, m, M}).transpose(1, 2), r.narrow(0, 0, m * s).view({s, m, N}));
-    } else {
-      parts = at::mm(g.t(), r);
-    }
-    if (s == 1 && left && split == N) {      // the product is the result already
-      *left = parts;
-      if (!bias) return;
-    }
-    if (left && !left->defined()) *left = new_f32({M, split}, dev);
+    parts = s > 1 ? new_f32({s, M, N}, dev) : new_f32({M, N}, dev);
+    if (left) *left = copied ? parts : new_f32({M, split}, dev);
     if (right) *right = new_f32({M, N - split}, dev);
   }
-  Tensor sc;
   if (bias) {
     *bias = new_f32({M}, dev);
     sc = new_scratch(lib.hc_slab_sums_scratch_bytes(M), dev);
   }
-  const bool copied = s == 1 && split == N;
+  keep = {parts, sc};      // the caller lets go of them behind the join
+  c10::cuda::CUDAStreamGuard on(stream);
+  if (parts.defined()) {
+    if (s > 1)
+      at::bmm_out(parts, g.narrow(0, 0, m * s).view({s, m, M}).transpose(1, 2), r.narrow(0, 0, m * s).view({s, m, N}));
+    else
+      at::mm_out(parts, g.t(), r);
+  }
+  if (!bias && copied) return;
   HC_SPAN("hc_slab_sums", dev);
   check(lib.hc_slab_sums(fdata(parts), (int32_t)s, M, (int32_t)N, rest ? fdata(g) + m * s * M : nullptr,
                          rest ? fdata(r) + m * s * N : nullptr, (int32_t)rest, (int32_t)split,
                          left && !copied ? fdata(*left) : nullptr, right ? fdata(*right) : nullptr, fdata(g), n,
-                         bias ? fdata(*bias) : nullptr, data(sc), stream_of(dev)),
+                         bias ? fdata(*bias) : nullptr, data(sc), stream.stream()),
         "hc_slab_sums");
   g_launches += (bias ? 1 : 0) + 1;
 }
@@ -1245,9 +1287,11 @@ struct RgcnBackward : public torch::autograd::Node {
     c10::cuda::CUDAGuard guard(dev);
     const int64_t F = xt.size(1), H = w.size(2);
     const Tensor g = grads[0].contiguous(), wide = sums.view({num_node, num_rel * F});
+    variable_list keep;
+    Branch beside(dev, task_should_compute_output(0) && task_should_compute_output(1));
     if (task_should_compute_output(1)) {
       Tensor gw;
-      tall_products(wide, g, kRgcnSlabs, H, &gw, nullptr, nullptr);
+      tall_products(wide, g, kRgcnSlabs, H, &gw, nullptr, nullptr, beside.stream(), keep);
       out[1] = gw.view({num_rel, F, H});
     }
     if (task_should_compute_output(0)) {
@@ -1367,7 +1411,15 @@ struct SageLinearBackward : public torch::autograd::Node {
     const Tensor g = grads[0].contiguous(), w = weight.unpack();
     const int64_t n = rows.size(0);
     const bool want_x = task_should_compute_output(4);
-    if (task_should_compute_output(0) || want_x || root) {
+    const bool want_l = task_should_compute_output(1), want_r = task_should_compute_output(3),
+               want_b = has_bias && task_should_compute_output(2);
+    const bool want_in = task_should_compute_output(0) || want_x || root;
+    variable_list keep;
+    Branch beside(rows.device(), want_in && (want_l || want_r || want_b));
+    if (want_l || want_r || want_b)
+      tall_products(g, rows, slabs, K, want_l ? &out[1] : nullptr, want_r ? &out[3] : nullptr, want_b ? &out[2] : nullptr,
+                    beside.stream(), keep);
+    if (want_in) {
       const Tensor g2 = at::mm(g, w);
       out[0] = g2.narrow(1, 0, K);
       if (root) root->rows = g2.narrow(1, K, K);
@@ -1376,10 +1428,6 @@ struct SageLinearBackward : public torch::autograd::Node {
         out[4].slice(0, 0, n).copy_(g2.narrow(1, K, K));
       }
     }
-    const bool want_l = task_should_compute_output(1), want_r = task_should_compute_output(3),
-               want_b = has_bias && task_should_compute_output(2);
-    if (want_l || want_r || want_b)
-      tall_products(g, rows, slabs, K, want_l ? &out[1] : nullptr, want_r ? &out[3] : nullptr, want_b ? &out[2] : nullptr);
     return out;
   }
 };
