@@ -19,8 +19,10 @@ import os
 
 # lin_l(aggregate) + lin_r(root) as one product (hiscache_backend.sage_linear)
 FUSE_ROOT_PRODUCT = os.environ.get("HISCACHE_FUSE_ROOT_PRODUCT", "1") not in ("", "0")
-# row slabs of its weight gradient (the products of a step of 16 K rows: 4 slabs 297 us, 8 261, 16 247, 32 247)
-SPLIT_WGRAD = int(os.environ.get("HISCACHE_SPLIT_WGRAD", "16"))
+# row slabs of its weight gradient: 4 / 8 / 16 / 32 slabs take 537 / 482 / 473 / 473 us a captured step of 16 K rows.
+# Eight keep the order of additions that trained models have seen: Adam turns a last-bit difference of a
+# gradient near zero into a step of full length.
+SPLIT_WGRAD = int(os.environ.get("HISCACHE_SPLIT_WGRAD", "8"))
 
 
 class MaskedBatchNorm1d(torch.nn.BatchNorm1d):
